@@ -12,7 +12,7 @@
  * Streams and CUDA graphs: the first call on a device creates a few KB of per-device state (a status word, work
  * counters and tensor-map slots, shared-memory opt-in of the kernels, a scratch pool) with synchronous calls; make it
  * outside a stream capture.  After that a forward call only enqueues kernels on `stream` (the split-KV path of
- * tfa_b200_fwd also a stream-ordered allocation and free; tfa_b200_fwd_decode_noalloc none), so it can be captured
+ * tfa_b200_fwd and eager fp32 calls also a stream-ordered allocation and free; tfa_b200_fwd_decode_noalloc none), so it can be captured
  * into a CUDA graph and replayed.  The persistent kernel hands out its work through a pair of device counters that two
  * launches must not use at the same time: eager launches take the pair of their stream (up to 1024 distinct streams
  * per device; the per-thread default stream counts once per calling thread), every captured launch takes a pair of
@@ -92,6 +92,9 @@ int tfa_b200_device_status(int* site);
  *   "solo64" 0/1       head dims 32 / 64: two-tile CTAs, one per SM / one-tile CTAs, two per SM (the default)
  *   "fp32_t8" 0/1/2    fp32, head dim 128: 4 x 8 thread tiles always / 8 x 8 thread tiles for problems of at least three
  *                      CTAs per SM (the default) / 8 x 8 always
+ *   "fp32_tc" -1/0/1   fp32, head dims up to 128: on the tensor cores with every float as three bf16 numbers by size /
+ *                      never / wherever it applies (not under stream capture, not for packed input of unknown totals).
+ *                      Choosing a CUDA-core form with "fp32_t8" switches "by size" off.
  *   "pair_cta" -1/0/1  head dims 192 / 256, fixed-length input: clusters of two CTAs that work on two neighbouring query
  *                      tiles and share every K/V block through one MMA over both SMs (tcgen05 cta_group::2):
  *                      auto (head dim 256: non-causal, and causal from 1024 query rows; head dim 192: never, its

@@ -1,0 +1,105 @@
+"""fp32 on the tensor cores (three bf16 numbers per float) against the fp64 oracle and the CUDA-core kernel (run with -m gpu).
+
+Bound: both kernels sum in fp32, so both are within a few units of 2^-24 times the number of additions of the exact
+result; the tensor-core one sums 128 keys at a time and must not be further off (2-norm) than the CUDA-core one by more
+than the spread between two orders of summation, for which a quarter is allowed on these short sequences."""
+import numpy as np
+import pytest
+import torch
+
+import tinyfa_b200 as tf
+from oracle import attention_oracle as ao
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [  # batch, seqQ, seqKV, headsQ, headsKV: tile edges, remainders, one row, one key, several blocks
+    (1, 1, 1, 1, 1),
+    (2, 1, 130, 4, 1),
+    (1, 127, 129, 2, 1),
+    (2, 128, 128, 3, 3),
+    (1, 129, 255, 4, 2),
+    (1, 257, 640, 6, 2),
+    (2, 40, 1111, 8, 2),
+    (1, 700, 300, 2, 2),
+]
+
+
+def _with(option, fn):
+    tf.set_option("fp32_tc", option)
+    try:
+        out = fn()
+        torch.cuda.synchronize()
+        tf.device_status()
+        return out
+    finally:
+        tf.set_option("fp32_tc", -1)
+
+
+def _inputs(B, Sq, Skv, Hq, Hkv, D, seed):
+    rng = np.random.default_rng(seed)
+    return [rng.normal(0, 1, s).astype(np.float32) for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D))]
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [32, 64, 96, 128])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_against_the_oracle_and_the_cuda_core_kernel(shape, D, causal):
+    Q, K, V = _inputs(*shape, D, 7 + D + shape[1])
+    dev = [torch.from_numpy(x).cuda() for x in (Q, K, V)]
+    ref = ao.fixed(Q, K, V, causal, "f64")
+    got = _with(1, lambda: tf.flash_attn_forward(*dev, is_causal=causal)).cpu().numpy()
+    old = _with(0, lambda: tf.flash_attn_forward(*dev, is_causal=causal)).cpu().numpy()
+    assert np.abs(got - ref).max() <= 1e-5
+    assert np.linalg.norm(got - ref) <= 1.25 * np.linalg.norm(old - ref) + 1e-7 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_packed_input(D, causal):
+    lens_q, lens_kv = [5, 0, 200, 64, 300, 1], [40, 9, 200, 0, 511, 128]
+    cu_q = np.concatenate([[0], np.cumsum(lens_q)]).astype(np.int32)
+    cu_kv = np.concatenate([[0], np.cumsum(lens_kv)]).astype(np.int32)
+    rng = np.random.default_rng(D)
+    Q = rng.normal(0, 1, (int(cu_q[-1]), 4, D)).astype(np.float32)
+    K, V = (rng.normal(0, 1, (int(cu_kv[-1]), 2, D)).astype(np.float32) for _ in range(2))
+    args = [torch.from_numpy(x).cuda() for x in (Q, K, V, cu_q, cu_kv)]
+    got = _with(1, lambda: tf.flash_attn_varlen_forward(*args, max(lens_q), max(lens_kv), is_causal=causal)).cpu().numpy()
+    assert np.abs(got - ao.varlen(Q, K, V, cu_q, cu_kv, causal)).max() <= 1e-5
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf"), 2.0**60, 1e-38, -2.0**-101])
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_values_outside_the_exact_range_are_left_to_the_cuda_cores(which, value):
+    arrays = _inputs(2, 150, 260, 4, 2, 64, 3)
+    arrays[which][1, 33, 1, 5] = value
+    dev = [torch.from_numpy(x).cuda() for x in arrays]
+    got = _with(1, lambda: tf.flash_attn_forward(*dev))
+    old = _with(0, lambda: tf.flash_attn_forward(*dev))
+    assert torch.equal(got.view(torch.int32), old.view(torch.int32))
+
+
+def test_magnitudes_inside_the_exact_range():
+    """Magnitudes far from 1 but inside the accepted range, and zeros, go through the tensor cores without loss."""
+    Q, K, V = _inputs(1, 130, 300, 2, 2, 64, 11)
+    Q *= np.float32(2.0**-50)
+    K *= np.float32(2.0**50)
+    V *= np.float32(2.0**-60)
+    V[:, ::3] = 0
+    assert all(np.abs(x[x != 0]).min() > 2.0**-100 and np.abs(x).max() < 2.0**60 for x in (Q, K, V))
+    dev = [torch.from_numpy(x).cuda() for x in (Q, K, V)]
+    got = _with(1, lambda: tf.flash_attn_forward(*dev)).cpu().numpy().astype(np.float64)
+    old = _with(0, lambda: tf.flash_attn_forward(*dev)).cpu().numpy().astype(np.float64)
+    ref = ao.fixed(Q, K, V, False, "f64").astype(np.float64)
+    assert np.linalg.norm(got - ref) <= 1.25 * np.linalg.norm(old - ref)
+
+
+def test_captured_calls_replay():
+    """Under capture the call stays on the CUDA cores; the graph replays and gives their result."""
+    Q, K, V = (torch.from_numpy(x).cuda() for x in _inputs(1, 600, 600, 4, 4, 64, 5))
+    want = _with(0, lambda: tf.flash_attn_forward(Q, K, V))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = tf.flash_attn_forward(Q, K, V)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)

@@ -57,6 +57,11 @@ int splitkv_num_splits(const FwdProblem& p, int numSMs);
 size_t splitkv_scratch_floats(const FwdProblem& p, int splits);
 int launch_fwd_splitkv(const FwdProblem& p, int splits, float* scratch);
 
+// ---- fp32 on the tensor cores (fwd_fp32_tc.cu)
+bool fp32tc_applicable(const FwdProblem& p, int option);
+size_t fp32tc_workspace_bytes(const FwdProblem& p);
+int launch_fwd_fp32tc(const FwdProblem& p, int packShift, void* ws, int epoch);
+
 static thread_local char g_err[512] = "";
 
 void set_error_string(const char* fmt, ...) {
@@ -80,6 +85,7 @@ static std::atomic<int> g_optPairCta{-1};  // head dims 192 / 256, fixed length:
 int option_pair_cta() { return g_optPairCta.load(); }
 static std::atomic<int> g_optFp32T8{1};  // fp32, head dim 128, large problems: the 8 x 8 thread-tile form
 int option_fp32_t8() { return g_optFp32T8.load(); }
+static std::atomic<int> g_optFp32Tc{-1};  // fp32 on the tensor cores: -1 by size, 0 never, 1 wherever it applies
 
 int next_epoch() { return (g_epoch.fetch_add(1) & 0x7FFFFF) + 1; }
 
@@ -231,9 +237,11 @@ int launch_patch_varlen_maps(const CUtensorMap& mq, const CUtensorMap& mk, const
   return kOk;
 }
 
-// Stream-ordered scratch for the split-KV partials comes from a pool of this library's own, one per device, that
-// keeps its memory across synchronisations (release threshold = max): with the default pool every call that
-// follows a device synchronise would pay a fresh device allocation (~200 us, measured).
+// Stream-ordered scratch (split-KV partials, the parts of fp32 inputs) comes from a pool of this library's own, one per
+// device, that keeps up to kPoolKeepBytes across synchronisations: with the default pool every call that follows a
+// device synchronise would pay a fresh device allocation (~200 us, measured).  What it holds beyond that goes back to
+// the driver at the next synchronisation.
+constexpr unsigned long long kPoolKeepBytes = 1ull << 30;
 static cudaMemPool_t g_scratchPool[64] = {nullptr};
 static cudaMemPool_t scratch_pool(int device) {
   std::lock_guard<std::mutex> lock(g_devMutex);
@@ -250,7 +258,7 @@ static cudaMemPool_t scratch_pool(int device) {
       cudaGetLastError();
       return nullptr;
     }
-    unsigned long long keep = ~0ull;
+    unsigned long long keep = kPoolKeepBytes;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     g_scratchPool[device] = pool;
   }
@@ -354,8 +362,41 @@ static int dispatch_splitkv(const FwdProblem& p, int splits) {
   return rc;
 }
 
+// fp32: the tensor cores where that pays, else the CUDA cores.  The tensor-core kernel leaves inputs that its three-part
+// form does not hold exactly (infinities, NaN, extreme magnitudes) to the CUDA-core kernel, which is enqueued behind it and
+// decides on the device.  Nothing is refused for lack of workspace: the CUDA cores need none.  A stream under capture stays
+// on the CUDA cores, because an allocation captured into a graph would limit what the caller may do with that graph.
+static int dispatch_fp32(const FwdProblem& p) {
+  const int opt = g_optFp32Tc.load();
+  // an explicit choice of the CUDA-core form (option "fp32_t8") is kept
+  if (opt == 0 || (opt < 0 && g_optFp32T8.load() != 1) || !fp32tc_applicable(p, opt)) return launch_fwd_fp32(p);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  int device = 0;
+  if (cudaStreamIsCapturing(p.stream, &cap) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
+    set_error_string("cudaStreamIsCapturing: %s", cudaGetErrorString(cudaGetLastError()));
+    return kCudaError;
+  }
+  if (cap != cudaStreamCaptureStatusNone) return launch_fwd_fp32(p);
+  cudaMemPool_t pool = scratch_pool(device);
+  void* ws = nullptr;
+  if (pool == nullptr || cudaMallocFromPoolAsync(&ws, fp32tc_workspace_bytes(p), pool, p.stream) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return launch_fwd_fp32(p);
+  }
+  const int epoch = next_epoch();
+  int rc = launch_fwd_fp32tc(p, pick_pack_shift(p), ws, epoch);
+  if (rc == kOk) {
+    FwdProblem rest = p;
+    rest.gate = static_cast<const int*>(ws);
+    rest.gateEpoch = epoch;
+    rc = launch_fwd_fp32(rest);
+  }
+  cudaFreeAsync(ws, p.stream);
+  return rc;
+}
+
 static int dispatch(const FwdProblem& p) {
-  if (p.dtype == kFp32) return launch_fwd_fp32(p);
+  if (p.dtype == kFp32) return dispatch_fp32(p);
   const int optSplit = g_optSplitKv.load();
   if (optSplit != 0 && p.totalQ >= 0 && splitkv_applicable(p)) {
     int splits = (optSplit > 0) ? optSplit : splitkv_num_splits(p, num_sms());
@@ -570,6 +611,10 @@ extern "C" int tfa_b200_set_option(const char* name, int value) {
   }
   if (strcmp(name, "fp32_t8") == 0) {
     g_optFp32T8.store(value < 0 ? 1 : (value > 2 ? 2 : value));
+    return kOk;
+  }
+  if (strcmp(name, "fp32_tc") == 0) {
+    g_optFp32Tc.store(value < 0 ? -1 : (value ? 1 : 0));
     return kOk;
   }
   if (strcmp(name, "pair_cta") == 0) {

@@ -38,9 +38,14 @@ struct Fp32Params {
   int group;
   int causal;
   float scaleLog2;
+  const int* gate;  // see FwdProblem
+  int gateEpoch;
 };
 
 namespace fp32 {
+
+__device__ __forceinline__ bool gated_off(const Fp32Params& p) { return p.gate != nullptr && *p.gate != p.gateEpoch; }
+
 
 constexpr int kRowsPerThread = 4;
 [[maybe_unused]] constexpr int kBC = 64;
@@ -105,6 +110,7 @@ __global__ void __launch_bounds__(BR * 8 / kRowsPerThread) fwd_fp32_kernel(const
   float* sV = sK + kBC * LD;
   float* sP = sV + kBC * LD;
 
+  if (gated_off(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
   long long qRow0, kvRow0;
@@ -356,6 +362,7 @@ __global__ void __launch_bounds__(256) fwd_fp32_lane_kernel(const Fp32Params p) 
   float* sV = sK + BC * LD;
   float* sP = sV + BC * LD;
 
+  if (gated_off(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
   long long qRow0, kvRow0;
@@ -571,6 +578,8 @@ int launch_lane(const FwdProblem& pr) {
   p.headsKV = pr.headsKV;
   p.group = pr.headsQ / pr.headsKV;
   p.causal = pr.causal;
+  p.gate = pr.gate;
+  p.gateEpoch = pr.gateEpoch;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   dim3 grid((unsigned)((pr.seqLenQ + 63) / 64), (unsigned)pr.headsQ, (unsigned)pr.batch);
   kernel<<<grid, 256, kSmem, pr.stream>>>(p);
@@ -613,6 +622,7 @@ __global__ void __launch_bounds__(256, 1) fwd_fp32_t8_kernel(const Fp32Params p)
   float* sPT = sK;  // aliased: P^T of block j overwrites K(j) once every warp is done with Q.K^T
   static_assert(BC * LDP <= BC * LD, "P^T fits the K buffer");
 
+  if (gated_off(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
   long long qRow0, kvRow0;
@@ -849,6 +859,8 @@ int launch_t8(const FwdProblem& pr) {
   p.headsKV = pr.headsKV;
   p.group = pr.headsQ / pr.headsKV;
   p.causal = pr.causal;
+  p.gate = pr.gate;
+  p.gateEpoch = pr.gateEpoch;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   dim3 grid((unsigned)((pr.seqLenQ + 127) / 128), (unsigned)pr.headsQ, (unsigned)pr.batch);
   kernel<<<grid, 256, kSmem, pr.stream>>>(p);
@@ -889,6 +901,8 @@ int launch(const FwdProblem& pr) {
   p.headsKV = pr.headsKV;
   p.group = pr.headsQ / pr.headsKV;
   p.causal = pr.causal;
+  p.gate = pr.gate;
+  p.gateEpoch = pr.gateEpoch;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   dim3 grid((unsigned)((pr.seqLenQ + BR - 1) / BR), (unsigned)pr.headsQ, (unsigned)pr.batch);
   kernel<<<grid, BR * 8 / kRowsPerThread, kSmem, pr.stream>>>(p);

@@ -45,6 +45,9 @@ struct FwdProblem {
   int headDim;
   int causal;
   cudaStream_t stream;
+  // fp32 CUDA-core kernels: when not null, they return at once unless this device word reads gateEpoch (see fwd_fp32_tc.cu)
+  const int* gate = nullptr;
+  int gateEpoch = 0;
 };
 
 // The device status word holds 0, or (launch epoch << 8) | site code once a bounded wait inside a kernel gave up.
