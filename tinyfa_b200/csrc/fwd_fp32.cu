@@ -44,7 +44,12 @@ struct Fp32Params {
 
 namespace fp32 {
 
-__device__ __forceinline__ bool gated_off(const Fp32Params& p) { return p.gate != nullptr && *p.gate != p.gateEpoch; }
+// kGated instantiations run behind the tensor-core kernel and return at once unless it left the call to them.  Calls that
+// come here straight away have instantiations of their own: the check at the top cost a 23 us call 4 %.
+template <bool kGated>
+__device__ __forceinline__ bool gated_off(const Fp32Params& p) {
+  return kGated && *p.gate != p.gateEpoch;
+}
 
 
 constexpr int kRowsPerThread = 4;
@@ -97,7 +102,7 @@ __device__ __forceinline__ void load_tile(float* sm, const float* base, long lon
   }
 }
 
-template <int D, int BR>
+template <int D, int BR, bool kGated>
 __global__ void __launch_bounds__(BR * 8 / kRowsPerThread) fwd_fp32_kernel(const Fp32Params p) {
   constexpr int kThreads = BR * 8 / kRowsPerThread;
   constexpr int LD = D + 4;
@@ -110,7 +115,7 @@ __global__ void __launch_bounds__(BR * 8 / kRowsPerThread) fwd_fp32_kernel(const
   float* sV = sK + kBC * LD;
   float* sP = sV + kBC * LD;
 
-  if (gated_off(p)) return;
+  if (gated_off<kGated>(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
   long long qRow0, kvRow0;
@@ -362,7 +367,6 @@ __global__ void __launch_bounds__(256) fwd_fp32_lane_kernel(const Fp32Params p) 
   float* sV = sK + BC * LD;
   float* sP = sV + BC * LD;
 
-  if (gated_off(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
   long long qRow0, kvRow0;
@@ -607,7 +611,7 @@ int launch_lane(const FwdProblem& pr) {
 // Measured at B2 S4096 H32: 46.4 -> 49.4 TFLOP/s non-causal, 41.8 -> 44.4 causal; shared-memory data pipe 77 % -> 52 %
 // busy, FMA pipe 65 % -> 70 %; 255 registers, so the SM runs these 8 warps and no more, and what is left is latency that
 // two warps per scheduler do not cover.
-template <int D>
+template <int D, bool kGated>
 __global__ void __launch_bounds__(256, 1) fwd_fp32_t8_kernel(const Fp32Params p) {
   static_assert(D == 128, "8 x 8 form: head dim 128");
   constexpr int BR = 128, BC = 128, kThreads = 256;
@@ -622,7 +626,7 @@ __global__ void __launch_bounds__(256, 1) fwd_fp32_t8_kernel(const Fp32Params p)
   float* sPT = sK;  // aliased: P^T of block j overwrites K(j) once every warp is done with Q.K^T
   static_assert(BC * LDP <= BC * LD, "P^T fits the K buffer");
 
-  if (gated_off(p)) return;
+  if (gated_off<kGated>(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
   long long qRow0, kvRow0;
@@ -834,13 +838,16 @@ __global__ void __launch_bounds__(256, 1) fwd_fp32_t8_kernel(const Fp32Params p)
 template <int D>
 int launch_t8(const FwdProblem& pr) {
   constexpr int kSmem = (D * (128 + 4) + 2 * 128 * (D + 4)) * (int)sizeof(float);
-  auto kernel = fwd_fp32_t8_kernel<D>;
+  auto kernel = pr.gate != nullptr ? fwd_fp32_t8_kernel<D, true> : fwd_fp32_t8_kernel<D, false>;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return kCudaError;
   static std::once_flag once[64];
   static cudaError_t attrErr[64];
   std::call_once(once[device], [&] {
-    attrErr[device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    attrErr[device] = cudaFuncSetAttribute(fwd_fp32_t8_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (attrErr[device] == cudaSuccess) {
+      attrErr[device] = cudaFuncSetAttribute(fwd_fp32_t8_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    }
   });
   if (attrErr[device] != cudaSuccess) {
     set_error_string("cudaFuncSetAttribute(%d bytes): %s", kSmem, cudaGetErrorString(attrErr[device]));
@@ -876,13 +883,16 @@ template <int D, int BR>
 int launch(const FwdProblem& pr) {
   constexpr int LD = D + 4;
   constexpr int kSmem = (BR * LD + 2 * kBC * LD + BR * (kBC + 4)) * (int)sizeof(float);
-  auto kernel = fwd_fp32_kernel<D, BR>;
+  auto kernel = pr.gate != nullptr ? fwd_fp32_kernel<D, BR, true> : fwd_fp32_kernel<D, BR, false>;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return kCudaError;
   static std::once_flag once[64];
   static cudaError_t attrErr[64];
   std::call_once(once[device], [&] {
-    attrErr[device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    attrErr[device] = cudaFuncSetAttribute(fwd_fp32_kernel<D, BR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (attrErr[device] == cudaSuccess) {
+      attrErr[device] = cudaFuncSetAttribute(fwd_fp32_kernel<D, BR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    }
   });
   if (attrErr[device] != cudaSuccess) {
     set_error_string("cudaFuncSetAttribute(%d bytes): %s", kSmem, cudaGetErrorString(attrErr[device]));
