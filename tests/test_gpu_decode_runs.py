@@ -1,0 +1,57 @@
+"""Even partition of the decode path: equal runs of key blocks across batch entries, against the fp64 oracle (run with -m gpu).
+
+Sizes where it can go wrong: an entry that is one run, runs that end inside an entry and go on into the next one, last
+blocks that are nearly empty, more entries than runs, one KV head and many, and the same call through the entry point that
+allocates nothing.  Tolerance: weights and output are rounded to 16 bits, 2^-9 (bf16) or 2^-12 (fp16) of values below 4."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import tinyfa_b200 as tf
+from oracle import attention_oracle as ao
+from tinyfa_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [  # batch, seqQ, seqKV, headsQ, headsKV
+    (1, 1, 256, 1, 1),
+    (3, 1, 257, 8, 8),
+    (5, 2, 1000, 8, 2),
+    (37, 1, 320, 32, 32),
+    (1, 1, 20000, 4, 1),
+    (7, 3, 4097, 10, 2),
+    (300, 1, 300, 2, 1),
+    (70, 1, 449, 16, 16),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [32, 64, 96, 128, 192, 256])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_even_partition(shape, D, dtype):
+    B, Sq, Skv, Hq, Hkv = shape
+    g = torch.Generator(device="cuda").manual_seed(D + Skv)
+    Q, K, V = (torch.randn(*s, device="cuda", generator=g).to(dtype)
+               for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
+    got = tf.flash_attn_forward(Q, K, V)
+    flat = torch.empty_like(Q)
+    rc = _lib.load().tfa_b200_fwd_decode_noalloc(
+        *(ctypes.c_void_p(t.data_ptr()) for t in (Q, K, V, flat)), 1 if dtype == torch.float16 else 2, B, Sq, Skv, Hq, Hkv,
+        D, 0, 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    tf.device_status()
+    assert torch.equal(got, flat)
+    pick = sorted({0, B // 2, B - 1})
+    ref = ao.fixed(*(t[pick].float().cpu().numpy() for t in (Q, K, V)), False, "f64")
+    assert np.abs(got[pick].float().cpu().numpy() - ref).max() <= (2e-3 if dtype == torch.float16 else 1.6e-2)
+
+
+def test_nan_key_poisons_its_rows_and_no_others():
+    Q, K, V = (torch.randn(*s, device="cuda").bfloat16() for s in ((4, 1, 8, 64), (4, 3000, 2, 64), (4, 3000, 2, 64)))
+    K[2, 1234, 1] = float("nan")
+    out = tf.flash_attn_forward(Q, K, V)
+    assert torch.isnan(out[2, :, 4:]).all()
+    out[2, :, 4:] = 0
+    assert torch.isfinite(out).all()

@@ -53,9 +53,9 @@ TFA_DECLARE_TC(256)
 
 // ---- split-KV path for short query blocks (fwd_decode.cu)
 bool splitkv_applicable(const FwdProblem& p);
-int splitkv_num_splits(const FwdProblem& p, int numSMs);
-size_t splitkv_scratch_floats(const FwdProblem& p, int splits);
-int launch_fwd_splitkv(const FwdProblem& p, int splits, float* scratch);
+SplitPlan splitkv_plan(const FwdProblem& p, int numSMs, int forced);
+size_t splitkv_scratch_floats(const FwdProblem& p, const SplitPlan& plan);
+int launch_fwd_splitkv(const FwdProblem& p, const SplitPlan& plan, float* scratch);
 
 // ---- fp32 on the tensor cores (fwd_fp32_tc.cu)
 bool fp32tc_applicable(const FwdProblem& p, int option);
@@ -341,8 +341,8 @@ static int num_sms() {
 
 // Short query blocks: stream K/V once for all Q heads of a KV head and split the key range over CTAs.  The partial
 // results live in a stream-ordered scratch allocation that is released behind the combine kernel.
-static int dispatch_splitkv(const FwdProblem& p, int splits) {
-  const size_t floats = splitkv_scratch_floats(p, splits);
+static int dispatch_splitkv(const FwdProblem& p, const SplitPlan& plan) {
+  const size_t floats = splitkv_scratch_floats(p, plan);
   float* scratch = nullptr;
   if (floats > 0) {
     int device = 0;
@@ -357,7 +357,7 @@ static int dispatch_splitkv(const FwdProblem& p, int splits) {
       return kCudaError;
     }
   }
-  const int rc = launch_fwd_splitkv(p, splits, scratch);
+  const int rc = launch_fwd_splitkv(p, plan, scratch);
   if (scratch != nullptr) cudaFreeAsync(scratch, p.stream);
   return rc;
 }
@@ -399,10 +399,7 @@ static int dispatch(const FwdProblem& p) {
   if (p.dtype == kFp32) return dispatch_fp32(p);
   const int optSplit = g_optSplitKv.load();
   if (optSplit != 0 && p.totalQ >= 0 && splitkv_applicable(p)) {
-    int splits = (optSplit > 0) ? optSplit : splitkv_num_splits(p, num_sms());
-    const int maxSplits = (p.seqLenKV + 63) / 64;
-    if (splits > maxSplits) splits = maxSplits;
-    return dispatch_splitkv(p, splits);
+    return dispatch_splitkv(p, splitkv_plan(p, num_sms(), optSplit));
   }
   const bool bf = (p.dtype == kBf16);
   const int ps = pick_pack_shift(p);

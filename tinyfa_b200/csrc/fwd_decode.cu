@@ -6,11 +6,16 @@
 // around memory parallelism, not around the tcgen05 pipe:
 //   * the (seqQ x group) query rows that share one KV head (at most 16) form one 16-row MMA tile, so a KV head is
 //     streamed once for all of its Q heads;
-//   * the key range is split over gridDim.x CTAs so that B x Hkv x splits fills the 148 SMs several times;
+//   * the key blocks of all batch entries are cut into equal runs, so that every CTA that fits the GPU streams the same
+//     amount whatever the batch and the lengths are (packed input: key-range splits of every sequence);
 //   * each CTA streams 64-key K and V blocks through a 3-stage cp.async ring (16-byte chunks, XOR-swizzled so that
 //     ldmatrix is conflict-free); each of its 4 warps owns 16 keys of a block with its own online softmax
 //     (mma.sync m16n8k16, fp32 accumulate: the tensor work is negligible next to the memory stream);
-//   * warps are merged through shared memory, splits through a small fp32 scratch buffer and a combine kernel.
+//   * warps are merged through shared memory, partial results through a small fp32 scratch buffer and a combine kernel
+//     that is launched while the split kernel runs (programmatic dependent launch) and reads a row's partials side by side.
+// Measured against a fixed number of splits per pair and a combine kernel that walked them (8 KV heads, D = 128, floor in
+// brackets at 6.54 TB/s): batch 1 x 32768 keys 37.8 -> 31 us (20.5), 8 x 20011 113 -> 103 (100), 40 x 5000 174 -> 135 (125), 13 x
+// 8000 74 -> 74 (65), 6 x 12000 58 -> 55 (45).  What is left at small batch is launch, the first loads and the combine.
 // Numerical contract as in the main kernel (reference csrc/flash_attn/mma/softmax.cuh:67-138): scale 1/sqrt(D)
 // folded into exp2, top-left causal mask, "col >= seqLenKV" mask, P rounded to the 16-bit type before P.V, row sum
 // from unrounded P, empty rows give 0.
@@ -48,8 +53,13 @@ struct Params {
   int headsKV;
   int group;
   int causal;
-  int splits;
-  int keysPerSplit;  // multiple of kBlockKeys
+  // Even partition (fixed-length input): the key blocks of all batch entries, in order, are cut into `runs` equal runs; a
+  // CTA is one KV head of a run.  runs == 0: one CTA per (split, KV head, batch entry) of a three-dimensional grid.
+  int runs;
+  int blocksPerEntry;
+  long long totalBlocks;
+  int splits;        // three-dimensional grid: key-range splits
+  int keysPerSplit;  // three-dimensional grid: multiple of kBlockKeys
   long long totalQ;  // rows of Q (for the partial buffers' stride)
   float scaleLog2;
 };
@@ -90,6 +100,11 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float fmax_nan(float a, float b) {  // NaN is kept
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
 template <bool kBf16>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   if constexpr (kBf16) {
@@ -116,6 +131,13 @@ __device__ __forceinline__ uint32_t swz(int r, int c) {
   }
 }
 
+// Row pitch (floats) of the merge buffer: eight floats past a multiple of the 32 banks, so that the eight rows of a warp's
+// accumulator fragment do not share a bank.
+template <int D>
+constexpr int merge_ld() {
+  return D + 8;
+}
+
 // 64 keys x D of one KV head -> one stage; keys >= keyEnd are zero-filled.
 template <int D>
 __device__ __forceinline__ void load_block(uint32_t smemDst, const uint16_t* base, long long rowStride, long long key0,
@@ -132,282 +154,372 @@ __device__ __forceinline__ void load_block(uint32_t smemDst, const uint16_t* bas
   }
 }
 
+// Run of the even partition that holds block `u`, i.e. the c with total * c / runs <= u < total * (c + 1) / runs.
+__host__ __device__ __forceinline__ int run_of_block(long long u, long long total, int runs) {
+  return (int)(((u + 1) * runs - 1) / total);
+}
+
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
   constexpr int kTileBytes = kBlockKeys * D * 2;
   constexpr int kNT = D / 8;  // 8-wide output column tiles
+  constexpr int kLdO = merge_ld<D>();
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sBase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  float* sO = reinterpret_cast<float*>(smem + kStages * 2 * kTileBytes);  // [16][kLdO]
+  float* sM = sO + kRows * kLdO;                                          // [4][16]
+  float* sL = sM + 4 * kRows;                                             // [4][16]
 
-  const int split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
-  long long qRow0, kvRow0;
+  // the combine kernel may be launched (it waits for the end of this grid before it reads anything)
+  asm volatile("griddepcontrol.launch_dependents;");
+  const bool even = p.runs > 0;
+  int b, part;         // batch entry and partial-result slot of the current segment
+  int hkv;
   int sq, skv;
-  if (p.cuQ != nullptr) {
-    qRow0 = p.cuQ[b];
-    sq = p.cuQ[b + 1] - p.cuQ[b];
-    kvRow0 = p.cuKV[b];
-    skv = p.cuKV[b + 1] - p.cuKV[b];
-  } else {
+  long long qRow0, kvRow0;
+  int key0, keyEnd;    // keys of the entry that this CTA starts at / may see
+  int count;           // blocks of this CTA
+  if (even) {
+    // neighbouring CTAs are the KV heads of one run: they read neighbouring parts of the same rows at the same time
+    const int run = (int)blockIdx.x / p.headsKV;
+    hkv = (int)blockIdx.x - run * p.headsKV;
+    const long long u0 = p.totalBlocks * run / p.runs, u1 = p.totalBlocks * (run + 1) / p.runs;
+    b = (int)(u0 / p.blocksPerEntry);
+    const long long first = (long long)b * p.blocksPerEntry;
+    key0 = (int)(u0 - first) * kBlockKeys;
+    count = (int)(u1 - u0);
+    part = run - run_of_block(first, p.totalBlocks, p.runs);
     sq = p.seqLenQ;
     skv = p.seqLenKV;
     qRow0 = (long long)b * sq;
     kvRow0 = (long long)b * skv;
+    keyEnd = p.causal ? min(skv, sq) : skv;  // top-left causal: key j needs j <= i <= sq-1
+  } else {
+    part = blockIdx.x;
+    hkv = blockIdx.y;
+    b = blockIdx.z;
+    if (p.cuQ != nullptr) {
+      qRow0 = p.cuQ[b];
+      sq = p.cuQ[b + 1] - p.cuQ[b];
+      kvRow0 = p.cuKV[b];
+      skv = p.cuKV[b + 1] - p.cuKV[b];
+    } else {
+      sq = p.seqLenQ;
+      skv = p.seqLenKV;
+      qRow0 = (long long)b * sq;
+      kvRow0 = (long long)b * skv;
+    }
+    if (sq <= 0) return;
+    if (skv <= 0 && p.splits == 1) return;  // nothing to write; with splits > 1 the partials must still be defined
+    keyEnd = p.causal ? min(skv, sq) : skv;
+    // keysPerSplit comes from the caller's maximum key length, which only sizes the launch: the last split runs to
+    // the real end of the sequence, so an understated maximum loses no keys (the reference derives its key loop from
+    // the actual length as well, reference csrc/flash_attn/params.cuh:156-163).
+    key0 = part * p.keysPerSplit;
+    if (part != p.splits - 1) keyEnd = min(key0 + p.keysPerSplit, keyEnd);
+    count = (keyEnd > key0) ? (keyEnd - key0 + kBlockKeys - 1) / kBlockKeys : 0;
   }
-  if (sq <= 0) return;
-  if (skv <= 0 && p.splits == 1) return;  // nothing to write; with splits > 1 the partials must still be defined
   const int nRows = sq * p.group;  // <= 16 by dispatch
-  int keyEnd = skv;
-  if (p.causal) keyEnd = min(keyEnd, sq);  // top-left causal: key j needs j <= i <= sq-1
-  // keysPerSplit comes from the caller's maximum key length, which only sizes the launch: the last split runs to
-  // the real end of the sequence, so an understated maximum loses no keys (the reference derives its key loop from
-  // the actual length as well, reference csrc/flash_attn/params.cuh:156-163).
-  const int key0 = split * p.keysPerSplit;
-  const int key1 = (split == p.splits - 1) ? keyEnd : min(key0 + p.keysPerSplit, keyEnd);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
 
   const long long qStride = (long long)p.headsQ * D;
   const long long kvStride = (long long)p.headsKV * D;
-  const uint16_t* gK = reinterpret_cast<const uint16_t*>(p.K) + kvRow0 * kvStride + (long long)hkv * D;
-  const uint16_t* gV = reinterpret_cast<const uint16_t*>(p.V) + kvRow0 * kvStride + (long long)hkv * D;
 
   // rows of this thread's fragments: r0 = g, r1 = g + 8; row r <-> (query position r / group, head hkv*group + r % group)
   const int rowA = g, rowB = g + 8;
   const int qposA = rowA / p.group, qposB = rowB / p.group;
-  const int headA = hkv * p.group + rowA % p.group, headB = hkv * p.group + rowB % p.group;
   const bool validA = rowA < nRows, validB = rowB < nRows;
+  const float c = p.scaleLog2;
 
   float o[kNT][4];
+  float mA, mB, lA, lB;
+  uint32_t qf[D / 16][4];
+  auto startSegment = [&]() {
 #pragma unroll
-  for (int i = 0; i < kNT; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;
-
-  const int nBlocks = (key1 > key0) ? (key1 - key0 + kBlockKeys - 1) / kBlockKeys : 0;
-  if (nBlocks > 0) {
-    // Q fragments (A operand), loaded once straight from global memory.
-    uint32_t qf[D / 16][4];
-    {
-      const uint16_t* gQ = reinterpret_cast<const uint16_t*>(p.Q);
-      const uint16_t* qa = gQ + (qRow0 + qposA) * qStride + (long long)headA * D;
-      const uint16_t* qb = gQ + (qRow0 + qposB) * qStride + (long long)headB * D;
+    for (int i = 0; i < kNT; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    mA = mB = -INFINITY;
+    lA = lB = 0.f;
+    // Q fragments (A operand), straight from global memory.
+    const uint16_t* gQ = reinterpret_cast<const uint16_t*>(p.Q);
+    const uint16_t* qa = gQ + (qRow0 + qposA) * qStride + (long long)(hkv * p.group + rowA % p.group) * D;
+    const uint16_t* qb = gQ + (qRow0 + qposB) * qStride + (long long)(hkv * p.group + rowB % p.group) * D;
 #pragma unroll
-      for (int ks = 0; ks < D / 16; ks++) {
-        const int c0 = ks * 16 + 2 * tig;
-        qf[ks][0] = validA ? *reinterpret_cast<const uint32_t*>(qa + c0) : 0u;
-        qf[ks][1] = validB ? *reinterpret_cast<const uint32_t*>(qb + c0) : 0u;
-        qf[ks][2] = validA ? *reinterpret_cast<const uint32_t*>(qa + c0 + 8) : 0u;
-        qf[ks][3] = validB ? *reinterpret_cast<const uint32_t*>(qb + c0 + 8) : 0u;
-      }
+    for (int ks = 0; ks < D / 16; ks++) {
+      const int c0 = ks * 16 + 2 * tig;
+      qf[ks][0] = validA ? *reinterpret_cast<const uint32_t*>(qa + c0) : 0u;
+      qf[ks][1] = validB ? *reinterpret_cast<const uint32_t*>(qb + c0) : 0u;
+      qf[ks][2] = validA ? *reinterpret_cast<const uint32_t*>(qa + c0 + 8) : 0u;
+      qf[ks][3] = validB ? *reinterpret_cast<const uint32_t*>(qb + c0 + 8) : 0u;
     }
-    const float c = p.scaleLog2;
+  };
 
-#pragma unroll
-    for (int s = 0; s < kStages - 1; s++) {
-      if (s < nBlocks) {
-        load_block<D>(sBase + s * 2 * kTileBytes, gK, kvStride, key0 + s * kBlockKeys, key1);
-        load_block<D>(sBase + s * 2 * kTileBytes + kTileBytes, gV, kvStride, key0 + s * kBlockKeys, key1);
-      }
-      cp_async_commit();
+  // Merges the four warps (each saw a disjoint quarter of the keys of every block) and stores the segment's result:
+  // the final output when `whole`, else partial `part`.
+  auto storeSegment = [&](bool whole) {
+    lA += __shfl_xor_sync(0xffffffffu, lA, 1);
+    lA += __shfl_xor_sync(0xffffffffu, lA, 2);
+    lB += __shfl_xor_sync(0xffffffffu, lB, 1);
+    lB += __shfl_xor_sync(0xffffffffu, lB, 2);
+    if (tig == 0) {
+      sM[warp * kRows + rowA] = mA;
+      sM[warp * kRows + rowB] = mB;
+      sL[warp * kRows + rowA] = lA;
+      sL[warp * kRows + rowB] = lB;
     }
-    for (int blk = 0; blk < nBlocks; blk++) {
-      {
-        const int nb = blk + kStages - 1;
-        if (nb < nBlocks) {
-          const int s = nb % kStages;
-          load_block<D>(sBase + s * 2 * kTileBytes, gK, kvStride, key0 + nb * kBlockKeys, key1);
-          load_block<D>(sBase + s * 2 * kTileBytes + kTileBytes, gV, kvStride, key0 + nb * kBlockKeys, key1);
-        }
-        cp_async_commit();
-      }
-      cp_async_wait<kStages - 1>();
-      __syncthreads();
-      const uint32_t sK = sBase + (blk % kStages) * 2 * kTileBytes;
-      const uint32_t sV = sK + kTileBytes;
-      const int kb = key0 + blk * kBlockKeys + warp * 16;  // first key of this warp's 16-key slice
-      if (kb < key1) {
-        // ---- S = Q K^T for 16 rows x 16 keys
-        float sc[2][4];
-#pragma unroll
-        for (int n = 0; n < 2; n++) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ks++) {
-          // matrices: (keys 0-7, dims lo), (keys 0-7, dims hi), (keys 8-15, dims lo), (keys 8-15, dims hi)
-          const int r = warp * 16 + (lane & 7) + ((lane >> 4) << 3);
-          const int ch = ks * 2 + ((lane >> 3) & 1);
-          uint32_t kf[4];
-          ldmatrix_x4(sK + swz<D>(r, ch), kf);
-          mma16816<kBf16>(sc[0], qf[ks], kf[0], kf[1]);
-          mma16816<kBf16>(sc[1], qf[ks], kf[2], kf[3]);
-        }
-        // ---- mask (tail of the key range, top-left causal)
-        const bool needMask = (kb + 16 > key1) || p.causal;
-        if (needMask) {
-#pragma unroll
-          for (int n = 0; n < 2; n++) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-              const int key = kb + n * 8 + 2 * tig + (e & 1);
-              const int qpos = (e < 2) ? qposA : qposB;
-              if (key >= key1 || (p.causal && key > qpos)) sc[n][e] = -INFINITY;
-            }
-          }
-        }
-        // ---- online softmax for rows g (A) and g+8 (B)
-        float mxA = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
-        float mxB = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
-        mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 1));
-        mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2));
-        mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 1));
-        mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 2));
-        const float mnA = fmaxf(mA, mxA), mnB = fmaxf(mB, mxB);
-        const float muA = (mnA == -INFINITY) ? 0.f : mnA, muB = (mnB == -INFINITY) ? 0.f : mnB;
-        const float scA = (mA == -INFINITY) ? 0.f : ex2((mA - muA) * c);
-        const float scB = (mB == -INFINITY) ? 0.f : ex2((mB - muB) * c);
-        mA = mnA;
-        mB = mnB;
-        float pA[4], pB[4];
-#pragma unroll
-        for (int n = 0; n < 2; n++) {
-          pA[n * 2 + 0] = ex2(fmaf(sc[n][0], c, -muA * c));
-          pA[n * 2 + 1] = ex2(fmaf(sc[n][1], c, -muA * c));
-          pB[n * 2 + 0] = ex2(fmaf(sc[n][2], c, -muB * c));
-          pB[n * 2 + 1] = ex2(fmaf(sc[n][3], c, -muB * c));
-        }
-        lA = lA * scA + (pA[0] + pA[1] + pA[2] + pA[3]);  // per-thread partial, reduced over the quad at the end
-        lB = lB * scB + (pB[0] + pB[1] + pB[2] + pB[3]);
-        uint32_t pf[4];
-        pf[0] = pack2<kBf16>(pA[0], pA[1]);
-        pf[1] = pack2<kBf16>(pB[0], pB[1]);
-        pf[2] = pack2<kBf16>(pA[2], pA[3]);
-        pf[3] = pack2<kBf16>(pB[2], pB[3]);
-        // ---- O = O * scale + P V
-#pragma unroll
-        for (int nt = 0; nt < kNT; nt += 2) {
-          // matrices (transposed on load): (keys 0-7, dims nt), (keys 8-15, dims nt), (keys 0-7, dims nt+1), (keys 8-15, dims nt+1)
-          const int r = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3);
-          const int ch = nt + (lane >> 4);
-          uint32_t vf[4];
-          ldmatrix_x4_trans(sV + swz<D>(r, ch), vf);
-          o[nt][0] *= scA;
-          o[nt][1] *= scA;
-          o[nt][2] *= scB;
-          o[nt][3] *= scB;
-          o[nt + 1][0] *= scA;
-          o[nt + 1][1] *= scA;
-          o[nt + 1][2] *= scB;
-          o[nt + 1][3] *= scB;
-          mma16816<kBf16>(o[nt], pf, vf[0], vf[1]);
-          mma16816<kBf16>(o[nt + 1], pf, vf[2], vf[3]);
-        }
-      }
-      __syncthreads();
-    }
-    cp_async_wait<0>();
-  }
-
-  // ---- merge the four warps (each saw a disjoint quarter of the keys) through shared memory
-  lA += __shfl_xor_sync(0xffffffffu, lA, 1);
-  lA += __shfl_xor_sync(0xffffffffu, lA, 2);
-  lB += __shfl_xor_sync(0xffffffffu, lB, 1);
-  lB += __shfl_xor_sync(0xffffffffu, lB, 2);
-  float* sO = reinterpret_cast<float*>(smem);          // [4][16][D]
-  float* sM = sO + 4 * kRows * D;                        // [4][16]
-  float* sL = sM + 4 * kRows;                            // [4][16]
-  __syncthreads();
-  if (tig == 0) {
-    sM[warp * kRows + rowA] = mA;
-    sM[warp * kRows + rowB] = mB;
-    sL[warp * kRows + rowA] = lA;
-    sL[warp * kRows + rowB] = lB;
-  }
-#pragma unroll
-  for (int nt = 0; nt < kNT; nt++) {
-    const int col = nt * 8 + 2 * tig;
-    *reinterpret_cast<float2*>(sO + (warp * kRows + rowA) * D + col) = make_float2(o[nt][0], o[nt][1]);
-    *reinterpret_cast<float2*>(sO + (warp * kRows + rowB) * D + col) = make_float2(o[nt][2], o[nt][3]);
-  }
-  __syncthreads();
-  const float c = p.scaleLog2;
-  for (int idx = threadIdx.x; idx < kRows * (D / 4); idx += kThreads) {
-    const int r = idx / (D / 4), c4 = idx % (D / 4);
-    if (r >= nRows) continue;
-    float m = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 4; w++) m = fmaxf(m, sM[w * kRows + r]);
-    float l = 0.f;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    float MA = -INFINITY, MB = -INFINITY;
 #pragma unroll
     for (int w = 0; w < 4; w++) {
-      const float mw = sM[w * kRows + r];
-      const float f = (mw == -INFINITY) ? 0.f : ex2((mw - m) * c);
-      l += sL[w * kRows + r] * f;
-      const float4 v = *reinterpret_cast<const float4*>(sO + (w * kRows + r) * D + c4 * 4);
-      acc.x += v.x * f;
-      acc.y += v.y * f;
-      acc.z += v.z * f;
-      acc.w += v.w * f;
+      MA = fmaxf(MA, sM[w * kRows + rowA]);
+      MB = fmaxf(MB, sM[w * kRows + rowB]);
     }
-    const float inv = (l > 0.f) ? (1.f / l) : 0.f;
-    acc.x *= inv;
-    acc.y *= inv;
-    acc.z *= inv;
-    acc.w *= inv;
-    const int qpos = r / p.group, head = hkv * p.group + r % p.group;
-    const long long orow = (qRow0 + qpos) * p.headsQ + head;
-    if (p.splits == 1) {
-      uint2 out;
-      out.x = pack2<kBf16>(acc.x, acc.y);
-      out.y = pack2<kBf16>(acc.z, acc.w);
-      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.O) + orow * D + c4 * 4) = out;
-    } else {
-      const long long prow = (long long)split * p.totalQ * p.headsQ + orow;
-      *reinterpret_cast<float4*>(p.partO + prow * D + c4 * 4) = acc;
-      if (c4 == 0) p.partLse[prow] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
+    const float fA = (mA == -INFINITY) ? 0.f : ex2((mA - MA) * c), fB = (mB == -INFINITY) ? 0.f : ex2((mB - MB) * c);
+#pragma unroll 1
+    for (int w = 0; w < 4; w++) {  // one warp after the other adds its share
+      if (w == warp) {
+#pragma unroll
+        for (int nt = 0; nt < kNT; nt++) {
+          float2* a = reinterpret_cast<float2*>(sO + rowA * kLdO + nt * 8 + 2 * tig);
+          float2* bq = reinterpret_cast<float2*>(sO + rowB * kLdO + nt * 8 + 2 * tig);
+          const float2 za = (w == 0) ? make_float2(0.f, 0.f) : *a, zb = (w == 0) ? make_float2(0.f, 0.f) : *bq;
+          *a = make_float2(fmaf(o[nt][0], fA, za.x), fmaf(o[nt][1], fA, za.y));
+          *bq = make_float2(fmaf(o[nt][2], fB, zb.x), fmaf(o[nt][3], fB, zb.y));
+        }
+      }
+      __syncthreads();
+    }
+    for (int idx = threadIdx.x; idx < nRows * (D / 4); idx += kThreads) {
+      const int r = idx / (D / 4), c4 = idx % (D / 4);
+      float m = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < 4; w++) m = fmaxf(m, sM[w * kRows + r]);
+      float l = 0.f;
+#pragma unroll
+      for (int w = 0; w < 4; w++) {
+        const float mw = sM[w * kRows + r];
+        l += sL[w * kRows + r] * ((mw == -INFINITY) ? 0.f : ex2((mw - m) * c));
+      }
+      const float inv = (l > 0.f) ? (1.f / l) : 0.f;
+      float4 acc = *reinterpret_cast<const float4*>(sO + r * kLdO + c4 * 4);
+      acc.x *= inv;
+      acc.y *= inv;
+      acc.z *= inv;
+      acc.w *= inv;
+      const long long orow = (qRow0 + r / p.group) * p.headsQ + hkv * p.group + r % p.group;
+      if (whole) {
+        uint2 out;
+        out.x = pack2<kBf16>(acc.x, acc.y);
+        out.y = pack2<kBf16>(acc.z, acc.w);
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.O) + orow * D + c4 * 4) = out;
+      } else {
+        const long long prow = (long long)part * p.totalQ * p.headsQ + orow;
+        *reinterpret_cast<float4*>(p.partO + prow * D + c4 * 4) = acc;
+        if (c4 == 0) p.partLse[prow] = (l == 0.f) ? -INFINITY : (m * c + log2f(l));  // NaN stays NaN
+      }
+    }
+  };
+
+  startSegment();
+  // load cursor: runs kStages - 1 blocks ahead, across segment ends
+  int ldKey = key0;
+  const uint16_t* gK = reinterpret_cast<const uint16_t*>(p.K) + kvRow0 * kvStride + (long long)hkv * D;
+  const uint16_t* gV = reinterpret_cast<const uint16_t*>(p.V) + kvRow0 * kvStride + (long long)hkv * D;
+  auto loadNext = [&](int stage) {
+    load_block<D>(sBase + stage * 2 * kTileBytes, gK, kvStride, ldKey, keyEnd);
+    load_block<D>(sBase + stage * 2 * kTileBytes + kTileBytes, gV, kvStride, ldKey, keyEnd);
+    ldKey += kBlockKeys;
+    if (even && ldKey >= keyEnd) {  // the next batch entry
+      ldKey = 0;
+      const long long step = (long long)skv * kvStride;
+      gK += step;
+      gV += step;
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < kStages - 1; s++) {
+    if (s < count) loadNext(s);
+    cp_async_commit();
+  }
+  int segStart = key0, kbase = key0;  // first key of the segment / of the block
+  for (int blk = 0; blk < count; blk++) {
+    if (blk + kStages - 1 < count) loadNext((blk + kStages - 1) % kStages);
+    cp_async_commit();
+    cp_async_wait<kStages - 1>();
+    __syncthreads();
+    const uint32_t sK = sBase + (blk % kStages) * 2 * kTileBytes;
+    const uint32_t sV = sK + kTileBytes;
+    const int kb = kbase + warp * 16;  // first key of this warp's 16-key slice
+    if (kb < keyEnd) {
+      // ---- S = Q K^T for 16 rows x 16 keys
+      float sc[2][4];
+#pragma unroll
+      for (int n = 0; n < 2; n++) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < D / 16; ks++) {
+        // matrices: (keys 0-7, dims lo), (keys 0-7, dims hi), (keys 8-15, dims lo), (keys 8-15, dims hi)
+        const int r = warp * 16 + (lane & 7) + ((lane >> 4) << 3);
+        const int ch = ks * 2 + ((lane >> 3) & 1);
+        uint32_t kf[4];
+        ldmatrix_x4(sK + swz<D>(r, ch), kf);
+        mma16816<kBf16>(sc[0], qf[ks], kf[0], kf[1]);
+        mma16816<kBf16>(sc[1], qf[ks], kf[2], kf[3]);
+      }
+      // ---- mask (tail of the key range, top-left causal)
+      const bool needMask = (kb + 16 > keyEnd) || p.causal;
+      if (needMask) {
+#pragma unroll
+        for (int n = 0; n < 2; n++) {
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const int key = kb + n * 8 + 2 * tig + (e & 1);
+            const int qpos = (e < 2) ? qposA : qposB;
+            if (key >= keyEnd || (p.causal && key > qpos)) sc[n][e] = -INFINITY;
+          }
+        }
+      }
+      // ---- online softmax for rows g (A) and g+8 (B)
+      float mxA = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1]));
+      float mxB = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
+      mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 1));
+      mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2));
+      mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 1));
+      mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 2));
+      const float mnA = fmaxf(mA, mxA), mnB = fmaxf(mB, mxB);
+      const float muA = (mnA == -INFINITY) ? 0.f : mnA, muB = (mnB == -INFINITY) ? 0.f : mnB;
+      const float scA = (mA == -INFINITY) ? 0.f : ex2((mA - muA) * c);
+      const float scB = (mB == -INFINITY) ? 0.f : ex2((mB - muB) * c);
+      mA = mnA;
+      mB = mnB;
+      float pA[4], pB[4];
+#pragma unroll
+      for (int n = 0; n < 2; n++) {
+        pA[n * 2 + 0] = ex2(fmaf(sc[n][0], c, -muA * c));
+        pA[n * 2 + 1] = ex2(fmaf(sc[n][1], c, -muA * c));
+        pB[n * 2 + 0] = ex2(fmaf(sc[n][2], c, -muB * c));
+        pB[n * 2 + 1] = ex2(fmaf(sc[n][3], c, -muB * c));
+      }
+      lA = lA * scA + (pA[0] + pA[1] + pA[2] + pA[3]);  // per-thread partial, reduced over the quad at the end
+      lB = lB * scB + (pB[0] + pB[1] + pB[2] + pB[3]);
+      uint32_t pf[4];
+      pf[0] = pack2<kBf16>(pA[0], pA[1]);
+      pf[1] = pack2<kBf16>(pB[0], pB[1]);
+      pf[2] = pack2<kBf16>(pA[2], pA[3]);
+      pf[3] = pack2<kBf16>(pB[2], pB[3]);
+      // ---- O = O * scale + P V
+#pragma unroll
+      for (int nt = 0; nt < kNT; nt += 2) {
+        // matrices (transposed on load): (keys 0-7, dims nt), (keys 8-15, dims nt), (keys 0-7, dims nt+1), (keys 8-15, dims nt+1)
+        const int r = warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3);
+        const int ch = nt + (lane >> 4);
+        uint32_t vf[4];
+        ldmatrix_x4_trans(sV + swz<D>(r, ch), vf);
+        o[nt][0] *= scA;
+        o[nt][1] *= scA;
+        o[nt][2] *= scB;
+        o[nt][3] *= scB;
+        o[nt + 1][0] *= scA;
+        o[nt + 1][1] *= scA;
+        o[nt + 1][2] *= scB;
+        o[nt + 1][3] *= scB;
+        mma16816<kBf16>(o[nt], pf, vf[0], vf[1]);
+        mma16816<kBf16>(o[nt + 1], pf, vf[2], vf[3]);
+      }
+    }
+    __syncthreads();
+    kbase += kBlockKeys;
+    const bool entryDone = even && kbase >= keyEnd;
+    if (entryDone || blk + 1 == count) {
+      storeSegment(even ? (entryDone && segStart == 0) : p.splits == 1);
+      if (blk + 1 < count) {  // on to the next batch entry, whose blocks are already on their way
+        qRow0 += sq;
+        segStart = kbase = 0;
+        part = 0;
+        startSegment();
+      }
     }
   }
+  cp_async_wait<0>();
+  if (count == 0) storeSegment(p.splits == 1);  // a split without keys (never in an even partition): zeros, lse = -inf
 }
 
-// O[row] = sum_s 2^(lse_s - M) O_s / sum_s 2^(lse_s - M); one thread per 4 output elements.
+// O[row] = sum_s 2^(lse_s - M) O_s / sum_s 2^(lse_s - M), one CTA per output row.  Bound by the latency of two dependent
+// reads (the partials' log-sum-exps, the partials), so both are spread over the CTA: every warp reads all lse of the row,
+// D / 4 threads read one split's partial row and 128 / (D / 4) such groups take turns over the splits, four in flight each.
+// The kernel is launched while the split kernel still runs and waits for its end with griddepcontrol.wait.
+constexpr int kCombineThreads = 128;
 template <int D, bool kBf16>
-__global__ void combine_kernel(const float* __restrict__ partO, const float* __restrict__ partLse, void* O,
-                               long long rows /* totalQ * Hq */, int splits, const int* cuQ, const int* cuKV, int batch,
-                               int headsQ) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= rows * (D / 4)) return;
-  const long long row = idx / (D / 4);
-  const int c4 = (int)(idx % (D / 4));
+__global__ void __launch_bounds__(kCombineThreads)
+combine_kernel(const float* __restrict__ partO, const float* __restrict__ partLse, void* O,
+               long long rows /* totalQ * Hq */, int splits, const int* cuQ, int batch, int headsQ, int runs,
+               int blocksPerEntry, long long totalBlocks, int seqLenQ) {
+  constexpr int kVec = D / 4, kGroups = kCombineThreads / kVec;
+  __shared__ float4 sAcc[kGroups][kVec];
+  __shared__ float sSum[kGroups];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const long long row = blockIdx.x;
   // packed input: rows past the last sequence (a Q tensor longer than cu_seqlens_q[batch]) have no partials
   if (cuQ != nullptr && row / headsQ >= cuQ[batch]) return;
-  float M = -INFINITY;
-  for (int s = 0; s < splits; s++) M = fmaxf(M, partLse[(long long)s * rows + row]);
-  if (M == -INFINITY) return;  // no keys at all for this row: leave O untouched
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  float wsum = 0.f;
-  for (int s = 0; s < splits; s++) {
-    const float lse = partLse[(long long)s * rows + row];
-    if (lse == -INFINITY) continue;
-    const float w = exp2f(lse - M);
-    const float4 v = *reinterpret_cast<const float4*>(partO + ((long long)s * rows + row) * D + c4 * 4);
-    acc.x += w * v.x;
-    acc.y += w * v.y;
-    acc.z += w * v.z;
-    acc.w += w * v.w;
-    wsum += w;
+  if (runs > 0) {  // even partition: how many runs touch this row's batch entry
+    const long long first = row / headsQ / seqLenQ * blocksPerEntry;
+    splits = run_of_block(first + blocksPerEntry - 1, totalBlocks, runs) - run_of_block(first, totalBlocks, runs) + 1;
+    if (splits == 1) return;  // the split kernel has written the output
   }
-  const float inv = 1.f / wsum;
-  uint2 out;
-  out.x = pack2<kBf16>(acc.x * inv, acc.y * inv);
-  out.y = pack2<kBf16>(acc.z * inv, acc.w * inv);
-  *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(O) + row * D + c4 * 4) = out;
-  (void)cuKV;
+  float M = -INFINITY;
+  for (int s = threadIdx.x & 31; s < splits; s += 32) M = fmax_nan(M, partLse[(long long)s * rows + row]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) M = fmax_nan(M, __shfl_xor_sync(0xffffffffu, M, off));
+  if (M == -INFINITY) return;  // no keys at all for this row: leave O untouched
+  const int g = threadIdx.x / kVec, c4 = threadIdx.x % kVec;
+  if (g < kGroups) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float wsum = 0.f;
+#pragma unroll 4
+    for (int s = g; s < splits; s += kGroups) {
+      const float lse = partLse[(long long)s * rows + row];
+      const float4 v = *reinterpret_cast<const float4*>(partO + ((long long)s * rows + row) * D + c4 * 4);
+      const float w = exp2f(lse - M);  // 0 for a split without keys, whose partial is zero
+      acc.x += w * v.x;
+      acc.y += w * v.y;
+      acc.z += w * v.z;
+      acc.w += w * v.w;
+      wsum += w;
+    }
+    sAcc[g][c4] = acc;
+    if (c4 == 0) sSum[g] = wsum;
+  }
+  __syncthreads();
+  if (threadIdx.x < kVec) {
+    float4 acc = sAcc[0][threadIdx.x];
+    float wsum = sSum[0];
+#pragma unroll
+    for (int i = 1; i < kGroups; i++) {
+      const float4 v = sAcc[i][threadIdx.x];
+      acc.x += v.x;
+      acc.y += v.y;
+      acc.z += v.z;
+      acc.w += v.w;
+      wsum += sSum[i];
+    }
+    const float inv = 1.f / wsum;
+    uint2 out;
+    out.x = pack2<kBf16>(acc.x * inv, acc.y * inv);
+    out.y = pack2<kBf16>(acc.z * inv, acc.w * inv);
+    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(O) + row * D + threadIdx.x * 4) = out;
+  }
 }
 
+constexpr int smem_bytes(int D) { return kStages * 2 * kBlockKeys * D * 2 + (kRows * (D + 8) + 8 * kRows) * (int)sizeof(float); }
+// CTAs of the even partition, in quarters of an SM's share.  Not all that shared memory holds where it holds more than
+// one: measured us at 8 KV heads, batch 4 / 8 / 28 of D = 128: 296 CTAs 93.2 / 110.6 / 114.4, 280 89.3 / 106.0 / 112.1, 256
+// 86.8 / 102.6 / 108.3, 224 88.5 / 105.1 / 106.6, 148 107 / 125 / 137; D = 64, batch 4 / 24: 592 49.9 / 72.8, 444 46.8 / 66.8,
+// 296 46.8 / 68.0; D = 32: 592 47.3, 444 50.4, 296 58.6; D = 96: 296 44.2, 256 44.5; D = 192 / 256 hold one per SM.
+constexpr int quarter_ctas_per_sm(int D) { return D == 32 ? 16 : D == 64 ? 12 : D <= 128 ? 7 : 4; }
+
 template <int D, bool kBf16>
-int launch(const FwdProblem& pr, int splits, float* partO, float* partLse) {
-  constexpr int kTileBytes = kBlockKeys * D * 2;
-  constexpr int kPipeBytes = kStages * 2 * kTileBytes;
-  constexpr int kMergeBytes = (4 * kRows * D + 8 * kRows) * (int)sizeof(float);
-  constexpr int kSmem = kPipeBytes > kMergeBytes ? kPipeBytes : kMergeBytes;
+int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* partLse) {
+  constexpr int kSmem = smem_bytes(D);
+  static_assert(kSmem <= 227 * 1024 && merge_ld<D>() == D + 8, "shared memory");
   auto kernel = fwd_splitkv_kernel<D, kBf16>;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return kCudaError;
@@ -435,20 +547,30 @@ int launch(const FwdProblem& pr, int splits, float* partO, float* partLse) {
   p.headsKV = pr.headsKV;
   p.group = pr.headsQ / pr.headsKV;
   p.causal = pr.causal;
-  p.splits = splits;
+  p.splits = plan.splits;
+  p.runs = plan.runs;
+  p.blocksPerEntry = plan.blocksPerEntry;
+  p.totalBlocks = (long long)plan.blocksPerEntry * pr.batch;
   const int blocks = (pr.seqLenKV + kBlockKeys - 1) / kBlockKeys;
-  p.keysPerSplit = ((blocks + splits - 1) / splits) * kBlockKeys;
+  p.keysPerSplit = ((blocks + plan.splits - 1) / plan.splits) * kBlockKeys;
   p.totalQ = pr.totalQ;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
-  dim3 grid((unsigned)splits, (unsigned)pr.headsKV, (unsigned)pr.batch);
+  const dim3 grid = plan.runs > 0 ? dim3((unsigned)(plan.runs * pr.headsKV)) : dim3((unsigned)plan.splits, (unsigned)pr.headsKV, (unsigned)pr.batch);
   kernel<<<grid, kThreads, kSmem, pr.stream>>>(p);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess && splits > 1) {
+  if (e == cudaSuccess && plan.splits > 1) {
     const long long rows = pr.totalQ * pr.headsQ;
-    const long long threads = rows * (D / 4);
-    combine_kernel<D, kBf16><<<(unsigned)((threads + 255) / 256), 256, 0, pr.stream>>>(
-        partO, partLse, pr.O, rows, splits, pr.cuQ, pr.cuKV, pr.batch, pr.headsQ);
-    e = cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)rows);
+    cfg.blockDim = dim3(kCombineThreads);
+    cfg.stream = pr.stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, combine_kernel<D, kBf16>, (const float*)partO, (const float*)partLse, pr.O, rows, plan.splits,
+                           pr.cuQ, pr.batch, pr.headsQ, p.runs, p.blocksPerEntry, p.totalBlocks, pr.seqLenQ);
   }
   if (e != cudaSuccess) {
     set_error_string("split-KV kernel launch failed: %s", cudaGetErrorString(e));
@@ -466,43 +588,61 @@ bool splitkv_applicable(const FwdProblem& p) {
   return (long long)p.seqLenQ * group <= decode::kRows && p.seqLenKV >= 256;
 }
 
-// Number of key-range splits.  The kernel runs two CTAs per SM; what costs time is a grid that is slightly larger than
-// a whole number of such waves (batch 8 x 8 KV heads with 5 splits = 320 CTAs on 296 slots: 256 us, with 4 or 8
-// splits 190 us), while splitting itself costs 20-25 % in partials and the combine pass once there are enough
-// (batch, KV head) pairs to fill the GPU without it (batch 64: 7.1 TB/s unsplit, 6.8 with 2-4 splits).  So: no split
-// from one full wave of pairs on, otherwise as many splits as fit two waves exactly or just under, at most 32
-// (measured at 32768 keys, 8 KV heads, batch 1 / 4 / 8 / 16: 60 / 121 / 196 / 331 us; best seen 60 / 114 / 188 / 331),
-// at least 256 keys per split.
-int splitkv_num_splits(const FwdProblem& p, int numSMs) {
-  const long long base = (long long)p.batch * p.headsKV;
-  const long long slots = 2LL * numSMs;
-  if (base >= slots) return 1;
-  long long splits = (2 * slots) / base;
-  if (splits > 32) splits = 32;
-  const long long maxSplits = (p.seqLenKV + 255) / 256;
-  if (splits > maxSplits) splits = maxSplits;
-  if (splits < 1) splits = 1;
-  return (int)splits;
+// How a call is cut.  forced > 0: that many key-range splits of every pair, on a three-dimensional grid; the same with
+// a number of its own for packed input, whose lengths the host does not know.  Fixed-length input is cut evenly: the key
+// blocks of all batch entries in a row, as many equal runs as the GPU holds at once, so that no SM waits for another at the
+// end whatever the batch is.  All KV heads of a run are cut at the same keys: cut one by one, their CTAs drift apart and
+// read the pieces of a row of K at different times, which cost up to half of the bandwidth (D = 32, 64-byte pieces).
+SplitPlan splitkv_plan(const FwdProblem& p, int numSMs, int forced) {
+  SplitPlan plan = {1, 0, 0};
+  const long long pairs = (long long)p.batch * p.headsKV;
+  const int maxSplits = (p.seqLenKV + decode::kBlockKeys - 1) / decode::kBlockKeys;
+  if (forced > 0) {
+    plan.splits = forced < maxSplits ? forced : maxSplits;
+    return plan;
+  }
+  const int seen = p.causal ? (p.seqLenQ < p.seqLenKV ? p.seqLenQ : p.seqLenKV) : p.seqLenKV;
+  const long long blocks = (seen + decode::kBlockKeys - 1) / decode::kBlockKeys;
+  const long long slots = (long long)numSMs * decode::quarter_ctas_per_sm(p.headDim) / 4;
+  if (p.cuQ == nullptr && blocks >= 4 && pairs < 8 * slots && p.headsKV <= slots) {
+    const long long total = p.batch * blocks;
+    long long runs = total / 4 > p.batch ? total / 4 : p.batch;  // a run has at least four blocks, an entry at least one run
+    if (runs > slots / p.headsKV) runs = slots / p.headsKV;
+    plan.runs = (int)runs;
+    plan.blocksPerEntry = (int)blocks;
+    const long long run = total / runs;  // the shortest run; partial results per pair:
+    plan.splits = (int)(runs % p.batch == 0 ? runs / p.batch : (blocks - 2) / run + 2);
+    return plan;
+  }
+  // packed input (and more pairs than the even partition is for): no split from one wave of pairs on, otherwise as many
+  // as fit two waves of two CTAs per SM, at most 32, at least 256 keys each
+  if (pairs < 2ll * numSMs) {
+    long long splits = 4ll * numSMs / pairs;
+    if (splits > 32) splits = 32;
+    if (splits > (p.seqLenKV + 255) / 256) splits = (p.seqLenKV + 255) / 256;
+    plan.splits = splits < 1 ? 1 : (int)splits;
+  }
+  return plan;
 }
 
-size_t splitkv_scratch_floats(const FwdProblem& p, int splits) {
-  if (splits <= 1) return 0;
+size_t splitkv_scratch_floats(const FwdProblem& p, const SplitPlan& plan) {
+  if (plan.splits <= 1) return 0;
   const size_t rows = (size_t)p.totalQ * p.headsQ;
-  return (size_t)splits * rows * (p.headDim + 1);
+  return (size_t)plan.splits * rows * (p.headDim + 1);
 }
 
 // partO = scratch, partLse = scratch + splits*rows*D
-int launch_fwd_splitkv(const FwdProblem& p, int splits, float* scratch) {
+int launch_fwd_splitkv(const FwdProblem& p, const SplitPlan& plan, float* scratch) {
   const size_t rows = (size_t)p.totalQ * p.headsQ;
   float* partO = scratch;
-  float* partLse = scratch ? scratch + (size_t)splits * rows * p.headDim : nullptr;
+  float* partLse = scratch ? scratch + (size_t)plan.splits * rows * p.headDim : nullptr;
   const bool bf = (p.dtype == kBf16);
 #define TFA_DECODE_CASE(D)                                                                   \
   case D:                                                                                    \
     if (bf) {                                                                                \
-      if constexpr (TFA_HAVE_BF16) return decode::launch<D, true>(p, splits, partO, partLse);  \
+      if constexpr (TFA_HAVE_BF16) return decode::launch<D, true>(p, plan, partO, partLse);  \
     } else {                                                                                 \
-      if constexpr (TFA_HAVE_FP16) return decode::launch<D, false>(p, splits, partO, partLse); \
+      if constexpr (TFA_HAVE_FP16) return decode::launch<D, false>(p, plan, partO, partLse); \
     }                                                                                        \
     return kBadDtype;
   (void)bf; (void)partO; (void)partLse;
@@ -608,19 +748,21 @@ extern "C" int tfa_b200_fwd_decode_noalloc(const void* Q, const void* K, const v
   }
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  int splits = (numSplits > 0) ? numSplits : splitkv_num_splits(p, sms);
-  const int maxSplits = (seqLenKV + decode::kBlockKeys - 1) / decode::kBlockKeys;
-  if (splits > maxSplits) splits = maxSplits;
-  const size_t need = splitkv_scratch_floats(p, splits);
+  SplitPlan plan = splitkv_plan(p, sms, numSplits);
+  if (plan.runs > 0 && splitkv_scratch_floats(p, plan) > (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS) {
+    // the even partition's partials do not fit: whole pairs, as many at a time as the GPU holds
+    plan = SplitPlan{1, 0, 0};
+  }
+  const size_t need = splitkv_scratch_floats(p, plan);
   if (need > (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS) {
     set_error_string("split-KV partials need %zu floats (%d splits x %lld rows x (%d + 1)) but the built-in scratch holds "
                      "%zu; use fewer splits or tfa_b200_fwd",
-                     need, splits, (long long)p.totalQ * numHeadsQ, headDim, (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS);
+                     need, plan.splits, (long long)p.totalQ * numHeadsQ, headDim, (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS);
     return kTooLarge;
   }
   float* scratch = nullptr;
   if ((rc = decode::static_scratch_ptr(&scratch)) != kOk) return rc;
   // Every (split, row) partial that the combine kernel reads is written by the split kernel of the same call, so
   // nothing in the array has to start at zero and contents left by an earlier call are never consumed.
-  return launch_fwd_splitkv(p, splits, need > 0 ? scratch : nullptr);
+  return launch_fwd_splitkv(p, plan, need > 0 ? scratch : nullptr);
 }

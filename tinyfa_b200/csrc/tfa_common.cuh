@@ -50,6 +50,14 @@ struct FwdProblem {
   int gateEpoch = 0;
 };
 
+// How the split-KV path cuts a call (fwd_decode.cu): `runs` equal runs over the key blocks of all batch entries, or, with
+// runs == 0, `splits` key ranges of every (batch, KV head) pair.  splits is the largest number of partial results of a pair.
+struct SplitPlan {
+  int splits;
+  int runs;
+  int blocksPerEntry;
+};
+
 // The device status word holds 0, or (launch epoch << 8) | site code once a bounded wait inside a kernel gave up.
 
 int launch_fwd_fp32(const FwdProblem& p);    // fp32: CUDA-core FMA kernel
