@@ -12,8 +12,9 @@
  * Streams and CUDA graphs: the first call on a device creates a few KB of per-device state (a status word, work
  * counters and tensor-map slots, shared-memory opt-in of the kernels, a scratch pool) with synchronous calls; make it
  * outside a stream capture.  After that a forward call only enqueues kernels on `stream` (the split-KV path of
- * tfa_b200_fwd and eager fp32 calls also a stream-ordered allocation and free; tfa_b200_fwd_decode_noalloc none), so it can be captured
- * into a CUDA graph and replayed.  The persistent kernel hands out its work through a pair of device counters that two
+ * tfa_b200_fwd, and eager calls in fp32 or with key ranges, also a stream-ordered allocation and free;
+ * tfa_b200_fwd_decode_noalloc none), so it can be captured into a CUDA graph and replayed.  The persistent kernel hands
+ * out its work through a pair of device counters that two
  * launches must not use at the same time: eager launches take the pair of their stream (up to 1024 distinct streams
  * per device; the per-thread default stream counts once per calling thread), every captured launch takes a pair of
  * its own for good (up to 3072 per device), past either limit the call returns TFA_B200_TOO_LARGE.  So eager launches
@@ -88,6 +89,9 @@ int tfa_b200_device_status(int* site);
  *   "pack_gqa" -1/0/1  interleave the Q heads of a KV group into one 128-row tile: auto (short query blocks and
  *                      causal problems) / never / always
  *   "split_kv" -1/0/n  split-KV path for short query blocks (seqQ * group <= 16): auto / never / exactly n splits
+ *   "split_tc" -1/0/n  tensor-core path, fixed-length input: every query tile's keys cut into n ranges whose partial results
+ *                      a second kernel combines: auto (few query tiles for long keys) / never / n ranges.  Not under
+ *                      stream capture.
  *   "narrow_mma" 0/1   head dims 32 / 96: MMAs of the padded width (64 / 128) / MMAs shaped for the head dim (the default)
  *   "solo64" 0/1       head dims 32 / 64: two-tile CTAs, one per SM / one-tile CTAs, two per SM (the default)
  *   "fp32_t8" 0/1/2    fp32, head dim 128: 4 x 8 thread tiles always / 8 x 8 thread tiles for problems of at least three

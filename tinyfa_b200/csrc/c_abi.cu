@@ -26,14 +26,14 @@ namespace tfa_b200 {
 // ---- instantiations (fwd_tc_inst.cu, one object per pair)
 // Only the (padded head dim, dtype) pairs selected at build time exist as objects.
 #define TFA_DECLARE_TC(HDP)                                                               \
-  int launch_fwd_tc_hdp##HDP##_bf0(const FwdProblem&, int);                               \
-  int launch_fwd_tc_hdp##HDP##_bf1(const FwdProblem&, int);                               \
-  static inline int tc_call_hdp##HDP(const FwdProblem& p, int packShift, bool bf16) {     \
-    (void)p; (void)packShift;                                                             \
+  int launch_fwd_tc_hdp##HDP##_bf0(const FwdProblem&, int, const TcSplit&);               \
+  int launch_fwd_tc_hdp##HDP##_bf1(const FwdProblem&, int, const TcSplit&);               \
+  static inline int tc_call_hdp##HDP(const FwdProblem& p, int packShift, const TcSplit& split, bool bf16) { \
+    (void)p; (void)packShift; (void)split;                                                \
     if (bf16) {                                                                           \
-      if constexpr (TFA_HAVE_BF16) return launch_fwd_tc_hdp##HDP##_bf1(p, packShift);     \
+      if constexpr (TFA_HAVE_BF16) return launch_fwd_tc_hdp##HDP##_bf1(p, packShift, split); \
     } else {                                                                              \
-      if constexpr (TFA_HAVE_FP16) return launch_fwd_tc_hdp##HDP##_bf0(p, packShift);     \
+      if constexpr (TFA_HAVE_FP16) return launch_fwd_tc_hdp##HDP##_bf0(p, packShift, split); \
     }                                                                                     \
     return kBadDtype;                                                                     \
   }
@@ -56,6 +56,7 @@ bool splitkv_applicable(const FwdProblem& p);
 SplitPlan splitkv_plan(const FwdProblem& p, int numSMs, int forced);
 size_t splitkv_scratch_floats(const FwdProblem& p, const SplitPlan& plan);
 int launch_fwd_splitkv(const FwdProblem& p, const SplitPlan& plan, float* scratch);
+int launch_combine_parts(const FwdProblem& p, int packShift, const TcSplit& split);
 
 // ---- fp32 on the tensor cores (fwd_fp32_tc.cu)
 bool fp32tc_applicable(const FwdProblem& p, int option);
@@ -85,6 +86,7 @@ static std::atomic<int> g_optPairCta{-1};  // head dims 192 / 256, fixed length:
 int option_pair_cta() { return g_optPairCta.load(); }
 static std::atomic<int> g_optFp32T8{1};  // fp32, head dim 128, large problems: the 8 x 8 thread-tile form
 int option_fp32_t8() { return g_optFp32T8.load(); }
+static std::atomic<int> g_optSplitTc{-1};  // tensor-core path, key ranges: -1 by size, 0 never, n > 0 exactly n
 static std::atomic<int> g_optFp32Tc{-1};  // fp32 on the tensor cores: -1 by size, 0 never, 1 wherever it applies
 
 int next_epoch() { return (g_epoch.fetch_add(1) & 0x7FFFFF) + 1; }
@@ -395,38 +397,32 @@ static int dispatch_fp32(const FwdProblem& p) {
   return rc;
 }
 
-static int dispatch(const FwdProblem& p) {
-  if (p.dtype == kFp32) return dispatch_fp32(p);
-  const int optSplit = g_optSplitKv.load();
-  if (optSplit != 0 && p.totalQ >= 0 && splitkv_applicable(p)) {
-    return dispatch_splitkv(p, splitkv_plan(p, num_sms(), optSplit));
-  }
+static int run_tc(const FwdProblem& p, int ps, const TcSplit& split) {
   const bool bf = (p.dtype == kBf16);
-  const int ps = pick_pack_shift(p);
   switch (p.headDim) {
     case 32:
     case 64:
 #if TFA_HAVE_HDP64
-      return tc_call_hdp64(p, ps, bf);
+      return tc_call_hdp64(p, ps, split, bf);
 #else
       break;
 #endif
     case 96:
     case 128:
 #if TFA_HAVE_HDP128
-      return tc_call_hdp128(p, ps, bf);
+      return tc_call_hdp128(p, ps, split, bf);
 #else
       break;
 #endif
     case 192:
 #if TFA_HAVE_HDP192
-      return tc_call_hdp192(p, ps, bf);
+      return tc_call_hdp192(p, ps, split, bf);
 #else
       break;
 #endif
     case 256:
 #if TFA_HAVE_HDP256
-      return tc_call_hdp256(p, ps, bf);
+      return tc_call_hdp256(p, ps, split, bf);
 #else
       break;
 #endif
@@ -434,8 +430,95 @@ static int dispatch(const FwdProblem& p) {
       return kBadHeadDim;
   }
   (void)ps;
+  (void)split;
   (void)bf;
   return not_compiled(p);
+}
+
+// Number of key ranges for a call with few query tiles for its key length (or, causal, with few heavy ones), from a model of
+// its time: key blocks on the longest path x the time of a block, against 5 us for the combine kernel and the partial
+// results' way to memory and back.  us per 128-key block, measured: 1.1 at head dims 32 / 64, 1.75 at 96 / 128, 1.6 at 192, 2.35
+// at 256 (1.4 in the pair form, which key ranges do not have).  What it decides, us per call whole -> in ranges: 2 x 8 rows x
+// 12289 keys, 32 over 8 heads of 128 152 -> 36, 1 x 8 x 32768 386 -> 45, 1 x 512 x 2048 16 heads 38 -> 30, causal 1 x 2048 4 heads
+// 38 -> 29; left whole: 1 x 1024 x 1024 8 heads 25.2 (27.1 in four), causal 1 x 2048 4 heads of 256 34 (39 in two).
+static TcSplit tc_split_plan(const FwdProblem& p, int packShift) {
+  TcSplit s;
+  const int opt = g_optSplitTc.load();
+  if (opt == 0 || p.cuQ != nullptr || !dtype_compiled(p.dtype) || !head_dim_compiled(p.headDim)) return s;
+  const int rowsPerItem = (p.headDim == 96 || p.headDim == 128 ? 2 : 1) * (128 >> packShift);
+  const long long items = (long long)((p.seqLenQ + rowsPerItem - 1) / rowsPerItem) * (p.headsQ >> packShift) * p.batch;
+  const long long slots = (long long)num_sms() * (p.headDim <= 64 ? 2 : 1);
+  const int seen = p.causal ? (p.seqLenQ < p.seqLenKV ? p.seqLenQ : p.seqLenKV) : p.seqLenKV;
+  const int blocks = (seen + 127) / 128;
+  long long parts = opt;
+  if (opt < 0) {
+    if (blocks < 8 || items >= 2 * slots) return s;  // enough items for every SM, or nothing to cut
+    const double usBlock = p.headDim <= 64 ? 1.1 : p.headDim <= 128 ? 1.75 : p.headDim == 192 ? 1.6 : 2.35;
+    const double usWhole = (p.headDim == 256 && p.seqLenQ > (128 >> packShift)) ? 1.4 : usBlock;
+    const double usPart = (double)p.totalQ * p.headsQ * p.headDim * 8.0 / 3.3e6;  // write and read one part, 3.3 TB/s
+    // mean key blocks of an item
+    const double sq = p.seqLenQ, skv = p.seqLenKV;
+    const double mean = !p.causal ? blocks : 0.5 + (sq <= skv ? sq * 0.5 : skv - skv * skv * 0.5 / sq) / 128.0;
+    const double share = items * mean / slots;  // key blocks per CTA slot when spread evenly
+    double best = 0.0;
+    for (int n = 1; n <= 32 && n <= blocks; n++) {
+      const int len = (blocks + n - 1) / n;
+      // equal pieces run in whole waves; causal ones of different lengths pack, with half a piece idle at the end
+      const long long waves = (items * n + slots - 1) / slots;
+      const double path = !p.causal ? (double)waves * len : (share + 0.5 * len > len ? share + 0.5 * len : len);
+      const double us = path * (n == 1 ? usWhole : usBlock) + (n == 1 ? 0.0 : 5.0 + n * usPart * (p.causal ? 0.6 : 1.0));
+      if (n == 1) {
+        best = us * 0.9 - 1.0;  // ranges have to gain a tenth and a microsecond
+        parts = 1;
+      } else if (us < best) {
+        best = us;
+        parts = n;
+      }
+    }
+  }
+  if (parts > blocks) parts = blocks;
+  if (parts < 2) return s;
+  s.partBlocks = (int)((blocks + parts - 1) / parts);
+  s.parts = (blocks + s.partBlocks - 1) / s.partBlocks;
+  return s;
+}
+
+// The tensor-core path.  Key ranges need scratch for their partial results: like the fp32 workspace they are not used
+// under stream capture (these calls capture as one kernel without an allocation), and without scratch the call runs whole.
+static int dispatch_tc(const FwdProblem& p) {
+  const int ps = pick_pack_shift(p);
+  TcSplit split = tc_split_plan(p, ps);
+  if (split.parts > 1) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    int device = 0;
+    if (cudaStreamIsCapturing(p.stream, &cap) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
+      set_error_string("cudaStreamIsCapturing: %s", cudaGetErrorString(cudaGetLastError()));
+      return kCudaError;
+    }
+    const size_t rows = (size_t)p.totalQ * p.headsQ;
+    cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? scratch_pool(device) : nullptr;
+    float* scratch = nullptr;
+    if (pool != nullptr && cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), split.parts * rows * (p.headDim + 1) * sizeof(float),
+                                                   pool, p.stream) == cudaSuccess) {
+      split.partO = scratch;
+      split.partLse = scratch + split.parts * rows * p.headDim;
+      int rc = run_tc(p, ps, split);
+      if (rc == kOk) rc = launch_combine_parts(p, ps, split);
+      cudaFreeAsync(scratch, p.stream);
+      return rc;
+    }
+    (void)cudaGetLastError();
+  }
+  return run_tc(p, ps, TcSplit());
+}
+
+static int dispatch(const FwdProblem& p) {
+  if (p.dtype == kFp32) return dispatch_fp32(p);
+  const int optSplit = g_optSplitKv.load();
+  if (optSplit != 0 && p.totalQ >= 0 && splitkv_applicable(p)) {
+    return dispatch_splitkv(p, splitkv_plan(p, num_sms(), optSplit));
+  }
+  return dispatch_tc(p);
 }
 
 int validate_common(const void* Q, const void* K, const void* V, void* O, int dtype, int batch, int sq, int skv,
@@ -608,6 +691,10 @@ extern "C" int tfa_b200_set_option(const char* name, int value) {
   }
   if (strcmp(name, "fp32_t8") == 0) {
     g_optFp32T8.store(value < 0 ? 1 : (value > 2 ? 2 : value));
+    return kOk;
+  }
+  if (strcmp(name, "split_tc") == 0) {
+    g_optSplitTc.store(value < 0 ? -1 : value);
     return kOk;
   }
   if (strcmp(name, "fp32_tc") == 0) {

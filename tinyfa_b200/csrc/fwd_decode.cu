@@ -509,6 +509,68 @@ combine_kernel(const float* __restrict__ partO, const float* __restrict__ partLs
   }
 }
 
+// Partial results of the tensor-core kernel's key ranges (kModeFixedSplit), many rows and few ranges: D / 4 threads per
+// row, several rows per CTA.
+template <int D, bool kBf16>
+__global__ void __launch_bounds__(kCombineThreads)
+combine_parts_kernel(const float* __restrict__ partO, const float* __restrict__ partLse, void* O, long long rows, int partBlocks,
+                     int seqLenQ, int seqLenKV, int headsQ, int causal, int rowsPerTile) {
+  constexpr int kVec = D / 4, kGroups = kCombineThreads / kVec;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int g = threadIdx.x / kVec, c4 = threadIdx.x % kVec;
+  const long long row = (long long)blockIdx.x * kGroups + g;
+  if (g >= kGroups || row >= rows) return;
+  int blocks = (seqLenKV + 127) / 128;
+  if (causal) {  // key blocks of this row's query tile, as in make_work
+    const int tile = (int)(row / headsQ % seqLenQ) / rowsPerTile;
+    blocks = min(blocks, (min((tile + 1) * rowsPerTile, seqLenQ) + 127) / 128);
+  }
+  const int parts = (blocks + partBlocks - 1) / partBlocks;
+  if (parts == 1) return;  // the attention kernel has written the output
+  float M = -INFINITY;
+#pragma unroll 8
+  for (int s = 0; s < parts; s++) M = fmax_nan(M, partLse[s * rows + row]);
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float wsum = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < parts; s++) {
+    const float4 v = *reinterpret_cast<const float4*>(partO + (s * rows + row) * D + c4 * 4);
+    const float w = exp2f(partLse[s * rows + row] - M);  // part 0 holds key 0, which every row sees: M is not -inf
+    acc.x += w * v.x;
+    acc.y += w * v.y;
+    acc.z += w * v.z;
+    acc.w += w * v.w;
+    wsum += w;
+  }
+  const float inv = 1.f / wsum;
+  uint2 out;
+  out.x = pack2<kBf16>(acc.x * inv, acc.y * inv);
+  out.y = pack2<kBf16>(acc.z * inv, acc.w * inv);
+  *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(O) + row * D + c4 * 4) = out;
+}
+
+template <int D, bool kBf16>
+int launch_combine(const FwdProblem& p, int packShift, const TcSplit& split) {
+  constexpr int kGroups = kCombineThreads / (D / 4);
+  const long long rows = p.totalQ * p.headsQ;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)((rows + kGroups - 1) / kGroups));
+  cfg.blockDim = dim3(kCombineThreads);
+  cfg.stream = p.stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, combine_parts_kernel<D, kBf16>, (const float*)split.partO, (const float*)split.partLse,
+                                           p.O, rows, split.partBlocks, p.seqLenQ, p.seqLenKV, p.headsQ, p.causal, 128 >> packShift);
+  if (e != cudaSuccess) {
+    set_error_string("combine kernel launch failed: %s", cudaGetErrorString(e));
+    return kCudaError;
+  }
+  return kOk;
+}
+
 constexpr int smem_bytes(int D) { return kStages * 2 * kBlockKeys * D * 2 + (kRows * (D + 8) + 8 * kRows) * (int)sizeof(float); }
 // CTAs of the even partition, in quarters of an SM's share.  Not all that shared memory holds where it holds more than
 // one: measured us at 8 KV heads, batch 4 / 8 / 28 of D = 128: 296 CTAs 93.2 / 110.6 / 114.4, 280 89.3 / 106.0 / 112.1, 256
@@ -629,6 +691,44 @@ size_t splitkv_scratch_floats(const FwdProblem& p, const SplitPlan& plan) {
   if (plan.splits <= 1) return 0;
   const size_t rows = (size_t)p.totalQ * p.headsQ;
   return (size_t)plan.splits * rows * (p.headDim + 1);
+}
+
+int launch_combine_parts(const FwdProblem& p, int packShift, const TcSplit& split) {
+  const bool bf = (p.dtype == kBf16);
+#define TFA_COMBINE_CASE(D)                                                                    \
+  case D:                                                                                      \
+    if (bf) {                                                                                  \
+      if constexpr (TFA_HAVE_BF16) return decode::launch_combine<D, true>(p, packShift, split);  \
+    } else {                                                                                   \
+      if constexpr (TFA_HAVE_FP16) return decode::launch_combine<D, false>(p, packShift, split); \
+    }                                                                                          \
+    return kBadDtype;
+  (void)bf;
+  (void)packShift;
+  (void)split;
+  switch (p.headDim) {
+#if TFA_HAVE_HD32
+    TFA_COMBINE_CASE(32)
+#endif
+#if TFA_HAVE_HD64
+    TFA_COMBINE_CASE(64)
+#endif
+#if TFA_HAVE_HD96
+    TFA_COMBINE_CASE(96)
+#endif
+#if TFA_HAVE_HD128
+    TFA_COMBINE_CASE(128)
+#endif
+#if TFA_HAVE_HD192
+    TFA_COMBINE_CASE(192)
+#endif
+#if TFA_HAVE_HD256
+    TFA_COMBINE_CASE(256)
+#endif
+    default:
+      return kBadHeadDim;
+  }
+#undef TFA_COMBINE_CASE
 }
 
 // partO = scratch, partLse = scratch + splits*rows*D

@@ -64,6 +64,13 @@ struct TcParams {
   // on the device by patch_varlen_maps from cuQ[batch] / cuKV[batch]; nullptr = use the maps passed as kernel arguments
   const CUtensorMap* devMaps;
   int epoch;        // launch epoch (24 bits)
+  // key ranges (kModeFixedSplit): every item is cut into parts of partBlocks key blocks, each a work item of its own that
+  // stores its normalised O and log-sum-exp (log2) as partial results
+  int partBlocks;
+  int numItems;     // numPairs * numUnits * batch; numWork = numItems * parts
+  long long rows;   // batch * seqLenQ * headsQ, stride of a part in partO / partLse
+  float* partO;     // [parts][rows][headDim]
+  float* partLse;   // [parts][rows]
 };
 
 namespace tc {
@@ -230,7 +237,7 @@ struct WorkSlot {
   int qlo[2];
   int nblk[2];
   int nmax;
-  int pad;
+  int part;        // key range (kModeFixedSplit)
 };
 
 struct Ctl {
@@ -409,6 +416,13 @@ struct Work {
   int nblk[2];         // KV blocks each tile consumes
   int nmax;
 };
+// ... of a key range (kModeFixedSplit), whose first block is part * partBlocks.  A type of its own: one more field in Work
+// changed the register allocation of the other modes' kernels, which lost up to 1 %.
+struct WorkPart : Work {
+  int part;
+};
+__device__ __forceinline__ int part_of(const Work&) { return 0; }
+__device__ __forceinline__ int part_of(const WorkPart& w) { return w.part; }
 
 // Packed variable-length input, last key block of a sequence: overwrite the rows of the V tile that lie past the end
 // of the sequence with zeros (they are the next sequence's, and P = 0 times a NaN or Inf stored there would still
@@ -438,11 +452,15 @@ __device__ __forceinline__ void zero_v_tail(uint32_t tileAddr, int lane, int tai
 // entries the items are handed out heaviest first (pair index slowest, descending) - the longest-processing-time-first
 // rule, which leaves only light items for the end of the launch; neighbouring indices are then the Q heads of one KV
 // group, which still share K/V, and the host sizes the chunk so that the K/V of its heads stay resident in L2.
-template <int NT, bool kVarlen>
-__device__ __forceinline__ bool make_work(const TcParams& p, int idx, Work& w) {
+template <int NT, bool kVarlen, bool kSplit = false, class W = Work>
+__device__ __forceinline__ bool make_work(const TcParams& p, int idx, W& w) {
   int pr, rest;
+  if constexpr (kSplit) {
+    w.part = idx / p.numItems;
+    idx -= w.part * p.numItems;
+  }
   if (p.chunk > 0) {
-    const int per = p.numWork / p.numPairs;  // (head unit, batch) entries
+    const int per = (kSplit ? p.numItems : p.numWork) / p.numPairs;  // (head unit, batch) entries
     const int chunkItems = p.chunk * p.numPairs;
     const int c = idx / chunkItems;
     const int within = idx - c * chunkItems;
@@ -488,11 +506,30 @@ __device__ __forceinline__ bool make_work(const TcParams& p, int idx, Work& w) {
     int n = 0;
     if (t < NT && w.qlo[t] < w.sq) {
       n = p.causal ? min(nTotal, (w.qhi[t] + kBlockN - 1) / kBlockN) : nTotal;
+      if constexpr (kSplit) n = max(0, min(n - w.part * p.partBlocks, p.partBlocks));
     }
     w.nblk[t] = n;
     w.nmax = max(w.nmax, n);
   }
-  return true;
+  return !kSplit || w.nmax > 0;
+}
+
+// Does a tile's whole key range fit its first part?  Such rows (the early ones of a causal problem) get their final output
+// straight away.
+__device__ __forceinline__ bool whole_tile(const TcParams& p, const Work& w, int t) {
+  int n = (w.skv + kBlockN - 1) / kBlockN;
+  if (p.causal) n = min(n, (min(w.qlo[t] + (kBlockM >> p.packShift), w.sq) + kBlockN - 1) / kBlockN);
+  return n <= p.partBlocks;
+}
+// 32 columns of a row's partial result, normalised by the row sum of its key range
+__device__ __forceinline__ void store_part(const TcParams& p, const Work& w, int part, int qpos, int head, int col, const uint32_t (&o)[32],
+                                           float inv) {
+  float4* dst = reinterpret_cast<float4*>(p.partO + (part * p.rows + (w.qRow0 + qpos) * p.headsQ + head) * p.headDim + col);
+#pragma unroll
+  for (int g = 0; g < 8; g++) {
+    dst[g] = make_float4(__uint_as_float(o[g * 4]) * inv, __uint_as_float(o[g * 4 + 1]) * inv, __uint_as_float(o[g * 4 + 2]) * inv,
+                         __uint_as_float(o[g * 4 + 3]) * inv);
+  }
 }
 
 // Persistent kernel: gridDim.x CTAs (one per SM) pull work items from a global counter until it runs out, so the
@@ -502,8 +539,10 @@ __device__ __forceinline__ bool make_work(const TcParams& p, int idx, Work& w) {
 // (not causal, key length a multiple of the 128-key block).  Separate instantiations, because code that a path never
 // executes still costs it when it sits in the softmax loop (measured: the variable-length code 4-5 % of the
 // fixed-length speed; the masking code 8 % at head dim 64 and nothing at 128 / 256, so mode 2 is only built for
-// the 64 kernel).
-constexpr int kModeFixed = 0, kModeVarlen = 1, kModeFixedNoMask = 2;
+// the 64 kernel), 3 fixed length with every item cut into key ranges (few query tiles, long keys).
+// Mode 3 is for calls that leave SMs idle otherwise: 2 x 8 query rows x 12289 keys, 32 heads over 8 of 128, 16 CTAs and 150
+// us whole, 144 CTAs and 36 us in nine ranges (19 us of key blocks, the rest launch, first loads and the combine kernel).
+constexpr int kModeFixed = 0, kModeVarlen = 1, kModeFixedNoMask = 2, kModeFixedSplit = 3;
 // kHD: the head dim the MMAs are shaped for.  The tiles in shared memory are always HDP wide (64-element slabs, TMA
 // zero-fills past the true head dim); with kHD < HDP (32 in the 64-wide kernel, 96 in the 128-wide one) Q.K^T stops
 // after kHD / 16 k-steps, P.V produces kHD output columns, and the rescale and output passes touch kHD columns.
@@ -523,6 +562,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   constexpr int kEpilogueEnd = kSolo ? 4 : 12;  // epilogue warps are [kSoftmaxWarps, kEpilogueEnd): none in the solo form
   constexpr int kIssueWarpA = kSolo ? 4 : 12, kIssueWarpB = kSolo ? -1 : kIssuerB, kLoadWarp = kSolo ? 5 : 13;
   constexpr bool kVarlen = (kMode == kModeVarlen);
+  constexpr bool kSplit = (kMode == kModeFixedSplit);
   // Packed input has one more role: a warp that is idle otherwise (14, or 6 in the one-tile form) zeroes the V rows
   // past a sequence's end and takes part in every "first half of P ready" barrier, so that no P.V can start before
   // the rows are clean.  Kept out of the softmax warps: the same code inside their block loop, executed once per
@@ -543,6 +583,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   // re-uses a stage is consumed at or after P.V of the block whose scores the waiting warp is about to produce.
   constexpr bool kRingSig = (NT == 1 && NS >= 3);
   static_assert(!kRingSig || C::kTwoPos, "one-tile forms alternate S between two positions");
+
+  if constexpr (kSplit) asm volatile("griddepcontrol.launch_dependents;");  // the combine kernel waits for this grid's end
 
   extern __shared__ uint8_t smemRaw[];
   const uint32_t rawAddr = ptx::smem_u32(smemRaw);
@@ -636,7 +678,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 
   // Every consumer of work items (8 softmax warps, 4 epilogue warps, 2 MMA threads) reads item k from slot k & 1
   // and frees the slot; a negative index ends the loop.
-  auto fetchWork = [&](int k, Work& w) -> int {
+  using WorkT = typename std::conditional<kSplit, WorkPart, Work>::type;
+  auto fetchWork = [&](int k, WorkT& w) -> int {
     wait_bar(bar(kBarWorkFull + (k & 1)), (k >> 1) & 1, wc, 20);
     // plain loads: the barrier wait above is an acquire and a compiler-level memory fence, and fields that a role
     // does not use cost it neither a load nor a register
@@ -650,6 +693,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     w.nblk[0] = ws->nblk[0];
     w.nblk[1] = ws->nblk[1];
     w.nmax = ws->nmax;
+    if constexpr (kSplit) w.part = ws->part;
     return ws->idx;
   };
 
@@ -664,7 +708,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     int items = 0;   // work items in which this tile was active
     int ldBase = 0;  // K/V ring loads of all earlier items (packed variable-length input only, see below)
     for (int k = 0;; k++) {
-      Work w;
+      WorkT w;
       const int idx = fetchWork(k, w);
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar(kBarWorkEmpty + (k & 1)));
@@ -700,7 +744,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
           if (lane == 0) ptx::mbar_arrive(bar(kBarSFree + t));
         }
 
-        const int kbase = j * kBlockN;
+        const int kbase = (kSplit ? part_of(w) * p.partBlocks + j : j) * kBlockN;
         const bool needMask = (kMode != kModeFixedNoMask) &&
                               ((kbase + kBlockN > w.skv) || (p.causal && (kbase + kBlockN - 1 > w.qlo[t])));
         if (needMask) {
@@ -809,6 +853,12 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         }
         l += sum2.x + sum2.y;
       }
+      if constexpr (kSplit) {  // log-sum-exp of this key range; NaN stays NaN
+        if (qpos < w.sq && !whole_tile(p, w, t)) {
+          const int head = (w.unit << p.packShift) + (r & ((1 << p.packShift) - 1));
+          p.partLse[part_of(w) * p.rows + (w.qRow0 + qpos) * p.headsQ + head] = (l == 0.f) ? -INFINITY : m * c + __log2f(l);
+        }
+      }
       if constexpr (kSolo) {
         // This warp is also the epilogue of its 32 rows: wait for the last P.V of the item, read O, release the
         // accumulator to the next item, normalise, convert and store.  Meanwhile the SM's other CTA keeps computing.
@@ -833,7 +883,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(bar(kBarOFree + t));
           }
-          if (valid && ch * 32 < p.headDim) {
+          if (kSplit && !whole_tile(p, w, t)) {
+            if (valid && ch * 32 < p.headDim) store_part(p, w, part_of(w), qpos, head, ch * 32, o, inv);
+          } else if (valid && ch * 32 < p.headDim) {
 #pragma unroll
             for (int g = 0; g < 4; g++) {
               uint4 q;
@@ -865,7 +917,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     int pvTotal[2] = {0, 0};  // blocks of tile t issued so far
     int ldBase = 0;           // K/V ring loads of all earlier items
     for (int k = 0;; k++) {
-      Work w;
+      WorkT w;
       const int idx = fetchWork(k, w);
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar(kBarWorkEmpty + (k & 1)));
@@ -913,7 +965,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             }
           }
           const int hdOff = o_chunk_offset<HDP, kPair>(ch);  // a constant once the loop is unrolled
-          if (valid && hdOff < p.headDim) {
+          if (kSplit && !whole_tile(p, w, t)) {
+            if (valid && hdOff < p.headDim) store_part(p, w, part_of(w), qpos, head, hdOff, o, inv);
+          } else if (valid && hdOff < p.headDim) {
 #pragma unroll
             for (int g = 0; g < 4; g++) {
               uint4 q;
@@ -1007,7 +1061,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       int it = 0;    // blocks of this tile issued so far
       int qc = 0;    // work items in which this tile was active
       for (int k = 0;; k++) {
-        Work w;
+        WorkT w;
         const int idx = fetchWork(k, w);
         ptx::mbar_arrive(bar(kBarWorkEmpty + (k & 1)));
         if (idx < 0 || *wc.failed) break;
@@ -1169,10 +1223,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       int qc[2] = {0, 0};    // Q loads issued so far per tile
       // Takes the next work index, works out its description and publishes both in slot k & 1 (free once every
       // consumer has read item k - 2 from it).  Returns false when the work has run out.
-      Work wq[2];
+      WorkT wq[2];
       auto publish = [&](int k) -> bool {
         if (k >= 2) wait_bar(bar(kBarWorkEmpty + (k & 1)), ((k >> 1) - 1) & 1, wc, 21);
-        Work& w = wq[k & 1];
+        WorkT& w = wq[k & 1];
         // indices whose tile pair lies past the end of a short sequence (packed variable-length input) are
         // dropped here: nobody else hears of them
         int idx;
@@ -1208,7 +1262,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
           do {
             idx = atomicAdd(p.workCounter, 1);
             if (idx >= p.numWork || *reinterpret_cast<volatile int*>(&ctl->failed)) idx = -1;
-          } while (idx >= 0 && !make_work<NT, kVarlen>(p, idx, w));
+          } while (idx >= 0 && !make_work<NT, kVarlen, kSplit>(p, idx, w));
         }
         volatile WorkSlot* ws = &ctl->work[k & 1];
         ws->idx = idx;
@@ -1221,6 +1275,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         ws->nblk[0] = w.nblk[0];
         ws->nblk[1] = w.nblk[1];
         ws->nmax = w.nmax;
+        if constexpr (kSplit) ws->part = w.part;
         ptx::mbar_arrive(bar(kBarWorkFull + (k & 1)));  // release: the stores above are visible to whoever waits
         return idx >= 0;
       };
@@ -1230,7 +1285,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         // only waiting for ring stages, and nobody waits for the atomic round trip and the divisions between two
         // items.  (Doing it right after the first loads of the item, when the ring is still filling, cost 6 %.)
         bool nextDone = false;
-        const Work& w = wq[k & 1];
+        const WorkT& w = wq[k & 1];
         // The Q tiles of this item cannot land in shared memory before the previous item's last Q.K^T has
         // finished; pulling them into L2 now shortens that exposed load at the item boundary.
 #pragma unroll
@@ -1294,7 +1349,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             blkIdx = i >> 1;
           }
           const CUtensorMap* tm = isV ? mapV : mapK;
-          const int row = w.kvRowTma + blkIdx * kBlockN;
+          const int row = w.kvRowTma + (kSplit ? part_of(w) * p.partBlocks + blkIdx : blkIdx) * kBlockN;
           if constexpr (kPair) {
             // This CTA's half of the block, counted on rank 0's barrier together with the other half.
             // K: keys [64 rank, 64 rank + 64), all of the head dim (the K map's box is 64 rows high);
@@ -1335,7 +1390,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       int ldBase = 0;         // K/V ring loads of all earlier items
       int cnt[2] = {0, 0};    // blocks of tile t so far, over all items (phase of its P-ready barriers)
       for (int k = 0;; k++) {
-        Work w;
+        WorkT w;
         const int idx = fetchWork(k, w);
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(bar(kBarWorkEmpty + (k & 1)));

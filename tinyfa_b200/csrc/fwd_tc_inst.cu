@@ -62,7 +62,7 @@ static int make_map(CUtensorMap* m, const void* base, long long batches, long lo
   return kOk;
 }
 
-int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift) {
+int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSplit& split) {
   using C = tc::Cfg<TFA_HDP>;
   const bool varlen = (pr.cuQ != nullptr);
   constexpr bool kBf = (TFA_BF16 != 0);
@@ -97,6 +97,21 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift) {
   }
 #endif
 
+  const bool parts = split.parts > 1;  // key ranges: few query tiles, long keys (fixed length)
+  if (parts) {
+#if TFA_HDP == 64
+    kernel = pr.headDim == 32 ? tc::fwd_tc_kernel<64, kBf, tc::kModeFixedSplit, true, 32> : tc::fwd_tc_kernel<64, kBf, tc::kModeFixedSplit, true>;
+    solo = true;
+    kNT = 1;
+    smemBytes = tc::CfgSolo64::kSmemBytes;
+    threads = tc::kThreadsSolo;
+#elif TFA_HDP == 128
+    kernel = pr.headDim == 96 ? tc::fwd_tc_kernel<128, kBf, tc::kModeFixedSplit, false, 96> : tc::fwd_tc_kernel<128, kBf, tc::kModeFixedSplit>;
+#else
+    kernel = tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit>;
+#endif
+  }
+
   bool pair = false;  // clusters of two CTAs, one Q tile each, K/V shared (head dims 192 / 256, fixed length)
 #if TFA_HDP >= 192
   // Measured (fp16, H16, batch x length = 16 K tokens, 600-800-launch loops, one-tile form -> pair form): head dim 256
@@ -107,7 +122,7 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift) {
   // boundaries that are twice as heavy; "auto" is head dim 256 only, and its causal problems from 1024 query rows.
   const int pairOpt = option_pair_cta();
   const bool pairAuto = (TFA_HDP == 256) && (!pr.causal || pr.seqLenQ >= 1024);
-  pair = !varlen && pr.seqLenQ > (tc::kBlockM >> packShift) && (pairOpt > 0 || (pairOpt < 0 && pairAuto));
+  pair = !parts && !varlen && pr.seqLenQ > (tc::kBlockM >> packShift) && (pairOpt > 0 || (pairOpt < 0 && pairAuto));
   if (pair) {
     kernel = tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixed, false, TFA_HDP, true>;
     kNT = 2;  // a work item is the two tiles of a pair
@@ -128,6 +143,9 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift) {
     attrErr[device] = cudaSuccess;
     bigAttr(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixed>);
     bigAttr(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeVarlen>);
+#if TFA_HDP != 64
+    bigAttr(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit>);
+#endif
 #if TFA_HDP >= 192
     if (attrErr[device] == cudaSuccess) {
       attrErr[device] = cudaFuncSetAttribute(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixed, false, TFA_HDP, true>,
@@ -137,6 +155,7 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift) {
 #if TFA_HDP == 128
     bigAttr(tc::fwd_tc_kernel<128, kBf, tc::kModeFixed, false, 96>);
     bigAttr(tc::fwd_tc_kernel<128, kBf, tc::kModeVarlen, false, 96>);
+    bigAttr(tc::fwd_tc_kernel<128, kBf, tc::kModeFixedSplit, false, 96>);
 #endif
 #if TFA_HDP == 64
     bigAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedNoMask>);
@@ -154,6 +173,8 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift) {
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixed, true, 32>);
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeVarlen, true, 32>);
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedNoMask, true, 32>);
+    soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedSplit, true>);
+    soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedSplit, true, 32>);
 #endif
   });
   if (attrErr[device] != cudaSuccess) {
@@ -194,12 +215,18 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift) {
   p.epoch = next_epoch();
   if (p.status == nullptr) return kCudaError;
   p.numUnits = pr.headsQ / gp;
-  const long long numWork = (long long)p.numPairs * p.numUnits * pr.batch;
+  const long long numItems = (long long)p.numPairs * p.numUnits * pr.batch;
+  const long long numWork = numItems * split.parts;
+  p.partBlocks = split.partBlocks;
+  p.partO = split.partO;
+  p.partLse = split.partLse;
+  p.rows = pr.totalQ * pr.headsQ;
   if (numWork > 0x7FFFFFFFll) {
     set_error_string("too many work items (%lld)", numWork);
     return kTooLarge;
   }
   p.numWork = (int)numWork;
+  p.numItems = (int)numItems;
   // Causal problems: heaviest query tile pairs first inside chunks of (head unit, batch) entries.  A chunk is as wide
   // as the KV heads whose K and V fit a quarter of the L2 (32 MB) together, and at least wide enough to hold two
   // items per SM.  Option "work_order": -1 this rule, 0 pair index fastest, n > 0 chunks of n entries.

@@ -58,6 +58,15 @@ struct SplitPlan {
   int blocksPerEntry;
 };
 
+// How the tensor-core path cuts a call with few query tiles into key ranges: `parts` ranges of partBlocks 128-key blocks
+// (parts == 1: not at all), and where their partial results go ([parts][rows][headDim] and [parts][rows] floats).
+struct TcSplit {
+  int parts = 1;
+  int partBlocks = 0;
+  float* partO = nullptr;
+  float* partLse = nullptr;
+};
+
 // The device status word holds 0, or (launch epoch << 8) | site code once a bounded wait inside a kernel gave up.
 
 int launch_fwd_fp32(const FwdProblem& p);    // fp32: CUDA-core FMA kernel
