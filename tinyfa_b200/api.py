@@ -31,8 +31,23 @@ def _dtype_code(t, fn):
     return code
 
 
-def flash_attn_forward(Q, K, V, is_causal=False):
-    """Fixed-length attention forward.  Q [B,Sq,Hq,D]; K,V [B,Skv,Hkv,D]; returns O like Q."""
+# Current stream and device as plain integers.  torch.cuda.current_stream() and the torch.cuda.device guard build Python
+# objects: 3.2 and 1.5 us of a call whose native part takes 4.3.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+
+
+def _usable(*tensors):
+    """Contiguous CUDA tensors of one device?  One pass without messages; the checks below say what is wrong."""
+    for t in tensors:
+        if not (isinstance(t, torch.Tensor) and t.is_cuda and t.is_contiguous()):
+            return False
+    index = tensors[0].get_device()
+    return all([t.get_device() == index for t in tensors])
+
+
+def _check_fixed(Q, K, V):
     _check_input(Q, "Q")
     _check_input(K, "K")
     _check_input(V, "V")
@@ -40,30 +55,50 @@ def flash_attn_forward(Q, K, V, is_causal=False):
     _check(K.dim() == 4, "K must be 4D [batch, seqKV, numHeadsKV, headDim]")
     _check(V.dim() == 4, "V must be 4D [batch, seqKV, numHeadsKV, headDim]")
     _check(Q.dtype == K.dtype and Q.dtype == V.dtype, "Q, K, V must have the same dtype")
-    batch, seq_q, heads_q, head_dim = Q.shape
+    batch, _, heads_q, head_dim = Q.shape
     seq_kv, heads_kv = K.shape[1], K.shape[2]
     _check(K.shape[0] == batch and V.shape[0] == batch, "Batch sizes must match")
     _check(V.shape[1] == seq_kv, "K and V must have the same seqlen")
     _check(K.shape[3] == head_dim and V.shape[3] == head_dim, "Head dims must match")
     _check(V.shape[2] == heads_kv, "K and V must have the same number of heads")
     _check(heads_kv > 0 and heads_q % heads_kv == 0, "numHeadsQ must be divisible by numHeadsKV (GQA)")
-    code = _dtype_code(Q, "flash_attn_forward")
+    _dtype_code(Q, "flash_attn_forward")
     _check(K.device == Q.device and V.device == Q.device, "Q, K, V must be on the same device")
 
-    lib = _lib.load()
-    with torch.cuda.device(Q.device):
-        # Every query row is written when there is at least one key, so the reference's zero fill
-        # (binding:106) only matters for the degenerate shapes.
-        O = torch.empty_like(Q) if (seq_kv > 0 and Q.numel() > 0) else torch.zeros_like(Q)
-        stream = torch.cuda.current_stream().cuda_stream
-        rc = lib.tfa_b200_fwd(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), code, batch, seq_q, seq_kv,
-                              heads_q, heads_kv, head_dim, 1 if is_causal else 0, stream)
-    _lib.check(rc, "flash_attn_forward")
+
+def _run_fixed(lib, device, Q, K, V, code, q_shape, seq_kv, heads_kv, is_causal):
+    # Every query row is written when there is at least one key, so the reference's zero fill
+    # (binding:106) only matters for the degenerate shapes.
+    batch, seq_q, heads_q, head_dim = q_shape
+    O = torch.empty_like(Q) if (seq_kv > 0 and Q.numel() > 0) else torch.zeros_like(Q)
+    rc = lib.tfa_b200_fwd(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), code, batch, seq_q, seq_kv,
+                          heads_q, heads_kv, head_dim, 1 if is_causal else 0, _raw_stream(device))
+    if rc != 0:
+        _lib.check(rc, "flash_attn_forward")
     return O
 
 
-def flash_attn_varlen_forward(Q, K, V, cu_seqlens_q, cu_seqlens_kv, max_seqlen_q, max_seqlen_kv, is_causal=False):
-    """Packed variable-length forward.  Q [totalQ,Hq,D]; K,V [totalKV,Hkv,D]; cu_seqlens int32 [B+1] on the device."""
+def flash_attn_forward(Q, K, V, is_causal=False):
+    """Fixed-length attention forward.  Q [B,Sq,Hq,D]; K,V [B,Skv,Hkv,D]; returns O like Q."""
+    ok = _usable(Q, K, V)
+    if ok:
+        q_shape, kv_shape, dtype = Q.shape, K.shape, Q.dtype
+        code = _DTYPE_CODE.get(dtype)
+        ok = (code is not None and K.dtype == dtype and V.dtype == dtype and len(q_shape) == 4 and len(kv_shape) == 4
+              and V.shape == kv_shape and kv_shape[0] == q_shape[0] and kv_shape[3] == q_shape[3]
+              and kv_shape[2] > 0 and q_shape[2] % kv_shape[2] == 0)
+    if not ok:
+        _check_fixed(Q, K, V)
+        raise RuntimeError("flash_attn_forward: unsupported input")
+    lib = _lib.load()
+    device = Q.get_device()
+    if _current_device() == device:
+        return _run_fixed(lib, device, Q, K, V, code, q_shape, kv_shape[1], kv_shape[2], is_causal)
+    with torch.cuda.device(device):
+        return _run_fixed(lib, device, Q, K, V, code, q_shape, kv_shape[1], kv_shape[2], is_causal)
+
+
+def _check_varlen(Q, K, V, cu_seqlens_q, cu_seqlens_kv):
     _check_input(Q, "Q")
     _check_input(K, "K")
     _check_input(V, "V")
@@ -83,21 +118,45 @@ def flash_attn_varlen_forward(Q, K, V, cu_seqlens_q, cu_seqlens_kv, max_seqlen_q
     _check(heads_kv > 0 and heads_q % heads_kv == 0, "numHeadsQ must be divisible by numHeadsKV (GQA)")
     _check(cu_seqlens_kv.shape[0] == batch + 1, "cu_seqlens_q and cu_seqlens_kv must have the same length")
     _check(V.shape[0] == K.shape[0], "K and V must have the same seqlen")
-    code = _dtype_code(Q, "flash_attn_varlen_forward")
+    _dtype_code(Q, "flash_attn_varlen_forward")
     _check(all(t.device == Q.device for t in (K, V, cu_seqlens_q, cu_seqlens_kv)),
            "Q, K, V and cu_seqlens must be on the same device")
 
-    lib = _lib.load()
-    with torch.cuda.device(Q.device):
-        O = torch.zeros_like(Q)  # sequences without keys keep zeros (binding:148)
-        if batch > 0:
-            stream = torch.cuda.current_stream().cuda_stream
-            rc = lib.tfa_b200_fwd_varlen(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(),
-                                         cu_seqlens_q.data_ptr(), cu_seqlens_kv.data_ptr(), code, batch,
-                                         int(max_seqlen_q), int(max_seqlen_kv), Q.shape[0], K.shape[0], heads_q,
-                                         heads_kv, head_dim, 1 if is_causal else 0, stream)
+
+def _run_varlen(lib, device, Q, K, V, cu_seqlens_q, cu_seqlens_kv, max_seqlen_q, max_seqlen_kv, code, is_causal):
+    O = torch.zeros_like(Q)  # sequences without keys keep zeros (binding:148)
+    batch = cu_seqlens_q.shape[0] - 1
+    if batch > 0:
+        total_q, heads_q, head_dim = Q.shape
+        total_kv, heads_kv, _ = K.shape
+        rc = lib.tfa_b200_fwd_varlen(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), cu_seqlens_q.data_ptr(),
+                                     cu_seqlens_kv.data_ptr(), code, batch, int(max_seqlen_q), int(max_seqlen_kv),
+                                     total_q, total_kv, heads_q, heads_kv, head_dim, 1 if is_causal else 0,
+                                     _raw_stream(device))
+        if rc != 0:
             _lib.check(rc, "flash_attn_varlen_forward")
     return O
+
+
+def flash_attn_varlen_forward(Q, K, V, cu_seqlens_q, cu_seqlens_kv, max_seqlen_q, max_seqlen_kv, is_causal=False):
+    """Packed variable-length forward.  Q [totalQ,Hq,D]; K,V [totalKV,Hkv,D]; cu_seqlens int32 [B+1] on the device."""
+    ok = _usable(Q, K, V, cu_seqlens_q, cu_seqlens_kv)
+    if ok:
+        q_shape, kv_shape, dtype = Q.shape, K.shape, Q.dtype
+        code = _DTYPE_CODE.get(dtype)
+        ok = (code is not None and K.dtype == dtype and V.dtype == dtype and len(q_shape) == 3 and len(kv_shape) == 3
+              and V.shape == kv_shape and kv_shape[2] == q_shape[2] and kv_shape[1] > 0 and q_shape[1] % kv_shape[1] == 0
+              and cu_seqlens_q.dtype == torch.int32 and cu_seqlens_kv.dtype == torch.int32 and cu_seqlens_q.dim() == 1
+              and cu_seqlens_kv.shape == cu_seqlens_q.shape)
+    if not ok:
+        _check_varlen(Q, K, V, cu_seqlens_q, cu_seqlens_kv)
+        raise RuntimeError("flash_attn_varlen_forward: unsupported input")
+    lib = _lib.load()
+    device = Q.get_device()
+    if _current_device() == device:
+        return _run_varlen(lib, device, Q, K, V, cu_seqlens_q, cu_seqlens_kv, max_seqlen_q, max_seqlen_kv, code, is_causal)
+    with torch.cuda.device(device):
+        return _run_varlen(lib, device, Q, K, V, cu_seqlens_q, cu_seqlens_kv, max_seqlen_q, max_seqlen_kv, code, is_causal)
 
 
 def is_head_dim_compiled(head_dim):
