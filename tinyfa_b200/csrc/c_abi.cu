@@ -445,9 +445,9 @@ static TcSplit tc_split_plan(const FwdProblem& p, int packShift) {
   TcSplit s;
   const int opt = g_optSplitTc.load();
   if (opt == 0 || p.cuQ != nullptr || !dtype_compiled(p.dtype) || !head_dim_compiled(p.headDim)) return s;
-  const int rowsPerItem = (p.headDim == 96 || p.headDim == 128 ? 2 : 1) * (128 >> packShift);
+  const int rowsPerItem = 128 >> packShift;
   const long long items = (long long)((p.seqLenQ + rowsPerItem - 1) / rowsPerItem) * (p.headsQ >> packShift) * p.batch;
-  const long long slots = (long long)num_sms() * (p.headDim <= 64 ? 2 : 1);
+  const long long slots = (long long)num_sms() * (p.headDim <= 128 ? 2 : 1);
   const int seen = p.causal ? (p.seqLenQ < p.seqLenKV ? p.seqLenQ : p.seqLenKV) : p.seqLenKV;
   const int blocks = (seen + 127) / 128;
   long long parts = opt;

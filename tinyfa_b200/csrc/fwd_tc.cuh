@@ -64,7 +64,11 @@ struct TcParams {
   // on the device by patch_varlen_maps from cuQ[batch] / cuKV[batch]; nullptr = use the maps passed as kernel arguments
   const CUtensorMap* devMaps;
   int epoch;        // launch epoch (24 bits)
-  // key ranges (kModeFixedSplit): every item is cut into parts of partBlocks key blocks, each a work item of its own that
+};
+// ... and of a call cut into key ranges.  A type of its own, like WorkPart below: the kernels without ranges, whose register
+// allocation and schedule sit in a narrow optimum, lost up to 3 % to fields that they do not use.
+struct TcPartParams : TcParams {
+  // every item is cut into parts of partBlocks key blocks, each a work item of its own that
   // stores its normalised O and log-sum-exp (log2) as partial results
   int partBlocks;
   int numItems;     // numPairs * numUnits * batch; numWork = numItems * parts
@@ -153,6 +157,27 @@ struct CfgSolo64 {
   static constexpr int kPPosStride = 128;
   static constexpr int kSRegion = 192;
   static constexpr int kOCol0 = 192;
+  static constexpr int kStageBytes = kTileBytes;
+  static constexpr int kSmemBytes = kNT * kQBufs * kTileBytes + kStages * kStageBytes + 2048 + 1024;
+};
+
+// Head dims 96 / 128, key ranges (kModeFixedSplit): the same with tiles twice as wide.  One S position (S 128 columns, O 128)
+// and two 32 KB ring stages are what fits twice on an SM; a block's K loads under the softmax and P.V of the block before,
+// its V under its own Q.K^T and softmax.
+struct CfgSolo128 {
+  static constexpr int kSub = 2;
+  static constexpr int kTileBytes = 2 * kSubTileBytes;
+  static constexpr int kNT = 1;
+  static constexpr int kQBufs = 1;
+  static constexpr int kStages = 2;
+  static constexpr int kTmemCols = 256;
+  static constexpr bool kRot = false;
+  static constexpr bool kDblS = false;
+  static constexpr bool kTwoPos = false;
+  static constexpr int kSPosStride = 0;
+  static constexpr int kPPosStride = 0;
+  static constexpr int kSRegion = 128;
+  static constexpr int kOCol0 = 128;
   static constexpr int kStageBytes = kTileBytes;
   static constexpr int kSmemBytes = kNT * kQBufs * kTileBytes + kStages * kStageBytes + 2048 + 1024;
 };
@@ -416,13 +441,10 @@ struct Work {
   int nblk[2];         // KV blocks each tile consumes
   int nmax;
 };
-// ... of a key range (kModeFixedSplit), whose first block is part * partBlocks.  A type of its own: one more field in Work
-// changed the register allocation of the other modes' kernels, which lost up to 1 %.
+// ... of a key range (kModeFixedSplit), whose first block is part * partBlocks
 struct WorkPart : Work {
   int part;
 };
-__device__ __forceinline__ int part_of(const Work&) { return 0; }
-__device__ __forceinline__ int part_of(const WorkPart& w) { return w.part; }
 
 // Packed variable-length input, last key block of a sequence: overwrite the rows of the V tile that lie past the end
 // of the sequence with zeros (they are the next sequence's, and P = 0 times a NaN or Inf stored there would still
@@ -452,15 +474,20 @@ __device__ __forceinline__ void zero_v_tail(uint32_t tileAddr, int lane, int tai
 // entries the items are handed out heaviest first (pair index slowest, descending) - the longest-processing-time-first
 // rule, which leaves only light items for the end of the launch; neighbouring indices are then the Q heads of one KV
 // group, which still share K/V, and the host sizes the chunk so that the K/V of its heads stay resident in L2.
-template <int NT, bool kVarlen, bool kSplit = false, class W = Work>
-__device__ __forceinline__ bool make_work(const TcParams& p, int idx, W& w) {
+template <int NT, bool kVarlen, bool kSplit = false, class P = TcParams, class W = Work>
+__device__ __forceinline__ bool make_work(const P& p, int idx, W& w) {
   int pr, rest;
   if constexpr (kSplit) {
     w.part = idx / p.numItems;
     idx -= w.part * p.numItems;
   }
   if (p.chunk > 0) {
-    const int per = (kSplit ? p.numItems : p.numWork) / p.numPairs;  // (head unit, batch) entries
+    int per;  // (head unit, batch) entries
+    if constexpr (kSplit) {
+      per = p.numItems / p.numPairs;
+    } else {
+      per = p.numWork / p.numPairs;
+    }
     const int chunkItems = p.chunk * p.numPairs;
     const int c = idx / chunkItems;
     const int within = idx - c * chunkItems;
@@ -511,20 +538,21 @@ __device__ __forceinline__ bool make_work(const TcParams& p, int idx, W& w) {
     w.nblk[t] = n;
     w.nmax = max(w.nmax, n);
   }
-  return !kSplit || w.nmax > 0;
+  if constexpr (kSplit) return w.nmax > 0;
+  return true;
 }
 
 // Does a tile's whole key range fit its first part?  Such rows (the early ones of a causal problem) get their final output
 // straight away.
-__device__ __forceinline__ bool whole_tile(const TcParams& p, const Work& w, int t) {
+__device__ __forceinline__ bool whole_tile(const TcPartParams& p, const Work& w, int t) {
   int n = (w.skv + kBlockN - 1) / kBlockN;
   if (p.causal) n = min(n, (min(w.qlo[t] + (kBlockM >> p.packShift), w.sq) + kBlockN - 1) / kBlockN);
   return n <= p.partBlocks;
 }
 // 32 columns of a row's partial result, normalised by the row sum of its key range
-__device__ __forceinline__ void store_part(const TcParams& p, const Work& w, int part, int qpos, int head, int col, const uint32_t (&o)[32],
+__device__ __forceinline__ void store_part(const TcPartParams& p, const WorkPart& w, int qpos, int head, int col, const uint32_t (&o)[32],
                                            float inv) {
-  float4* dst = reinterpret_cast<float4*>(p.partO + (part * p.rows + (w.qRow0 + qpos) * p.headsQ + head) * p.headDim + col);
+  float4* dst = reinterpret_cast<float4*>(p.partO + (w.part * p.rows + (w.qRow0 + qpos) * p.headsQ + head) * p.headDim + col);
 #pragma unroll
   for (int g = 0; g < 8; g++) {
     dst[g] = make_float4(__uint_as_float(o[g * 4]) * inv, __uint_as_float(o[g * 4 + 1]) * inv, __uint_as_float(o[g * 4 + 2]) * inv,
@@ -543,6 +571,10 @@ __device__ __forceinline__ void store_part(const TcParams& p, const Work& w, int
 // Mode 3 is for calls that leave SMs idle otherwise: 2 x 8 query rows x 12289 keys, 32 heads over 8 of 128, 16 CTAs and 150
 // us whole, 144 CTAs and 36 us in nine ranges (19 us of key blocks, the rest launch, first loads and the combine kernel).
 constexpr int kModeFixed = 0, kModeVarlen = 1, kModeFixedNoMask = 2, kModeFixedSplit = 3;
+template <int kMode>
+struct ParamsOf {
+  using type = typename std::conditional<kMode == kModeFixedSplit, TcPartParams, TcParams>::type;
+};
 // kHD: the head dim the MMAs are shaped for.  The tiles in shared memory are always HDP wide (64-element slabs, TMA
 // zero-fills past the true head dim); with kHD < HDP (32 in the 64-wide kernel, 96 in the 128-wide one) Q.K^T stops
 // after kHD / 16 k-steps, P.V produces kHD output columns, and the rescale and output passes touch kHD columns.
@@ -550,12 +582,14 @@ constexpr int kModeFixed = 0, kModeVarlen = 1, kModeFixedNoMask = 2, kModeFixedS
 template <int HDP, bool kBf16, int kMode, bool kSolo = false, int kHD = HDP, bool kPair = false>
 __global__ void __launch_bounds__(kSolo ? kThreadsSolo : kThreads, kSolo ? 2 : 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-              const __grid_constant__ CUtensorMap tmV, const TcParams p) {
-  static_assert(!kSolo || HDP == 64, "the one-tile, two-CTAs-per-SM form exists for padded head dim 64 only");
+              const __grid_constant__ CUtensorMap tmV, const typename ParamsOf<kMode>::type p) {
+  static_assert(!kSolo || HDP == 64 || (HDP == 128 && kMode == kModeFixedSplit),
+                "the one-tile, two-CTAs-per-SM form exists for padded head dim 64, and at 128 for key ranges");
   static_assert(kHD == HDP || (HDP == 64 && kHD == 32) || (HDP == 128 && kHD == 96), "MMA head dim");
   static_assert(!kPair || (HDP >= 192 && kMode == kModeFixed && !kSolo), "pair form: head dims 192 / 256, fixed length");
   using C = typename std::conditional<kPair, CfgPair<(kPair ? HDP : 256)>,
-                                      typename std::conditional<kSolo, CfgSolo64, Cfg<HDP>>::type>::type;
+                                      typename std::conditional<kSolo, typename std::conditional<HDP == 64, CfgSolo64, CfgSolo128>::type,
+                                                                Cfg<HDP>>::type>::type;
   constexpr int NT = C::kNT;
   // warp roles: softmax warps [0, 4 * NT'), epilogue warps, the two MMA-issuing warps, the loading warp
   constexpr int kSoftmaxWarps = kSolo ? 4 : 8;
@@ -744,7 +778,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
           if (lane == 0) ptx::mbar_arrive(bar(kBarSFree + t));
         }
 
-        const int kbase = (kSplit ? part_of(w) * p.partBlocks + j : j) * kBlockN;
+        int kbase = j * kBlockN;
+        if constexpr (kSplit) kbase += w.part * p.partBlocks * kBlockN;
         const bool needMask = (kMode != kModeFixedNoMask) &&
                               ((kbase + kBlockN > w.skv) || (p.causal && (kbase + kBlockN - 1 > w.qlo[t])));
         if (needMask) {
@@ -856,14 +891,18 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       if constexpr (kSplit) {  // log-sum-exp of this key range; NaN stays NaN
         if (qpos < w.sq && !whole_tile(p, w, t)) {
           const int head = (w.unit << p.packShift) + (r & ((1 << p.packShift) - 1));
-          p.partLse[part_of(w) * p.rows + (w.qRow0 + qpos) * p.headsQ + head] = (l == 0.f) ? -INFINITY : m * c + __log2f(l);
+          p.partLse[w.part * p.rows + (w.qRow0 + qpos) * p.headsQ + head] = (l == 0.f) ? -INFINITY : m * c + __log2f(l);
         }
       }
       if constexpr (kSolo) {
         // This warp is also the epilogue of its 32 rows: wait for the last P.V of the item, read O, release the
         // accumulator to the next item, normalise, convert and store.  Meanwhile the SM's other CTA keeps computing.
-        const int gLast = ldItem + 2 * w.nmax - 1;  // the item's last load is V of its last block
-        wait_bar(bar(kBarKvEmpty + gLast % NS), (gLast / NS) & 1, wc, 7);
+        if constexpr (kRingSig) {
+          const int gLast = ldItem + 2 * w.nmax - 1;  // the item's last load is V of its last block
+          wait_bar(bar(kBarKvEmpty + gLast % NS), (gLast / NS) & 1, wc, 7);
+        } else {  // P.V of the next block cannot finish before this warp has written its P
+          wait_bar(bar(kBarPvDone + 2 * t), (it - 1) & 1, wc, 7);
+        }
         ptx::tc_fence_after();
         const float inv = (l > 0.f) ? (1.f / l) : 0.f;
         const int gp = 1 << p.packShift;
@@ -883,9 +922,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(bar(kBarOFree + t));
           }
-          if (kSplit && !whole_tile(p, w, t)) {
-            if (valid && ch * 32 < p.headDim) store_part(p, w, part_of(w), qpos, head, ch * 32, o, inv);
-          } else if (valid && ch * 32 < p.headDim) {
+          if constexpr (kSplit) {
+            if (!whole_tile(p, w, t)) {
+              if (valid) store_part(p, w, qpos, head, ch * 32, o, inv);
+              continue;
+            }
+          }
+          if (valid && ch * 32 < p.headDim) {
 #pragma unroll
             for (int g = 0; g < 4; g++) {
               uint4 q;
@@ -965,9 +1008,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             }
           }
           const int hdOff = o_chunk_offset<HDP, kPair>(ch);  // a constant once the loop is unrolled
-          if (kSplit && !whole_tile(p, w, t)) {
-            if (valid && hdOff < p.headDim) store_part(p, w, part_of(w), qpos, head, hdOff, o, inv);
-          } else if (valid && hdOff < p.headDim) {
+          if constexpr (kSplit) {
+            if (!whole_tile(p, w, t)) {
+              if (valid) store_part(p, w, qpos, head, hdOff, o, inv);
+              continue;
+            }
+          }
+          if (valid && hdOff < p.headDim) {
 #pragma unroll
             for (int g = 0; g < 4; g++) {
               uint4 q;
@@ -1349,7 +1396,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             blkIdx = i >> 1;
           }
           const CUtensorMap* tm = isV ? mapV : mapK;
-          const int row = w.kvRowTma + (kSplit ? part_of(w) * p.partBlocks + blkIdx : blkIdx) * kBlockN;
+          int row = w.kvRowTma + blkIdx * kBlockN;
+          if constexpr (kSplit) row += w.part * p.partBlocks * kBlockN;
           if constexpr (kPair) {
             // This CTA's half of the block, counted on rank 0's barrier together with the other half.
             // K: keys [64 rank, 64 rank + 64), all of the head dim (the K map's box is 64 rows high);

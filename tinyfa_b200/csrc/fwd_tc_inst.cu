@@ -67,7 +67,7 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
   const bool varlen = (pr.cuQ != nullptr);
   constexpr bool kBf = (TFA_BF16 != 0);
   auto kernel = varlen ? tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeVarlen> : tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixed>;
-  bool solo = false;  // one Q tile per CTA, two CTAs per SM (padded head dim 64 only)
+  bool solo = false;  // one Q tile per CTA, two CTAs per SM (padded head dim 64; 128 with key ranges)
   int kNT = C::kNT, smemBytes = C::kSmemBytes, threads = tc::kThreads;
 #if TFA_HDP == 128
   // head dim 96 has MMAs of its own shape in the 128-wide kernel (6 of 8 k-steps, 96 output columns)
@@ -99,16 +99,11 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
 
   const bool parts = split.parts > 1;  // key ranges: few query tiles, long keys (fixed length)
   if (parts) {
-#if TFA_HDP == 64
-    kernel = pr.headDim == 32 ? tc::fwd_tc_kernel<64, kBf, tc::kModeFixedSplit, true, 32> : tc::fwd_tc_kernel<64, kBf, tc::kModeFixedSplit, true>;
+#if TFA_HDP <= 128
     solo = true;
     kNT = 1;
-    smemBytes = tc::CfgSolo64::kSmemBytes;
+    smemBytes = TFA_HDP == 64 ? tc::CfgSolo64::kSmemBytes : tc::CfgSolo128::kSmemBytes;
     threads = tc::kThreadsSolo;
-#elif TFA_HDP == 128
-    kernel = pr.headDim == 96 ? tc::fwd_tc_kernel<128, kBf, tc::kModeFixedSplit, false, 96> : tc::fwd_tc_kernel<128, kBf, tc::kModeFixedSplit>;
-#else
-    kernel = tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit>;
 #endif
   }
 
@@ -143,8 +138,21 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
     attrErr[device] = cudaSuccess;
     bigAttr(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixed>);
     bigAttr(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeVarlen>);
-#if TFA_HDP != 64
+#if TFA_HDP >= 192
     bigAttr(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit>);
+#endif
+#if TFA_HDP <= 128
+    // the two-CTAs-per-SM forms: 99 KB each, and the largest shared-memory carve-out so that two fit
+    auto soloAttr = [&](auto k) {
+      if (attrErr[device] != cudaSuccess) return;
+      constexpr int bytes = TFA_HDP == 64 ? tc::CfgSolo64::kSmemBytes : tc::CfgSolo128::kSmemBytes;
+      attrErr[device] = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      if (attrErr[device] == cudaSuccess) {
+        attrErr[device] = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      }
+    };
+    soloAttr(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit, true>);
+    soloAttr(tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit, true, TFA_HDP == 64 ? 32 : 96>);
 #endif
 #if TFA_HDP >= 192
     if (attrErr[device] == cudaSuccess) {
@@ -155,26 +163,15 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
 #if TFA_HDP == 128
     bigAttr(tc::fwd_tc_kernel<128, kBf, tc::kModeFixed, false, 96>);
     bigAttr(tc::fwd_tc_kernel<128, kBf, tc::kModeVarlen, false, 96>);
-    bigAttr(tc::fwd_tc_kernel<128, kBf, tc::kModeFixedSplit, false, 96>);
 #endif
 #if TFA_HDP == 64
     bigAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedNoMask>);
-    // the two-CTAs-per-SM form: 99 KB each, and the largest shared-memory carve-out so that two fit
-    auto soloAttr = [&](auto k) {
-      if (attrErr[device] != cudaSuccess) return;
-      attrErr[device] = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::CfgSolo64::kSmemBytes);
-      if (attrErr[device] == cudaSuccess) {
-        attrErr[device] = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-      }
-    };
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixed, true>);
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeVarlen, true>);
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedNoMask, true>);
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixed, true, 32>);
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeVarlen, true, 32>);
     soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedNoMask, true, 32>);
-    soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedSplit, true>);
-    soloAttr(tc::fwd_tc_kernel<64, kBf, tc::kModeFixedSplit, true, 32>);
 #endif
   });
   if (attrErr[device] != cudaSuccess) {
@@ -217,16 +214,11 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
   p.numUnits = pr.headsQ / gp;
   const long long numItems = (long long)p.numPairs * p.numUnits * pr.batch;
   const long long numWork = numItems * split.parts;
-  p.partBlocks = split.partBlocks;
-  p.partO = split.partO;
-  p.partLse = split.partLse;
-  p.rows = pr.totalQ * pr.headsQ;
   if (numWork > 0x7FFFFFFFll) {
     set_error_string("too many work items (%lld)", numWork);
     return kTooLarge;
   }
   p.numWork = (int)numWork;
-  p.numItems = (int)numItems;
   // Causal problems: heaviest query tile pairs first inside chunks of (head unit, batch) entries.  A chunk is as wide
   // as the KV heads whose K and V fit a quarter of the L2 (32 MB) together, and at least wide enough to hold two
   // items per SM.  Option "work_order": -1 this rule, 0 pair index fastest, n > 0 chunks of n entries.
@@ -291,6 +283,20 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
     const long long clusters = numWork < maxClusters[device] ? numWork : maxClusters[device];
     cfg.gridDim = dim3((unsigned)(2 * clusters));
     e = cudaLaunchKernelEx(&cfg, kernel, tmQ, tmK, tmV, p);
+  } else if (parts) {
+    TcPartParams pp;
+    static_cast<TcParams&>(pp) = p;
+    pp.partBlocks = split.partBlocks;
+    pp.numItems = (int)numItems;
+    pp.rows = pr.totalQ * pr.headsQ;
+    pp.partO = split.partO;
+    pp.partLse = split.partLse;
+    auto partKernel = tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit, (TFA_HDP <= 128)>;
+#if TFA_HDP <= 128
+    if (pr.headDim != TFA_HDP) partKernel = tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit, true, TFA_HDP == 64 ? 32 : 96>;
+#endif
+    partKernel<<<dim3((unsigned)ctas), threads, smemBytes, pr.stream>>>(tmQ, tmK, tmV, pp);
+    e = cudaGetLastError();
   } else {
     kernel<<<dim3((unsigned)ctas), threads, smemBytes, pr.stream>>>(tmQ, tmK, tmV, p);
     e = cudaGetLastError();
