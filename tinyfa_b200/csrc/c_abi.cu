@@ -372,13 +372,8 @@ static int dispatch_fp32(const FwdProblem& p) {
   const int opt = g_optFp32Tc.load();
   // an explicit choice of the CUDA-core form (option "fp32_t8") is kept
   if (opt == 0 || (opt < 0 && g_optFp32T8.load() != 1) || !fp32tc_applicable(p, opt)) return launch_fwd_fp32(p);
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   int device = 0;
-  if (cudaStreamIsCapturing(p.stream, &cap) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
-    set_error_string("cudaStreamIsCapturing: %s", cudaGetErrorString(cudaGetLastError()));
-    return kCudaError;
-  }
-  if (cap != cudaStreamCaptureStatusNone) return launch_fwd_fp32(p);
+  if (!p.overlap || cudaGetDevice(&device) != cudaSuccess) return launch_fwd_fp32(p);  // under capture
   cudaMemPool_t pool = scratch_pool(device);
   void* ws = nullptr;
   if (pool == nullptr || cudaMallocFromPoolAsync(&ws, fp32tc_workspace_bytes(p), pool, p.stream) != cudaSuccess) {
@@ -489,14 +484,9 @@ static int dispatch_tc(const FwdProblem& p) {
   const int ps = pick_pack_shift(p);
   TcSplit split = tc_split_plan(p, ps);
   if (split.parts > 1) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     int device = 0;
-    if (cudaStreamIsCapturing(p.stream, &cap) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
-      set_error_string("cudaStreamIsCapturing: %s", cudaGetErrorString(cudaGetLastError()));
-      return kCudaError;
-    }
     const size_t rows = (size_t)p.totalQ * p.headsQ;
-    cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? scratch_pool(device) : nullptr;
+    cudaMemPool_t pool = p.overlap && cudaGetDevice(&device) == cudaSuccess ? scratch_pool(device) : nullptr;
     float* scratch = nullptr;
     if (pool != nullptr && cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), split.parts * rows * (p.headDim + 1) * sizeof(float),
                                                    pool, p.stream) == cudaSuccess) {
@@ -512,7 +502,18 @@ static int dispatch_tc(const FwdProblem& p) {
   return run_tc(p, ps, TcSplit());
 }
 
-static int dispatch(const FwdProblem& p) {
+// Captured launches stay plain: what a graph may do with programmatic dependencies is the caller's business.
+bool may_overlap(cudaStream_t stream) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return cap == cudaStreamCaptureStatusNone;
+}
+
+static int dispatch(FwdProblem p) {
+  p.overlap = may_overlap(p.stream);
   if (p.dtype == kFp32) return dispatch_fp32(p);
   const int optSplit = g_optSplitKv.load();
   if (optSplit != 0 && p.totalQ >= 0 && splitkv_applicable(p)) {

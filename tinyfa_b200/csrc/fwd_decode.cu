@@ -28,6 +28,7 @@
 
 #include "../../include/tinyfa_b200.h"
 #include "build_config.cuh"
+#include "ptx_sm100.cuh"
 #include "tfa_common.cuh"
 
 namespace tfa_b200 {
@@ -170,8 +171,8 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
   float* sM = sO + kRows * kLdO;                                          // [4][16]
   float* sL = sM + 4 * kRows;                                             // [4][16]
 
-  // the combine kernel may be launched (it waits for the end of this grid before it reads anything)
-  asm volatile("griddepcontrol.launch_dependents;");
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
   const bool even = p.runs > 0;
   int b, part;         // batch entry and partial-result slot of the current segment
   int hkv;
@@ -446,7 +447,7 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
 // O[row] = sum_s 2^(lse_s - M) O_s / sum_s 2^(lse_s - M), one CTA per output row.  Bound by the latency of two dependent
 // reads (the partials' log-sum-exps, the partials), so both are spread over the CTA: every warp reads all lse of the row,
 // D / 4 threads read one split's partial row and 128 / (D / 4) such groups take turns over the splits, four in flight each.
-// The kernel is launched while the split kernel still runs and waits for its end with griddepcontrol.wait.
+// The kernel is launched while the split kernel still runs (launch_kernel in tfa_common.cuh).
 constexpr int kCombineThreads = 128;
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kCombineThreads)
@@ -456,7 +457,8 @@ combine_kernel(const float* __restrict__ partO, const float* __restrict__ partLs
   constexpr int kVec = D / 4, kGroups = kCombineThreads / kVec;
   __shared__ float4 sAcc[kGroups][kVec];
   __shared__ float sSum[kGroups];
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
   const long long row = blockIdx.x;
   // packed input: rows past the last sequence (a Q tensor longer than cu_seqlens_q[batch]) have no partials
   if (cuQ != nullptr && row / headsQ >= cuQ[batch]) return;
@@ -516,7 +518,8 @@ __global__ void __launch_bounds__(kCombineThreads)
 combine_parts_kernel(const float* __restrict__ partO, const float* __restrict__ partLse, void* O, long long rows, int partBlocks,
                      int seqLenQ, int seqLenKV, int headsQ, int causal, int rowsPerTile) {
   constexpr int kVec = D / 4, kGroups = kCombineThreads / kVec;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
   const int g = threadIdx.x / kVec, c4 = threadIdx.x % kVec;
   const long long row = (long long)blockIdx.x * kGroups + g;
   if (g >= kGroups || row >= rows) return;
@@ -553,17 +556,9 @@ template <int D, bool kBf16>
 int launch_combine(const FwdProblem& p, int packShift, const TcSplit& split) {
   constexpr int kGroups = kCombineThreads / (D / 4);
   const long long rows = p.totalQ * p.headsQ;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3((unsigned)((rows + kGroups - 1) / kGroups));
-  cfg.blockDim = dim3(kCombineThreads);
-  cfg.stream = p.stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, combine_parts_kernel<D, kBf16>, (const float*)split.partO, (const float*)split.partLse,
-                                           p.O, rows, split.partBlocks, p.seqLenQ, p.seqLenKV, p.headsQ, p.causal, 128 >> packShift);
+  const cudaError_t e = launch_kernel(combine_parts_kernel<D, kBf16>, dim3((unsigned)((rows + kGroups - 1) / kGroups)), kCombineThreads, 0,
+                                      p.stream, p.overlap, split.partO, split.partLse, p.O, rows, split.partBlocks, p.seqLenQ,
+                                      p.seqLenKV, p.headsQ, p.causal, 128 >> packShift);
   if (e != cudaSuccess) {
     set_error_string("combine kernel launch failed: %s", cudaGetErrorString(e));
     return kCudaError;
@@ -618,21 +613,11 @@ int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* par
   p.totalQ = pr.totalQ;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   const dim3 grid = plan.runs > 0 ? dim3((unsigned)(plan.runs * pr.headsKV)) : dim3((unsigned)plan.splits, (unsigned)pr.headsKV, (unsigned)pr.batch);
-  kernel<<<grid, kThreads, kSmem, pr.stream>>>(p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_kernel(kernel, grid, kThreads, kSmem, pr.stream, pr.overlap, p);
   if (e == cudaSuccess && plan.splits > 1) {
     const long long rows = pr.totalQ * pr.headsQ;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3((unsigned)rows);
-    cfg.blockDim = dim3(kCombineThreads);
-    cfg.stream = pr.stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, combine_kernel<D, kBf16>, (const float*)partO, (const float*)partLse, pr.O, rows, plan.splits,
-                           pr.cuQ, pr.batch, pr.headsQ, p.runs, p.blocksPerEntry, p.totalBlocks, pr.seqLenQ);
+    e = launch_kernel(combine_kernel<D, kBf16>, dim3((unsigned)rows), kCombineThreads, 0, pr.stream, pr.overlap, partO, partLse,
+                      pr.O, rows, plan.splits, pr.cuQ, pr.batch, pr.headsQ, p.runs, p.blocksPerEntry, p.totalBlocks, pr.seqLenQ);
   }
   if (e != cudaSuccess) {
     set_error_string("split-KV kernel launch failed: %s", cudaGetErrorString(e));
@@ -840,6 +825,7 @@ extern "C" int tfa_b200_fwd_decode_noalloc(const void* Q, const void* K, const v
   p.headDim = headDim;
   p.causal = isCausal ? 1 : 0;
   p.stream = static_cast<cudaStream_t>(stream);
+  p.overlap = may_overlap(p.stream);
   if (!splitkv_applicable(p)) {
     set_error_string("tfa_b200_fwd_decode_noalloc handles fp16/bf16, seqLenQ * (Hq/Hkv) <= 16 and "
                      "seqLenKV >= 256 only (got dtype %d, headDim %d, seqLenQ %d, group %d, seqLenKV %d)",

@@ -17,6 +17,7 @@
 #include <mutex>
 
 #include "build_config.cuh"
+#include "ptx_sm100.cuh"
 #include "tfa_common.cuh"
 
 namespace tfa_b200 {
@@ -115,6 +116,8 @@ __global__ void __launch_bounds__(BR * 8 / kRowsPerThread) fwd_fp32_kernel(const
   float* sV = sK + kBC * LD;
   float* sP = sV + kBC * LD;
 
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
   if (gated_off<kGated>(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
@@ -367,6 +370,8 @@ __global__ void __launch_bounds__(256) fwd_fp32_lane_kernel(const Fp32Params p) 
   float* sV = sK + BC * LD;
   float* sP = sV + BC * LD;
 
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
   long long qRow0, kvRow0;
@@ -586,8 +591,7 @@ int launch_lane(const FwdProblem& pr) {
   p.gateEpoch = pr.gateEpoch;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   dim3 grid((unsigned)((pr.seqLenQ + 63) / 64), (unsigned)pr.headsQ, (unsigned)pr.batch);
-  kernel<<<grid, 256, kSmem, pr.stream>>>(p);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_kernel(kernel, grid, 256, kSmem, pr.stream, pr.overlap, p);
   if (e != cudaSuccess) {
     set_error_string("fp32 kernel launch failed: %s", cudaGetErrorString(e));
     return kCudaError;
@@ -626,6 +630,8 @@ __global__ void __launch_bounds__(256, 1) fwd_fp32_t8_kernel(const Fp32Params p)
   float* sPT = sK;  // aliased: P^T of block j overwrites K(j) once every warp is done with Q.K^T
   static_assert(BC * LDP <= BC * LD, "P^T fits the K buffer");
 
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
   if (gated_off<kGated>(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
@@ -870,8 +876,7 @@ int launch_t8(const FwdProblem& pr) {
   p.gateEpoch = pr.gateEpoch;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   dim3 grid((unsigned)((pr.seqLenQ + 127) / 128), (unsigned)pr.headsQ, (unsigned)pr.batch);
-  kernel<<<grid, 256, kSmem, pr.stream>>>(p);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_kernel(kernel, grid, 256, kSmem, pr.stream, pr.overlap, p);
   if (e != cudaSuccess) {
     set_error_string("fp32 kernel launch failed: %s", cudaGetErrorString(e));
     return kCudaError;
@@ -915,8 +920,7 @@ int launch(const FwdProblem& pr) {
   p.gateEpoch = pr.gateEpoch;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   dim3 grid((unsigned)((pr.seqLenQ + BR - 1) / BR), (unsigned)pr.headsQ, (unsigned)pr.batch);
-  kernel<<<grid, BR * 8 / kRowsPerThread, kSmem, pr.stream>>>(p);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_kernel(kernel, grid, BR * 8 / kRowsPerThread, kSmem, pr.stream, pr.overlap, p);
   if (e != cudaSuccess) {
     set_error_string("fp32 kernel launch failed: %s", cudaGetErrorString(e));
     return kCudaError;

@@ -85,6 +85,8 @@ __device__ __forceinline__ bool outside(float x) {
 
 // Bound by memory: 4 bytes read and 6 written per element.  Eight elements per thread and step.
 __global__ void __launch_bounds__(kSplitThreads) split_kernel(const SplitParams p) {
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
   bool bad = false;
 #pragma unroll
   for (int t = 0; t < 3; t++) {
@@ -152,6 +154,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
            const __grid_constant__ CUtensorMap tmV, const Params p) {
   using C = Cfg<HDP>;
   constexpr int NS = C::kStages;
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
   if (*p.flag == p.w.epoch) return;
   tc::Work w;
   if (!tc::make_work<1, kVarlen>(p.w, (int)blockIdx.x, w)) return;
@@ -543,9 +547,8 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
   sp.count[1] = sp.count[2] = pr.totalKV * pr.headsKV * pr.headDim;
   sp.flag = reinterpret_cast<int*>(ws);
   sp.epoch = epoch;
-  split_kernel<<<8 * device_num_sms(device), kSplitThreads, 0, pr.stream>>>(sp);
-  kernel<<<(unsigned)numWork, kThreads, C::kSmemBytes, pr.stream>>>(tmQ, tmK, tmV, p);
-  const cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_kernel(split_kernel, dim3(8u * (unsigned)device_num_sms(device)), kSplitThreads, 0, pr.stream, pr.overlap, sp);
+  if (e == cudaSuccess) e = launch_kernel(kernel, dim3((unsigned)numWork), kThreads, C::kSmemBytes, pr.stream, pr.overlap, tmQ, tmK, tmV, p);
   if (e != cudaSuccess) {
     set_error_string("fp32 tensor-core kernel launch failed: %s", cudaGetErrorString(e));
     return kCudaError;

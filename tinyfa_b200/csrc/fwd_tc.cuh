@@ -618,7 +618,6 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   constexpr bool kRingSig = (NT == 1 && NS >= 3);
   static_assert(!kRingSig || C::kTwoPos, "one-tile forms alternate S between two positions");
 
-  if constexpr (kSplit) asm volatile("griddepcontrol.launch_dependents;");  // the combine kernel waits for this grid's end
 
   extern __shared__ uint8_t smemRaw[];
   const uint32_t rawAddr = ptx::smem_u32(smemRaw);
@@ -694,6 +693,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   }
   if (warp == kLoadWarp && lane == 0) {
     if (kVarlen && p.devMaps != nullptr) {
+      ptx::grid_wait_previous();  // the kernel that completes the maps
       ptx::tensormap_acquire(mapQ);
       ptx::tensormap_acquire(mapK);
       ptx::tensormap_acquire(mapV);
@@ -708,6 +708,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   if constexpr (kPair) ptx::cluster_sync();  // the other CTA's barriers are initialised before anyone arrives on them
   ptx::tc_fence_after();
   const uint32_t tmem = ctl->tmemBase;
+  if (warp != kLoadWarp) ptx::grid_wait_previous();  // the loading thread: below
+  ptx::grid_allow_next();
   const WaitCtx wc{&ctl->failed, p.status, p.epoch};
 
   // Every consumer of work items (8 softmax warps, 4 epilogue warps, 2 MMA threads) reads item k from slot k & 1
@@ -1282,8 +1284,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
           // the index and hands it over through rank 1's shared memory (a mailbox per slot parity, full / empty
           // barriers); both then work out the same description and keep their own tile of it as tile 0.
           if (rank == 0) {
+            bool first = (k == 0);
             do {
-              idx = atomicAdd(p.workCounter, 1);
+              idx = first ? (int)blockIdx.x / 2 : (int)gridDim.x / 2 + atomicAdd(p.workCounter, 1);
+              first = false;
               if (idx >= p.numWork || *reinterpret_cast<volatile int*>(&ctl->failed)) idx = -1;
             } while (idx >= 0 && !make_work<2, kVarlen>(p, idx, w));
             if (k >= 2) wait_bar(bar(kBarIdxEmpty + (k & 1)), ((k >> 1) - 1) & 1, wc, 26);
@@ -1306,8 +1310,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             w.nblk[1] = 0;
           }
         } else {
+          bool first = (k == 0);
           do {
-            idx = atomicAdd(p.workCounter, 1);
+            idx = first ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(p.workCounter, 1);
+            first = false;
             if (idx >= p.numWork || *reinterpret_cast<volatile int*>(&ctl->failed)) idx = -1;
           } while (idx >= 0 && !make_work<NT, kVarlen, kSplit>(p, idx, w));
         }
@@ -1326,7 +1332,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         ptx::mbar_arrive(bar(kBarWorkFull + (k & 1)));  // release: the stores above are visible to whoever waits
         return idx >= 0;
       };
+      // Item 0 is the CTA's own index, so that a fixed-length kernel that was let in early works it out while the kernel
+      // before still runs; the counter hands out the items from gridDim.x on.  (Packed input reads its lengths from memory,
+      // and a key range that turns out empty takes its next index from the counter: both wait first.)
+      constexpr bool kEarlyItem = !kVarlen && !kSplit;
+      if constexpr (!kEarlyItem) ptx::grid_wait_previous();
       bool more = publish(0);
+      if constexpr (kEarlyItem) ptx::grid_wait_previous();
       for (int k = 0; more; k++) {
         // Item k + 1 is taken and published two blocks before the end of this item's loads: by then this thread is
         // only waiting for ring stages, and nobody waits for the atomic round trip and the divisions between two
@@ -1489,13 +1501,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     // fetches from the work counter precede its arrival on the done counter (same CTA, separated by the barrier above).
     __threadfence();
     if (atomicAdd(p.workCounter + 1, 1) == (int)gridDim.x - 1) {
-      // Every CTA stops at its first index past the end, so the work counter must now read numWork + gridDim.x.
+      // Every CTA (pair form: pair of CTAs) starts with an index of its own and stops at its first index past the end, so
+      // the work counter must now read numWork: numWork - workers indices handed out and one refusal per worker.
       // Anything else means another launch used the same counters at the same time (the host hands out a pair per
       // stream and per captured launch precisely to rule that out): report it rather than return a result with rows
       // that nobody computed.
       const int taken = *reinterpret_cast<volatile int*>(p.workCounter);
-      const int takers = kPair ? (int)gridDim.x / 2 : (int)gridDim.x;  // pair form: rank 0 of each pair takes indices
-      if (taken != p.numWork + takers && *wc.failed == 0) atomicExch(p.status, (p.epoch << 8) | 30);
+      if (taken != p.numWork && *wc.failed == 0) atomicExch(p.status, (p.epoch << 8) | 30);
       p.workCounter[0] = 0;
       p.workCounter[1] = 0;
     }

@@ -260,7 +260,7 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
   if (pair) {
     // one cluster of two CTAs per work item in flight; as many clusters as the device runs at once
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
@@ -282,6 +282,9 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
     }
     const long long clusters = numWork < maxClusters[device] ? numWork : maxClusters[device];
     cfg.gridDim = dim3((unsigned)(2 * clusters));
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = pr.overlap ? 2 : 1;
     e = cudaLaunchKernelEx(&cfg, kernel, tmQ, tmK, tmV, p);
   } else if (parts) {
     TcPartParams pp;
@@ -295,11 +298,9 @@ int TFA_NAME2(TFA_HDP, TFA_BF16)(const FwdProblem& pr, int packShift, const TcSp
 #if TFA_HDP <= 128
     if (pr.headDim != TFA_HDP) partKernel = tc::fwd_tc_kernel<TFA_HDP, kBf, tc::kModeFixedSplit, true, TFA_HDP == 64 ? 32 : 96>;
 #endif
-    partKernel<<<dim3((unsigned)ctas), threads, smemBytes, pr.stream>>>(tmQ, tmK, tmV, pp);
-    e = cudaGetLastError();
+    e = launch_kernel(partKernel, dim3((unsigned)ctas), threads, (size_t)smemBytes, pr.stream, pr.overlap, tmQ, tmK, tmV, pp);
   } else {
-    kernel<<<dim3((unsigned)ctas), threads, smemBytes, pr.stream>>>(tmQ, tmK, tmV, p);
-    e = cudaGetLastError();
+    e = launch_kernel(kernel, dim3((unsigned)ctas), threads, (size_t)smemBytes, pr.stream, pr.overlap, tmQ, tmK, tmV, p);
   }
   if (e != cudaSuccess) {
     set_error_string("kernel launch failed: %s", cudaGetErrorString(e));
