@@ -21,6 +21,8 @@ SHAPES = [  # batch, seqQ, seqKV, headsQ, headsKV: tile edges, remainders, one r
     (1, 257, 640, 6, 2),
     (2, 40, 1111, 8, 2),
     (1, 700, 300, 2, 2),
+    (1, 300, 1500, 2, 1),
+    (1, 1100, 1100, 2, 2),
 ]
 
 

@@ -60,7 +60,7 @@ int launch_combine_parts(const FwdProblem& p, int packShift, const TcSplit& spli
 
 // ---- fp32 on the tensor cores (fwd_fp32_tc.cu)
 bool fp32tc_applicable(const FwdProblem& p, int option);
-size_t fp32tc_workspace_bytes(const FwdProblem& p);
+size_t fp32tc_workspace_bytes(const FwdProblem& p, int packShift, int numSMs);
 int launch_fwd_fp32tc(const FwdProblem& p, int packShift, void* ws, int epoch);
 
 static thread_local char g_err[512] = "";
@@ -376,12 +376,13 @@ static int dispatch_fp32(const FwdProblem& p) {
   if (!p.overlap || cudaGetDevice(&device) != cudaSuccess) return launch_fwd_fp32(p);  // under capture
   cudaMemPool_t pool = scratch_pool(device);
   void* ws = nullptr;
-  if (pool == nullptr || cudaMallocFromPoolAsync(&ws, fp32tc_workspace_bytes(p), pool, p.stream) != cudaSuccess) {
+  const int ps = pick_pack_shift(p);
+  if (pool == nullptr || cudaMallocFromPoolAsync(&ws, fp32tc_workspace_bytes(p, ps, device_num_sms(device)), pool, p.stream) != cudaSuccess) {
     (void)cudaGetLastError();
     return launch_fwd_fp32(p);
   }
   const int epoch = next_epoch();
-  int rc = launch_fwd_fp32tc(p, pick_pack_shift(p), ws, epoch);
+  int rc = launch_fwd_fp32tc(p, ps, ws, epoch);
   if (rc == kOk) {
     FwdProblem rest = p;
     rest.gate = static_cast<const int*>(ws);

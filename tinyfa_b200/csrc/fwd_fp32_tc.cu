@@ -57,7 +57,7 @@ using tc::kSubTileBytes;
 
 constexpr int kThreads = 384;
 constexpr int kSplitThreads = 256;
-constexpr int kRegsIssue = 56, kRegsSoftmax = 216, kRegsOut = 232;
+constexpr int kRegsIssue = 56, kRegsSoftmax = 208, kRegsOut = 240;
 // the sum over the three warpgroups must fit the launch allocation (65536 / 384 = 168 registers a thread)
 static_assert(kRegsIssue + kRegsSoftmax + kRegsOut <= 3 * ((65536 / kThreads) / 8 * 8), "register budget");
 
@@ -146,6 +146,13 @@ struct Params {
   TcParams w;        // work description (make_work), output, mask, scale, status word
   int batches;       // batch entries of the tensor maps (1 for packed input): part i of entry b is entry i * batches + b
   const int* flag;   // inputs outside the exact range: leave the call to the CUDA-core kernel
+  // Key ranges (fixed-length input with few tiles): blockIdx.y is the range, partBlocks key blocks of the tile.  Partial
+  // results of a tile with more than one: O, row maximum, row sum relative to it.
+  int partBlocks;
+  long long rows;  // batch * seqLenQ * headsQ
+  float* partO;    // [ranges][rows][headDim]
+  float* partM;    // [ranges][rows]
+  float* partL;    // [ranges][rows]
 };
 
 template <int HDP, int kHD, bool kVarlen>
@@ -154,12 +161,21 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
            const __grid_constant__ CUtensorMap tmV, const Params p) {
   using C = Cfg<HDP>;
   constexpr int NS = C::kStages;
-  ptx::grid_wait_previous();
-  ptx::grid_allow_next();
-  if (*p.flag == p.w.epoch) return;
+  if constexpr (kVarlen) ptx::grid_wait_previous();  // the lengths are in global memory
   tc::Work w;
   if (!tc::make_work<1, kVarlen>(p.w, (int)blockIdx.x, w)) return;
-  const int n = w.nblk[0];
+  int n = w.nblk[0], j0 = 0;  // key blocks of this CTA and the first of them
+  bool whole = true;
+  if constexpr (!kVarlen) {
+    whole = n <= p.partBlocks;
+    j0 = (int)blockIdx.y * p.partBlocks;
+    n = min(n - j0, p.partBlocks);
+    // causal: a range past the end of an early tile.  Waiting first keeps this grid's end behind the end of the one before.
+    if (n <= 0) {
+      ptx::grid_wait_previous();
+      return;
+    }
+  }
 
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sQ = ptx::smem_u32(smem);
@@ -200,9 +216,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
   ptx::tc_fence_after();
   const uint32_t tmem = ctl->tmemBase;
   const tc::WaitCtx wc{&ctl->failed, p.w.status, p.w.epoch};
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
+  const bool skip = (*p.flag == p.w.epoch);  // left to the CUDA-core kernel
   constexpr uint32_t kPLoCol = 256, kOCol = 384;
 
-  if (warp < 4) {
+  if (skip) {
+    // straight to the end
+  } else if (warp < 4) {
     ptx::setmaxnreg_dec<kRegsIssue>();
     const bool isV = warp >= 2;  // which of the two streams
     const uint32_t ring = sKV + (isV ? NS * C::kTileBytes : 0u);
@@ -231,7 +252,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
 #pragma unroll
           for (int a = 0; a < C::kSub; a++) {
             ptx::tma_load_4d(ring + s * C::kTileBytes + a * kSubTileBytes, tm, bar(full + s), a * 64, w.hkv,
-                             w.kvRowTma + j * kBlockN, part * p.batches + w.batchTma);
+                             w.kvRowTma + (j0 + j) * kBlockN, part * p.batches + w.batchTma);
           }
         }
       }
@@ -324,7 +345,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
       ptx::tmem_wait_ld();
 #pragma unroll
       for (int q = 0; q < 4; q++) ptx::tmem_ld_fence(v[q]);
-      const int kbase = j * kBlockN;
+      const int kbase = (j0 + j) * kBlockN;
       if ((kbase + kBlockN > w.skv) || (p.w.causal && (kbase + kBlockN - 1 > w.qlo[0]))) {
         int lim = w.skv - kbase;
         if (p.w.causal) lim = min(lim, qpos - kbase + 1);
@@ -379,6 +400,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
       l = l * scale + (s2.x + s2.y);
     }
     ctl->sum[r] = l;
+    if (!whole && qpos < w.sq) {
+      const long long row = blockIdx.y * p.rows + (w.qRow0 + qpos) * p.w.headsQ + (w.unit << p.w.packShift) + (r & ((1 << p.w.packShift) - 1));
+      p.partM[row] = m;
+      p.partL[row] = l;
+    }
     __syncwarp();
     if (lane == 0) ptx::mbar_arrive(bar(kBarSumFull));
   } else {
@@ -416,11 +442,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     }
     tc::wait_bar(bar(kBarSumFull), 0, wc, 49);
     const float l = ctl->sum[r];
-    const float inv = (l > 0.f) ? (1.f / l) : 0.f;
+    const float inv = !whole ? 1.f : (l > 0.f) ? (1.f / l) : 0.f;
     const int qpos = w.qlo[0] + (r >> p.w.packShift);
     const int head = (w.unit << p.w.packShift) + (r & ((1 << p.w.packShift) - 1));
     if (qpos < w.sq) {
-      float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.w.O) + ((w.qRow0 + qpos) * p.w.headsQ + head) * (long long)kHD);
+      const long long row = (w.qRow0 + qpos) * p.w.headsQ + head;
+      float4* dst = reinterpret_cast<float4*>(whole ? reinterpret_cast<float*>(p.w.O) + row * kHD : p.partO + (blockIdx.y * p.rows + row) * kHD);
 #pragma unroll
       for (int i = 0; i < kHD / 4; i++) {
         dst[i] = make_float4(o[2 * i].x * inv, o[2 * i].y * inv, o[2 * i + 1].x * inv, o[2 * i + 1].y * inv);
@@ -435,6 +462,45 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, 512);
   }
+}
+
+// Adds up the key ranges of the tiles that have several: D / 4 threads per row.
+constexpr int kMergeThreads = 128;
+template <int kHD>
+__global__ void __launch_bounds__(kMergeThreads) merge_kernel(const Params p) {
+  constexpr int kVec = kHD / 4, kGroups = kMergeThreads / kVec;
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
+  const int g = threadIdx.x / kVec, c4 = threadIdx.x % kVec;
+  const long long row = (long long)blockIdx.x * kGroups + g;
+  if (*p.flag == p.w.epoch || g >= kGroups || row >= p.rows) return;
+  int blocks = (p.w.seqLenKV + kBlockN - 1) / kBlockN;
+  if (p.w.causal) {  // key blocks of this row's query tile, as in make_work
+    const int rowsPerTile = kBlockM >> p.w.packShift;
+    const int tile = (int)(row / p.w.headsQ % p.w.seqLenQ) / rowsPerTile;
+    blocks = min(blocks, (min((tile + 1) * rowsPerTile, p.w.seqLenQ) + kBlockN - 1) / kBlockN);
+  }
+  const int parts = (blocks + p.partBlocks - 1) / p.partBlocks;
+  if (parts == 1) return;  // the attention kernel has written the output
+  float M = -INFINITY;  // finite after range 0: key 0 is seen by every row
+#pragma unroll 4
+  for (int s = 0; s < parts; s++) M = fmaxf(M, p.partM[s * p.rows + row]);
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float l = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < parts; s++) {
+    const long long i = s * p.rows + row;
+    const float4 v = *reinterpret_cast<const float4*>(p.partO + i * kHD + c4 * 4);
+    const float f = tc::ex2((p.partM[i] - M) * p.w.scaleLog2);
+    l = fmaf(p.partL[i], f, l);
+    acc.x = fmaf(v.x, f, acc.x);
+    acc.y = fmaf(v.y, f, acc.y);
+    acc.z = fmaf(v.z, f, acc.z);
+    acc.w = fmaf(v.w, f, acc.w);
+  }
+  const float inv = (l > 0.f) ? (1.f / l) : 0.f;
+  *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.w.O) + row * kHD + c4 * 4) =
+      make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
 }
 
 // ---------------------------------------------------------------------------------------------------- host
@@ -458,17 +524,41 @@ static int make_map(CUtensorMap* m, const void* base, long long batches, long lo
   return kOk;
 }
 
-struct Layout {
-  size_t q, k, v, bytes;  // byte offsets of the parts behind the flag
+// Key ranges for fixed-length input with fewer query tiles than half of the SMs: as many as fill the GPU, at least two
+// blocks each, where that saves more than the two microseconds a block takes less than the merge kernel costs.
+struct Ranges {
+  int parts = 1, blocks = 0x7FFFFFFF;  // ranges, key blocks of each
 };
-static Layout layout(const FwdProblem& pr) {
+static Ranges plan_ranges(const FwdProblem& pr, int packShift, int numSMs) {
+  Ranges r;
+  if (pr.cuQ != nullptr) return r;
+  const int rows = kBlockM >> packShift;
+  const long long tiles = (long long)((pr.seqLenQ + rows - 1) / rows) * (pr.headsQ >> packShift) * pr.batch;
+  const int seen = pr.causal && pr.seqLenQ < pr.seqLenKV ? pr.seqLenQ : pr.seqLenKV;
+  const int n = (seen + kBlockN - 1) / kBlockN;
+  long long parts = numSMs / tiles;
+  if (parts > n / 2) parts = n / 2;
+  if (parts < 2) return r;
+  const int blocks = (int)((n + parts - 1) / parts);
+  if (n - blocks < 3) return r;
+  r.blocks = blocks;
+  r.parts = (n + blocks - 1) / blocks;
+  return r;
+}
+
+struct Layout {
+  size_t q, k, v, part, partRows, bytes;  // byte offsets of the parts behind the flag, and of the partial results
+};
+static Layout layout(const FwdProblem& pr, const Ranges& ranges) {
   auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
   const size_t q = (size_t)pr.totalQ * pr.headsQ * pr.headDim * 6, kv = (size_t)pr.totalKV * pr.headsKV * pr.headDim * 6;
   Layout l;
   l.q = 1024;
   l.k = l.q + up(q);
   l.v = l.k + up(kv);
-  l.bytes = l.v + up(kv);
+  l.part = l.v + up(kv);
+  l.partRows = ranges.parts > 1 ? (size_t)ranges.parts * pr.totalQ * pr.headsQ : 0;
+  l.bytes = l.part + l.partRows * (pr.headDim + 2) * sizeof(float);
   return l;
 }
 
@@ -491,7 +581,8 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
     set_error_string("cudaFuncSetAttribute(%d bytes): %s", C::kSmemBytes, cudaGetErrorString(attrErr[device]));
     return kCudaError;
   }
-  const Layout lay = layout(pr);
+  const Ranges ranges = plan_ranges(pr, packShift, device_num_sms(device));
+  const Layout lay = layout(pr, ranges);
   const int gp = 1 << packShift, rowsPerTile = kBlockM >> packShift;
   const long long nb = varlen ? 1 : pr.batch;
   const long long rowsQ = varlen ? pr.totalQ : pr.seqLenQ, rowsKV = varlen ? pr.totalKV : pr.seqLenKV;
@@ -533,6 +624,11 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
     if (width < minWidth) width = minWidth;
     p.w.chunk = (int)(width < per ? width : per);
   }
+  p.partBlocks = ranges.blocks;
+  p.rows = pr.totalQ * pr.headsQ;
+  p.partO = reinterpret_cast<float*>(ws + lay.part);
+  p.partM = p.partO + lay.partRows * kHD;
+  p.partL = p.partM + lay.partRows;
   p.batches = (int)nb;
   p.flag = reinterpret_cast<const int*>(ws);
 
@@ -548,7 +644,11 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
   sp.flag = reinterpret_cast<int*>(ws);
   sp.epoch = epoch;
   cudaError_t e = launch_kernel(split_kernel, dim3(8u * (unsigned)device_num_sms(device)), kSplitThreads, 0, pr.stream, pr.overlap, sp);
-  if (e == cudaSuccess) e = launch_kernel(kernel, dim3((unsigned)numWork), kThreads, C::kSmemBytes, pr.stream, pr.overlap, tmQ, tmK, tmV, p);
+  if (e == cudaSuccess) e = launch_kernel(kernel, dim3((unsigned)numWork, (unsigned)ranges.parts), kThreads, C::kSmemBytes, pr.stream, pr.overlap, tmQ, tmK, tmV, p);
+  if (e == cudaSuccess && ranges.parts > 1) {
+    constexpr int kGroups = kMergeThreads / (kHD / 4);
+    e = launch_kernel(merge_kernel<kHD>, dim3((unsigned)((p.rows + kGroups - 1) / kGroups)), kMergeThreads, 0, pr.stream, pr.overlap, p);
+  }
   if (e != cudaSuccess) {
     set_error_string("fp32 tensor-core kernel launch failed: %s", cudaGetErrorString(e));
     return kCudaError;
@@ -571,7 +671,9 @@ bool fp32tc_applicable(const FwdProblem& p, int option) {
   return (ctas + 147) / 148 * blocks * p.headDim >= 384;
 }
 
-size_t fp32tc_workspace_bytes(const FwdProblem& p) { return fp32tc::layout(p).bytes; }
+size_t fp32tc_workspace_bytes(const FwdProblem& p, int packShift, int numSMs) {
+  return fp32tc::layout(p, fp32tc::plan_ranges(p, packShift, numSMs)).bytes;
+}
 
 // Enqueues the split and the attention kernel.  *ws begins with the word that reads `epoch` when the call is left to the
 // CUDA-core kernel.
