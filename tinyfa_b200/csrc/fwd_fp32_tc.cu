@@ -658,17 +658,17 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
 
 }  // namespace fp32tc
 
-// Head dims up to 128 and a known number of rows.  By size: the CUDA-core kernel takes about D / 16 us per 64-key block
-// and wave of 64-row CTAs, this path about 24 us at least (four launches and an allocation).  Measured on both sides of
-// the line, us per call (CUDA cores, tensor cores), 16 heads where not given: D = 128 S128 x 4 heads 20.8, 24.1; S256 x 4
-// heads 37, 27; D = 96 S256 30, 26; D = 64 S256 22.8, 23.8, S512 43, 30; D = 32 S512 27, 28, S1024 x 8 heads 51, 42.
+// Head dims up to 128 and a known number of rows.  By size: the CUDA-core kernel takes about D / 20 us per 64-key block
+// and wave of 64-row CTAs, this path about 14 us at least (three or four launches and an allocation).  Measured on both
+// sides of the line, us per call (CUDA cores, tensor cores): D = 128 S64 B8 8 heads 10.9, 16.7; S128 4 heads 18.6, 15.4; D = 96
+// S128 15.2, 16.2; S256 27.7, 19.0; D = 64 S128 11.7, 13.6; S256 21.2, 15.7; D = 32 S256 13.7, 14.9; S512 25.4, 20.8.
 bool fp32tc_applicable(const FwdProblem& p, int option) {
   if (!TFA_HAVE_FP32 || p.dtype != kFp32 || p.headDim > 128 || p.totalQ < 0 || p.totalKV < 0) return false;
   if (option > 0) return true;
   const int seen = p.causal ? (p.seqLenQ < p.seqLenKV ? p.seqLenQ : p.seqLenKV) : p.seqLenKV;
   const long long blocks = (seen + 63) / 64;
   const long long ctas = (long long)((p.seqLenQ + 63) / 64) * p.headsQ * p.batch;
-  return (ctas + 147) / 148 * blocks * p.headDim >= 384;
+  return (ctas + 147) / 148 * blocks * p.headDim >= 256;
 }
 
 size_t fp32tc_workspace_bytes(const FwdProblem& p, int packShift, int numSMs) {
