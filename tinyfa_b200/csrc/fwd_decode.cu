@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
     if (part != p.splits - 1) keyEnd = min(key0 + p.keysPerSplit, keyEnd);
     count = (keyEnd > key0) ? (keyEnd - key0 + kBlockKeys - 1) / kBlockKeys : 0;
   }
-  const int nRows = sq * p.group;  // <= 16 by dispatch
+  // <= 16 by dispatch; packed input may hold a sequence longer than the caller's maximum: its further rows are not computed
+  const int nRows = min(sq * p.group, kRows);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
 
