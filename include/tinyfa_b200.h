@@ -66,6 +66,15 @@ int tfa_b200_fwd_varlen(const void* Q, const void* K, const void* V, void* O, co
                         long long totalQ, long long totalKV, int numHeadsQ, int numHeadsKV, int headDim,
                         int isCausal, void* stream);
 
+/*
+ * Zeroes the rows of a packed O [totalQ, numHeadsQ, headDim] that tfa_b200_fwd_varlen with the same arguments may leave
+ * untouched: those of sequences without keys, those past maxSeqLenQ in a longer sequence, and those outside
+ * [cuSeqLensQ[0], cuSeqLensQ[batchSize]).  Enqueued on `stream` ahead of the forward call it gives an uninitialised O the
+ * contents of a zero-filled one (reference csrc/binding/flash_attn_binding.cu:148) without writing every row twice.
+ */
+int tfa_b200_varlen_zero(void* O, const int* cuSeqLensQ, const int* cuSeqLensKV, int dtype, int batchSize, int maxSeqLenQ,
+                         long long totalQ, int numHeadsQ, int headDim, void* stream);
+
 /* Replaces tfa::isHeadDimCompiled (reference csrc/flash_attn/config.cuh:102-131): 1 for 32/64/96/128/192/256. */
 int tfa_b200_head_dim_supported(int headDim);
 

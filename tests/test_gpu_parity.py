@@ -767,3 +767,21 @@ def test_no_bounded_wait_gave_up():
     """Runs last in this file: every kernel launched above finished through its normal path."""
     site = ctypes.c_int(0)
     assert _lib.load().tfa_b200_device_status(ctypes.byref(site)) == 0, site.value
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_packed_rows_nobody_computes_are_zero(dtype):
+    """Sequences without keys, rows before the first and after the last sequence, rows past the stated maximum: zero, in an
+    output whose memory held something else before; every other row as in a call on that sequence alone."""
+    cu_q = torch.tensor([3, 10, 10, 410, 421], dtype=torch.int32, device="cuda")
+    cu_kv = torch.tensor([0, 50, 90, 90, 390], dtype=torch.int32, device="cuda")
+    Q, K, V = (torch.randn(n, h, 64, device="cuda").to(dtype) for n, h in ((430, 4), (400, 2), (400, 2)))
+    want = torch.zeros(Q.shape, device="cuda")
+    for a, b, c, d in ((3, 10, 0, 50), (410, 421, 90, 390)):
+        want[a:b] = tf.flash_attn_forward(Q[None, a:b], K[None, c:d], V[None, c:d])[0].float()
+    for _ in range(3):
+        junk = torch.full(Q.shape, float("nan"), device="cuda", dtype=dtype)
+        del junk  # the allocator hands this block out again
+        out = tf.flash_attn_varlen_forward(Q, K, V, cu_q, cu_kv, 400, 300).float()
+        assert torch.isfinite(out).all()
+        assert (out - want).abs().max() <= (2e-3 if dtype == torch.float16 else 5e-6)

@@ -23,6 +23,7 @@ STATUS_NAMES = {
 EXPORTED_SYMBOLS = (
     "tfa_b200_fwd",
     "tfa_b200_fwd_varlen",
+    "tfa_b200_varlen_zero",
     "tfa_b200_head_dim_supported",
     "tfa_b200_last_error_string",
     "tfa_b200_device_status",
@@ -50,6 +51,8 @@ def load():
     lib.tfa_b200_fwd.restype = ci
     lib.tfa_b200_fwd_varlen.argtypes = [vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ll, ll, ci, ci, ci, ci, vp]
     lib.tfa_b200_fwd_varlen.restype = ci
+    lib.tfa_b200_varlen_zero.argtypes = [vp, vp, vp, ci, ci, ci, ll, ci, ci, vp]
+    lib.tfa_b200_varlen_zero.restype = ci
     lib.tfa_b200_head_dim_supported.argtypes = [ci]
     lib.tfa_b200_head_dim_supported.restype = ci
     lib.tfa_b200_last_error_string.argtypes = []

@@ -124,17 +124,25 @@ def _check_varlen(Q, K, V, cu_seqlens_q, cu_seqlens_kv):
 
 
 def _run_varlen(lib, device, Q, K, V, cu_seqlens_q, cu_seqlens_kv, max_seqlen_q, max_seqlen_kv, code, is_causal):
-    O = torch.zeros_like(Q)  # sequences without keys keep zeros (binding:148)
     batch = cu_seqlens_q.shape[0] - 1
-    if batch > 0:
-        total_q, heads_q, head_dim = Q.shape
-        total_kv, heads_kv, _ = K.shape
-        rc = lib.tfa_b200_fwd_varlen(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), cu_seqlens_q.data_ptr(),
-                                     cu_seqlens_kv.data_ptr(), code, batch, int(max_seqlen_q), int(max_seqlen_kv),
-                                     total_q, total_kv, heads_q, heads_kv, head_dim, 1 if is_causal else 0,
-                                     _raw_stream(device))
+    total_q, heads_q, head_dim = Q.shape
+    total_kv, heads_kv, _ = K.shape
+    max_q, max_kv = int(max_seqlen_q), int(max_seqlen_kv)
+    if batch <= 0:
+        return torch.zeros_like(Q)
+    cu_q, cu_kv, stream = cu_seqlens_q.data_ptr(), cu_seqlens_kv.data_ptr(), _raw_stream(device)
+    if max_q > 0 and max_kv > 0 and total_q > 0 and total_kv > 0:
+        # Rows that no kernel writes (sequences without keys and the like) are zero (binding:148); the others are written once.
+        O = torch.empty_like(Q)
+        rc = lib.tfa_b200_varlen_zero(O.data_ptr(), cu_q, cu_kv, code, batch, max_q, total_q, heads_q, head_dim, stream)
         if rc != 0:
             _lib.check(rc, "flash_attn_varlen_forward")
+    else:
+        O = torch.zeros_like(Q)
+    rc = lib.tfa_b200_fwd_varlen(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), cu_q, cu_kv, code, batch, max_q, max_kv,
+                                 total_q, total_kv, heads_q, heads_kv, head_dim, 1 if is_causal else 0, stream)
+    if rc != 0:
+        _lib.check(rc, "flash_attn_varlen_forward")
     return O
 
 

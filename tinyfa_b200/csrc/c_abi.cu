@@ -228,6 +228,26 @@ __global__ void patch_varlen_maps(const __grid_constant__ CUtensorMap mq, const 
   for (int i = 0; i < 3; i++) ptx::tensormap_publish(out + i, ptx::smem_u32(&sm[i]));
 }
 
+// Rows of a packed output that the attention kernels do not write (tfa_b200_varlen_zero).  Grid: (batch + 1, y); index
+// `batch` stands for the rows before the first and after the last sequence.  rowChunks: 16-byte pieces of a row.
+__global__ void __launch_bounds__(256)
+varlen_zero_kernel(uint4* O, const int* cuQ, const int* cuKV, int batch, int maxSeqLenQ, long long totalQ, int rowChunks) {
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
+  const int b = blockIdx.x;
+  auto zero = [&](long long row0, long long row1) {
+    const long long i1 = row1 * rowChunks;
+    for (long long i = row0 * rowChunks + blockIdx.y * 256 + threadIdx.x; i < i1; i += 256ll * gridDim.y) O[i] = make_uint4(0, 0, 0, 0);
+  };
+  if (b == batch) {
+    zero(0, min((long long)cuQ[0], totalQ));
+    zero(max(cuQ[batch], 0), totalQ);
+  } else {
+    const long long q0 = cuQ[b], q1 = min((long long)cuQ[b + 1], totalQ);
+    zero(cuKV[b + 1] > cuKV[b] ? q0 + maxSeqLenQ : q0, q1);
+  }
+}
+
 int launch_patch_varlen_maps(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, CUtensorMap* out,
                              const int* cuQ, const int* cuKV, int batch, cudaStream_t stream) {
   patch_varlen_maps<<<1, 32, 0, stream>>>(mq, mk, mv, out, cuQ, cuKV, batch);
@@ -638,6 +658,27 @@ extern "C" int tfa_b200_fwd_varlen(const void* Q, const void* K, const void* V, 
   p.causal = isCausal ? 1 : 0;
   p.stream = s;
   return dispatch(p);
+}
+
+extern "C" int tfa_b200_varlen_zero(void* O, const int* cuSeqLensQ, const int* cuSeqLensKV, int dtype, int batchSize,
+                                    int maxSeqLenQ, long long totalQ, int numHeadsQ, int headDim, void* stream) {
+  int rc = validate_common(O, O, O, O, dtype, batchSize, maxSeqLenQ, maxSeqLenQ, numHeadsQ, numHeadsQ, headDim);
+  if (rc != kOk) return rc;
+  if (batchSize == 0 || totalQ <= 0) return kOk;
+  if (O == nullptr || cuSeqLensQ == nullptr || cuSeqLensKV == nullptr) {
+    set_error_string("null pointer");
+    return kBadArgument;
+  }
+  if ((rc = check_device()) != kOk) return rc;
+  const int rowChunks = (int)((long long)numHeadsQ * headDim * (dtype == kFp32 ? 4 : 2) / 16);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = launch_kernel(varlen_zero_kernel, dim3((unsigned)batchSize + 1, 16), 256, 0, s, may_overlap(s),
+                                      static_cast<uint4*>(O), cuSeqLensQ, cuSeqLensKV, batchSize, maxSeqLenQ, totalQ, rowChunks);
+  if (e != cudaSuccess) {
+    set_error_string("zero kernel launch failed: %s", cudaGetErrorString(e));
+    return kCudaError;
+  }
+  return kOk;
 }
 
 extern "C" int tfa_b200_head_dim_supported(int headDim) { return head_dim_compiled(headDim) ? 1 : 0; }
