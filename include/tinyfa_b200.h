@@ -105,7 +105,7 @@ int tfa_b200_device_status(int* site);
  *   "solo64" 0/1       head dims 32 / 64: two-tile CTAs, one per SM / one-tile CTAs, two per SM (the default)
  *   "fp32_t8" 0/1/2    fp32, head dim 128: 4 x 8 thread tiles always / 8 x 8 thread tiles for problems of at least three
  *                      CTAs per SM (the default) / 8 x 8 always
- *   "fp32_tc" -1/0/1   fp32, head dims up to 128: on the tensor cores with every float as three bf16 numbers by size /
+ *   "fp32_tc" -1/0/1   fp32: on the tensor cores with every float as three bf16 numbers by size /
  *                      never / wherever it applies (not under stream capture, not for packed input of unknown totals).
  *                      Choosing a CUDA-core form with "fp32_t8" switches "by size" off.
  *   "pair_cta" -1/0/1  head dims 192 / 256, fixed-length input: clusters of two CTAs that work on two neighbouring query

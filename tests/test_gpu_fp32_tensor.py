@@ -43,7 +43,7 @@ def _inputs(B, Sq, Skv, Hq, Hkv, D, seed):
 
 
 @pytest.mark.parametrize("causal", [False, True])
-@pytest.mark.parametrize("D", [32, 64, 96, 128])
+@pytest.mark.parametrize("D", [32, 64, 96, 128, 192, 256])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_against_the_oracle_and_the_cuda_core_kernel(shape, D, causal):
     Q, K, V = _inputs(*shape, D, 7 + D + shape[1])
@@ -56,7 +56,7 @@ def test_against_the_oracle_and_the_cuda_core_kernel(shape, D, causal):
 
 
 @pytest.mark.parametrize("causal", [False, True])
-@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("D", [32, 64, 128, 192, 256])
 def test_packed_input(D, causal):
     lens_q, lens_kv = [5, 0, 200, 64, 300, 1], [40, 9, 200, 0, 511, 128]
     cu_q = np.concatenate([[0], np.cumsum(lens_q)]).astype(np.int32)

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(BR * 8 / kRowsPerThread) fwd_fp32_kernel(const
 // broadcast loads are not as cheap as one shared-memory cycle, and with 8 + BC/32 loads per 8 x BC/32 x 4 FMAs the
 // kernel is as shared-memory-bound as the other form.  P goes through shared memory, but each warp reads back only the
 // rows it wrote.  The contract is the one stated at the top of this file.
-template <int D, int BC>
+template <int D, int BC, bool kGated>
 __global__ void __launch_bounds__(256) fwd_fp32_lane_kernel(const Fp32Params p) {
   constexpr int kThreads = 256;
   constexpr int BR = 64;            // query rows per CTA
@@ -372,6 +372,7 @@ __global__ void __launch_bounds__(256) fwd_fp32_lane_kernel(const Fp32Params p) 
 
   ptx::grid_wait_previous();
   ptx::grid_allow_next();
+  if (gated_off<kGated>(p)) return;
   const int b = blockIdx.z, h = blockIdx.y;
   const int hkv = h / p.group;
   long long qRow0, kvRow0;
@@ -562,13 +563,16 @@ int launch_lane(const FwdProblem& pr) {
   constexpr int LD = D + 4;
   constexpr int kSmem = (64 * LD + 2 * BC * LD + 64 * (BC + 4)) * (int)sizeof(float);
   static_assert(kSmem <= 227 * 1024, "shared memory");
-  auto kernel = fwd_fp32_lane_kernel<D, BC>;
+  auto kernel = pr.gate != nullptr ? fwd_fp32_lane_kernel<D, BC, true> : fwd_fp32_lane_kernel<D, BC, false>;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return kCudaError;
   static std::once_flag once[64];
   static cudaError_t attrErr[64];
   std::call_once(once[device], [&] {
-    attrErr[device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    attrErr[device] = cudaFuncSetAttribute(fwd_fp32_lane_kernel<D, BC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (attrErr[device] == cudaSuccess) {
+      attrErr[device] = cudaFuncSetAttribute(fwd_fp32_lane_kernel<D, BC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    }
   });
   if (attrErr[device] != cudaSuccess) {
     set_error_string("cudaFuncSetAttribute(%d bytes): %s", kSmem, cudaGetErrorString(attrErr[device]));

@@ -464,6 +464,351 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
   }
 }
 
+// ---------------------------------------------------------------------------------------------------- head dims 192, 256
+// The same computation where three parts of a Q tile (192 KB at 256) leave no room for K and V: parts 0 and 1 of Q stay in
+// shared memory, part 2 passes through the ring once per key block, and the ring holds units of 128 rows x 128 head-dim
+// elements (the second unit of head dim 192 is half as wide).  Each unit's share of S has an accumulator of its own, [0, 128)
+// and [128, 256) of tensor memory: the tensor core cuts off what it adds below the accumulator's last bit, and one
+// accumulator for all of the head dim was further off 64 bits than the CUDA cores (8.5e-7 against 5.1e-7 at S128 D256).
+// The softmax first writes the sum (rounded to nearest, masked) over the first share, then reads it again for the
+// exponentials - 128 scores do not fit beside two output warpgroups' registers - and leaves part 0 of P over the scores
+// already read and parts 1 and 2 over the second share; P.V is at 256.  With one S position the two products and the
+// softmax of a block follow one another, so one thread issues all MMAs.  16 warps: 0 loads, 1 issues, 4-7 softmax, 8-11
+// and 12-15 output columns [0, 128) and [128, head dim).  A block moves 14 units of 32 KB from L2 for 12.3 k clocks of MMAs.
+// Measured against the CUDA-core kernels at B2 S2048 H16 (2-norm error against 64 bits): D256 3670 -> 925 us (9.9e-7 -> 3.2e-7),
+// causal D192 1599 -> 475 us (4.0e-7 -> 1.8e-7).
+template <int kHD>
+struct CfgWide {
+  static constexpr int kSub = kHD / 64;
+  static constexpr int kUnitBytes = 2 * kSubTileBytes;
+  static constexpr int kQBytes = 2 * kSub * kSubTileBytes;  // parts 0 and 1
+  static constexpr int kStages = kHD == 256 ? 3 : 4;
+  static constexpr int kSmemBytes = kQBytes + kStages * kUnitBytes + 3072;
+};
+constexpr int kThreadsWide = 512;
+constexpr int kRegsIssueW = 64, kRegsSoftmaxW = 96, kRegsOutW = 176;
+static_assert(kRegsIssueW + kRegsSoftmaxW + 2 * kRegsOutW <= 4 * ((65536 / kThreadsWide) / 8 * 8), "register budget");
+
+template <int kHD, bool kVarlen>
+__global__ void __launch_bounds__(kThreadsWide, 1)
+fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                const __grid_constant__ CUtensorMap tmV, const Params p) {
+  using C = CfgWide<kHD>;
+  constexpr int NS = C::kStages;
+  if constexpr (kVarlen) ptx::grid_wait_previous();  // the lengths are in global memory
+  tc::Work w;
+  if (!tc::make_work<1, kVarlen>(p.w, (int)blockIdx.x, w)) return;
+  int n = w.nblk[0], j0 = 0;  // key blocks of this CTA and the first of them
+  bool whole = true;
+  if constexpr (!kVarlen) {
+    whole = n <= p.partBlocks;
+    j0 = (int)blockIdx.y * p.partBlocks;
+    n = min(n - j0, p.partBlocks);
+    if (n <= 0) {  // causal: a range past the end of an early tile
+      ptx::grid_wait_previous();
+      return;
+    }
+  }
+
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sQ = ptx::smem_u32(smem);
+  const uint32_t ring = sQ + C::kQBytes;
+  if ((sQ & 1023u) != 0) {
+    if (threadIdx.x == 0) atomicExch(p.w.status, (p.w.epoch << 8) | 50);
+    return;
+  }
+  Ctl* ctl = reinterpret_cast<Ctl*>(smem + C::kQBytes + NS * C::kUnitBytes);
+  const uint32_t barBase = ptx::smem_u32(&ctl->bars[0]);
+  auto bar = [&](int slot) { return barBase + 8u * (uint32_t)slot; };
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    ptx::mbar_init(bar(kBarQFull), 1);
+    ptx::mbar_init(bar(kBarSFull), 1);
+    ptx::mbar_init(bar(kBarPReady), 4);
+    for (int i = 0; i < 4; i++) ptx::mbar_init(bar(kBarScaleFull + i), 4);
+    ptx::mbar_init(bar(kBarOFull), 1);
+    ptx::mbar_init(bar(kBarOFree), 8);
+    ptx::mbar_init(bar(kBarSumFull), 4);
+    for (int s = 0; s < NS; s++) {
+      ptx::mbar_init(bar(kBarKvFull + s), 1);
+      ptx::mbar_init(bar(kBarKvEmpty + s), 1);
+    }
+    ctl->failed = 0;
+    ptx::fence_barrier_init();
+    ptx::fence_proxy_async_smem();
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(ptx::smem_u32(&ctl->tmemBase), 512);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = ctl->tmemBase;
+  const tc::WaitCtx wc{&ctl->failed, p.w.status, p.w.epoch};
+  ptx::grid_wait_previous();
+  ptx::grid_allow_next();
+  const bool skip = (*p.flag == p.w.epoch);  // left to the CUDA-core kernel
+  constexpr uint32_t kPCol1 = 128, kPCol2 = 192, kOCol = 256;
+
+  if (skip) {
+    // straight to the end
+  } else if (warp < 4) {
+    ptx::setmaxnreg_dec<kRegsIssueW>();
+    if (warp == 0 && lane == 0) {
+      // ============================================================== TMA loads
+      const int gp = 1 << p.w.packShift;
+      ptx::mbar_arrive_expect_tx(bar(kBarQFull), C::kQBytes);
+#pragma unroll
+      for (int part = 0; part < 2; part++) {
+#pragma unroll
+        for (int a = 0; a < C::kSub; a++) {
+          ptx::tma_load_4d(sQ + (part * C::kSub + a) * kSubTileBytes, &tmQ, bar(kBarQFull), a * 64, w.unit * gp,
+                           w.qRowTma + w.qlo[0], part * p.batches + w.batchTma);
+        }
+      }
+      int ld = 0;
+      auto load = [&](const CUtensorMap* tm, int part, int h, int y, int z) {  // one unit: head-dim elements from 128 h on
+        const int s = ld % NS, slabs = min(2, C::kSub - 2 * h);
+        if (ld >= NS) tc::wait_bar(bar(kBarKvEmpty + s), ((ld / NS) - 1) & 1, wc, 41);
+        ptx::mbar_arrive_expect_tx(bar(kBarKvFull + s), slabs * kSubTileBytes);
+        for (int a = 0; a < slabs; a++) {
+          ptx::tma_load_4d(ring + s * C::kUnitBytes + a * kSubTileBytes, tm, bar(kBarKvFull + s), h * 128 + a * 64, y, z,
+                           part * p.batches + w.batchTma);
+        }
+        ld++;
+      };
+      for (int j = 0; j < n; j++) {
+        const int row = w.kvRowTma + (j0 + j) * kBlockN;
+        for (int part = 2; part >= 0; part--) {
+          for (int h = 0; h < 2; h++) {
+            if (part == 0) load(&tmQ, 2, h, w.unit * gp, w.qRowTma + w.qlo[0]);
+            load(&tmK, part, h, w.hkv, row);
+          }
+        }
+        for (int part = 2; part >= 0; part--) {
+          for (int h = 0; h < 2; h++) load(&tmV, part, h, w.hkv, row);
+        }
+      }
+    } else if (warp == 1 && lane == 0) {
+      // ============================================================== MMA issue
+      const uint32_t idQK = ptx::instr_desc_f16(1, kBlockM, kBlockN, 0, 0);
+      const uint64_t descK = ptx::smem_desc_sw128(16, 1024);
+      const uint64_t descV = ptx::smem_desc_sw128(kSubTileBytes, 1024);
+      const uint32_t kHi = (uint32_t)(descK >> 32), vHi = (uint32_t)(descV >> 32);
+      const uint32_t kLoT = (uint32_t)descK, vLoT = (uint32_t)descV;
+      int ld = 0;
+      auto unitReady = [&]() -> int {
+        const int s = ld % NS;
+        tc::wait_bar(bar(kBarKvFull + s), (ld / NS) & 1, wc, 42);
+        ptx::tc_fence_after();
+        ld++;
+        return s;
+      };
+      tc::wait_bar(bar(kBarQFull), 0, wc, 43);
+      for (int j = 0; j < n; j++) {
+        // S, whose columns hold P of block j - 1: its P.V was issued earlier by this thread, MMAs run in order
+        uint32_t accS = 0;  // bit h: the accumulator of head-dim unit h holds something
+#pragma unroll 1
+        for (int part = 2; part >= 0; part--) {
+#pragma unroll 1
+          for (int h = 0; h < 2; h++) {
+            const int q2 = part == 0 ? unitReady() : 0;
+            const int s = unitReady();
+            const uint32_t kLo = kLoT | ((ring + (uint32_t)(s * C::kUnitBytes)) >> 4);
+            const int steps = (kHD == 192 && h == 1) ? 4 : 8;
+#pragma unroll 1
+            for (int qPart = 2 - part; qPart >= 0; qPart--) {
+              const uint32_t qAddr = qPart == 2 ? ring + (uint32_t)(q2 * C::kUnitBytes)
+                                                : sQ + (uint32_t)((qPart * C::kSub + 2 * h) * kSubTileBytes);
+              const uint32_t qLo = kLoT | (qAddr >> 4);
+#pragma unroll
+              for (int kk = 0; kk < 8; kk++) {
+                const uint32_t off = (uint32_t)((kk >> 2) * kSubTileBytes + (kk & 3) * 32) >> 4;
+                if (kHD == 256 || kk < 4 || steps == 8) {
+                  ptx::mma_ss_lohi(tmem + h * 128, qLo + off, kHi, kLo + off, kHi, idQK, kk > 0 ? 1u : (accS >> h) & 1u);
+                }
+              }
+              accS |= 1u << h;
+            }
+            if (part == 0) ptx::tc_commit(bar(kBarKvEmpty + q2));
+            ptx::tc_commit(bar(kBarKvEmpty + s));
+          }
+        }
+        ptx::tc_commit(bar(kBarSFull));
+        if (j > 0) tc::wait_bar(bar(kBarOFree), (j - 1) & 1, wc, 44);
+        tc::wait_bar(bar(kBarPReady), j & 1, wc, 45);
+        uint32_t accH[2] = {0, 0};
+#pragma unroll 1
+        for (int part = 2; part >= 0; part--) {
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const uint32_t idPV = ptx::instr_desc_f16(1, kBlockM, (kHD == 192 && h == 1) ? 64 : 128, 0, 1);
+            const int s = unitReady();
+            const uint32_t vLo = vLoT | ((ring + (uint32_t)(s * C::kUnitBytes)) >> 4);
+#pragma unroll 1
+            for (int pPart = 2 - part; pPart >= 0; pPart--) {
+              const uint32_t a = tmem + (pPart == 0 ? 0u : pPart == 1 ? kPCol1 : kPCol2);
+#pragma unroll
+              for (int kk = 0; kk < kBlockN / 16; kk++) {
+                ptx::mma_ts_lohi(tmem + kOCol + h * 128, a + kk * 8, vLo + ((kk * 2048) >> 4), vHi, idPV, kk > 0 ? 1u : accH[h]);
+              }
+              accH[h] = 1;
+            }
+            ptx::tc_commit(bar(kBarKvEmpty + s));
+          }
+        }
+        ptx::tc_commit(bar(kBarOFull));
+      }
+    }
+  } else if (warp < 8) {
+    // ================================================================ softmax
+    ptx::setmaxnreg_dec<kRegsSoftmaxW>();
+    const int r = threadIdx.x & 127;
+    const uint32_t tS = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const int qpos = w.qlo[0] + (r >> p.w.packShift);
+    const float c = p.w.scaleLog2;
+    float m = -INFINITY, l = 0.f;
+    for (int j = 0; j < n; j++) {
+      tc::wait_bar(bar(kBarSFull), j & 1, wc, 46);
+      ptx::tc_fence_after();
+      const int kbase = (j0 + j) * kBlockN;
+      int lim = kBlockN;  // columns [0, lim) are real keys that are not in the future
+      if ((kbase + kBlockN > w.skv) || (p.w.causal && (kbase + kBlockN - 1 > w.qlo[0]))) {
+        lim = w.skv - kbase;
+        if (p.w.causal) lim = min(lim, qpos - kbase + 1);
+      }
+      float mNew = m;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        uint32_t v[16], v2[16];
+        ptx::tmem_ld_32x32b_x16(tS + q * 16, v);
+        ptx::tmem_ld_32x32b_x16(tS + 128 + q * 16, v2);
+        ptx::tmem_wait_ld();
+        ptx::tmem_ld_fence(v);
+        ptx::tmem_ld_fence(v2);
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(v2[i]));
+        if (lim < q * 16 + 16) {
+#pragma unroll
+          for (int i = 0; i < 16; i++) {
+            if (q * 16 + i >= lim) v[i] = 0xff800000u;  // -inf
+          }
+        }
+        float mx = tc::fmax2(__uint_as_float(v[0]), __uint_as_float(v[1]));
+#pragma unroll
+        for (int i = 2; i < 16; i += 2) mx = tc::fmax3(mx, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+        mNew = fmaxf(mNew, mx);
+        ptx::tmem_st_32x32b_x16(tS + q * 16, v);
+      }
+      ptx::tmem_wait_st();
+      const float mUse = (mNew == -INFINITY) ? 0.f : mNew;
+      const float scale = (m == -INFINITY) ? 0.f : tc::ex2((m - mUse) * c);
+      m = mNew;
+      ctl->scale[j % 3][r] = scale;
+      const float negMc = -mUse * c;
+      const float2 c2 = make_float2(c, c), negMc2 = make_float2(negMc, negMc);
+      float2 sum2 = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        uint32_t v[16];
+        ptx::tmem_ld_32x32b_x16(tS + q * 16, v);
+        ptx::tmem_wait_ld();
+        ptx::tmem_ld_fence(v);
+        uint32_t p0[8], p1[8], p2[8];
+        float2 s2 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          float2 x = tc::ffma2(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), c2, negMc2);
+          x.x = tc::ex2(x.x);
+          x.y = tc::ex2(x.y);
+          s2 = tc::fadd2(s2, x);
+          split3(x.x, x.y, p0[i >> 1], p1[i >> 1], p2[i >> 1]);
+        }
+        sum2 = tc::fadd2(sum2, s2);
+        ptx::tmem_st_32x32b_x8(tS + q * 8, p0);  // inside the columns read so far
+        ptx::tmem_st_32x32b_x8(tS + kPCol1 + q * 8, p1);
+        ptx::tmem_st_32x32b_x8(tS + kPCol2 + q * 8, p2);
+      }
+      ptx::tmem_wait_st();
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        ptx::mbar_arrive(bar(kBarPReady));
+        ptx::mbar_arrive(bar(kBarScaleFull + j % 3));
+      }
+      l = l * scale + (sum2.x + sum2.y);
+    }
+    ctl->sum[r] = l;
+    if (!whole && qpos < w.sq) {
+      const long long row = blockIdx.y * p.rows + (w.qRow0 + qpos) * p.w.headsQ + (w.unit << p.w.packShift) + (r & ((1 << p.w.packShift) - 1));
+      p.partM[row] = m;
+      p.partL[row] = l;
+    }
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(bar(kBarSumFull));
+  } else {
+    // ================================================================ output, 128 (or the last 64) columns per warpgroup
+    ptx::setmaxnreg_inc<kRegsOutW>();
+    const int r = threadIdx.x & 127;
+    const int half = (warp >= 12) ? 1 : 0;
+    const int chunks = (kHD == 192 && half == 1) ? 2 : 4;
+    const uint32_t tO = tmem + ((uint32_t)((warp & 3) * 32) << 16) + kOCol + half * 128;
+    float2 o[64];
+#pragma unroll
+    for (int i = 0; i < 64; i++) o[i] = make_float2(0.f, 0.f);
+    for (int j = 0; j < n; j++) {
+      // Slot j % 3 is published again for block j + 3, whose scores are issued behind P.V of block j + 2 and with it behind
+      // this warp's arrival on kBarOFree for block j + 1: it is never two phases behind.
+      tc::wait_bar(bar(kBarScaleFull + j % 3), (j / 3) & 1, wc, 47);
+      const float scale = ctl->scale[j % 3][r];
+      const float2 scale2 = make_float2(scale, scale);
+      tc::wait_bar(bar(kBarOFull), j & 1, wc, 48);
+      ptx::tc_fence_after();
+#pragma unroll
+      for (int ch = 0; ch < 4; ch++) {
+        if (kHD == 192 && ch >= chunks) break;
+        uint32_t t[32];
+        ptx::tmem_ld_32x32b_x32(tO + ch * 32, t);
+        ptx::tmem_wait_ld();
+        ptx::tmem_ld_fence(t);
+        if (ch == chunks - 1) {
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(bar(kBarOFree));
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          o[ch * 16 + (i >> 1)] = tc::ffma2(o[ch * 16 + (i >> 1)], scale2, make_float2(__uint_as_float(t[i]), __uint_as_float(t[i + 1])));
+        }
+      }
+    }
+    tc::wait_bar(bar(kBarSumFull), 0, wc, 49);
+    const float l = ctl->sum[r];
+    const float inv = !whole ? 1.f : (l > 0.f) ? (1.f / l) : 0.f;
+    const int qpos = w.qlo[0] + (r >> p.w.packShift);
+    const int head = (w.unit << p.w.packShift) + (r & ((1 << p.w.packShift) - 1));
+    if (qpos < w.sq) {
+      const long long row = (w.qRow0 + qpos) * p.w.headsQ + head;
+      float4* dst = reinterpret_cast<float4*>((whole ? reinterpret_cast<float*>(p.w.O) + row * kHD : p.partO + (blockIdx.y * p.rows + row) * kHD) + half * 128);
+#pragma unroll
+      for (int i = 0; i < 32; i++) {
+        if (kHD == 192 && i >= chunks * 8) break;
+        dst[i] = make_float4(o[2 * i].x * inv, o[2 * i].y * inv, o[2 * i + 1].x * inv, o[2 * i + 1].y * inv);
+      }
+    }
+  }
+
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    if (*wc.failed) __nanosleep(200000);  // a wait gave up: let whatever is still in flight drain before freeing
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, 512);
+  }
+}
+
 // Adds up the key ranges of the tiles that have several: D / 4 threads per row.
 constexpr int kMergeThreads = 128;
 template <int kHD>
@@ -562,23 +907,34 @@ static Layout layout(const FwdProblem& pr, const Ranges& ranges) {
   return l;
 }
 
-template <int HDP, int kHD>
+// The kernel of a head dim: two 128-row K / V rings up to 128, the wide form above.
+template <int kHD, bool kVarlen>
+constexpr auto kernel_of() {
+  if constexpr (kHD > 128) {
+    return fwd_wide_kernel<kHD, kVarlen>;
+  } else {
+    return fwd_kernel<(kHD <= 64 ? 64 : 128), kHD, kVarlen>;
+  }
+}
+
+template <int kHD>
 int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
-  using C = Cfg<HDP>;
+  constexpr int kSmem = kHD > 128 ? CfgWide<(kHD > 128 ? kHD : 256)>::kSmemBytes : Cfg<(kHD <= 64 ? 64 : 128)>::kSmemBytes;
+  constexpr int threads = kHD > 128 ? kThreadsWide : kThreads;
   const bool varlen = (pr.cuQ != nullptr);
-  auto kernel = varlen ? fwd_kernel<HDP, kHD, true> : fwd_kernel<HDP, kHD, false>;
+  auto kernel = varlen ? kernel_of<kHD, true>() : kernel_of<kHD, false>();
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return kCudaError;
   static std::once_flag once[64];
   static cudaError_t attrErr[64];
   std::call_once(once[device], [&] {
-    attrErr[device] = cudaFuncSetAttribute(fwd_kernel<HDP, kHD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    attrErr[device] = cudaFuncSetAttribute(kernel_of<kHD, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     if (attrErr[device] == cudaSuccess) {
-      attrErr[device] = cudaFuncSetAttribute(fwd_kernel<HDP, kHD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+      attrErr[device] = cudaFuncSetAttribute(kernel_of<kHD, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     }
   });
   if (attrErr[device] != cudaSuccess) {
-    set_error_string("cudaFuncSetAttribute(%d bytes): %s", C::kSmemBytes, cudaGetErrorString(attrErr[device]));
+    set_error_string("cudaFuncSetAttribute(%d bytes): %s", kSmem, cudaGetErrorString(attrErr[device]));
     return kCudaError;
   }
   const Ranges ranges = plan_ranges(pr, packShift, device_num_sms(device));
@@ -644,7 +1000,7 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
   sp.flag = reinterpret_cast<int*>(ws);
   sp.epoch = epoch;
   cudaError_t e = launch_kernel(split_kernel, dim3(8u * (unsigned)device_num_sms(device)), kSplitThreads, 0, pr.stream, pr.overlap, sp);
-  if (e == cudaSuccess) e = launch_kernel(kernel, dim3((unsigned)numWork, (unsigned)ranges.parts), kThreads, C::kSmemBytes, pr.stream, pr.overlap, tmQ, tmK, tmV, p);
+  if (e == cudaSuccess) e = launch_kernel(kernel, dim3((unsigned)numWork, (unsigned)ranges.parts), threads, kSmem, pr.stream, pr.overlap, tmQ, tmK, tmV, p);
   if (e == cudaSuccess && ranges.parts > 1) {
     constexpr int kGroups = kMergeThreads / (kHD / 4);
     e = launch_kernel(merge_kernel<kHD>, dim3((unsigned)((p.rows + kGroups - 1) / kGroups)), kMergeThreads, 0, pr.stream, pr.overlap, p);
@@ -658,12 +1014,13 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
 
 }  // namespace fp32tc
 
-// Head dims up to 128 and a known number of rows.  By size: the CUDA-core kernel takes about D / 20 us per 64-key block
+// A known number of rows.  By size: the CUDA-core kernel takes about D / 20 us per 64-key block
 // and wave of 64-row CTAs, this path about 14 us at least (three or four launches and an allocation).  Measured on both
 // sides of the line, us per call (CUDA cores, tensor cores): D = 128 S64 B8 8 heads 10.9, 16.7; S128 4 heads 18.6, 15.4; D = 96
-// S128 15.2, 16.2; S256 27.7, 19.0; D = 64 S128 11.7, 13.6; S256 21.2, 15.7; D = 32 S256 13.7, 14.9; S512 25.4, 20.8.
+// S128 15.2, 16.2; S256 27.7, 19.0; D = 64 S128 11.7, 13.6; S256 21.2, 15.7; D = 32 S256 13.7, 14.9; S512 25.4, 20.8; D = 192
+// S128 28.8, 23.6; D = 256 S60 8 heads 22.5, 21.2.
 bool fp32tc_applicable(const FwdProblem& p, int option) {
-  if (!TFA_HAVE_FP32 || p.dtype != kFp32 || p.headDim > 128 || p.totalQ < 0 || p.totalKV < 0) return false;
+  if (!TFA_HAVE_FP32 || p.dtype != kFp32 || p.totalQ < 0 || p.totalKV < 0) return false;
   if (option > 0) return true;
   const int seen = p.causal ? (p.seqLenQ < p.seqLenKV ? p.seqLenQ : p.seqLenKV) : p.seqLenKV;
   const long long blocks = (seen + 63) / 64;
@@ -683,19 +1040,27 @@ int launch_fwd_fp32tc(const FwdProblem& p, int packShift, void* ws, int epoch) {
   switch (p.headDim) {
 #if TFA_HAVE_HD32
     case 32:
-      return fp32tc::launch<64, 32>(p, packShift, w, epoch);
+      return fp32tc::launch<32>(p, packShift, w, epoch);
 #endif
 #if TFA_HAVE_HD64
     case 64:
-      return fp32tc::launch<64, 64>(p, packShift, w, epoch);
+      return fp32tc::launch<64>(p, packShift, w, epoch);
 #endif
 #if TFA_HAVE_HD96
     case 96:
-      return fp32tc::launch<128, 96>(p, packShift, w, epoch);
+      return fp32tc::launch<96>(p, packShift, w, epoch);
 #endif
 #if TFA_HAVE_HD128
     case 128:
-      return fp32tc::launch<128, 128>(p, packShift, w, epoch);
+      return fp32tc::launch<128>(p, packShift, w, epoch);
+#endif
+#if TFA_HAVE_HD192
+    case 192:
+      return fp32tc::launch<192>(p, packShift, w, epoch);
+#endif
+#if TFA_HAVE_HD256
+    case 256:
+      return fp32tc::launch<256>(p, packShift, w, epoch);
 #endif
     default:
       break;
