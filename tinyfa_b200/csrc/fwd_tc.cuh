@@ -1334,11 +1334,12 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       };
       // Item 0 is the CTA's own index, so that a fixed-length kernel that was let in early works it out while the kernel
       // before still runs; the counter hands out the items from gridDim.x on.  (Packed input reads its lengths from memory,
-      // and a key range that turns out empty takes its next index from the counter: both wait first.)
-      constexpr bool kEarlyItem = !kVarlen && !kSplit;
-      if constexpr (!kEarlyItem) ptx::grid_wait_previous();
+      // and a key range that turns out empty - causal - takes its next index from the counter: both wait first.)
+      bool early = !kVarlen;
+      if constexpr (kSplit) early = !p.causal || p.numItems == p.numWork;
+      if (!early) ptx::grid_wait_previous();
       bool more = publish(0);
-      if constexpr (kEarlyItem) ptx::grid_wait_previous();
+      if (early) ptx::grid_wait_previous();
       for (int k = 0; more; k++) {
         // Item k + 1 is taken and published two blocks before the end of this item's loads: by then this thread is
         // only waiting for ring stages, and nobody waits for the atomic round trip and the divisions between two
