@@ -135,7 +135,8 @@ const char* tfa_b200_version(void);
  *
  * numSplits: 0 lets the library choose, n > 0 asks for n key-range splits.  The partials need
  * numSplits * batchSize * seqLenQ * numHeadsQ * (headDim + 1) floats (none for one split); a call that needs more
- * than the array holds returns TFA_B200_TOO_LARGE and launches nothing.
+ * than the array holds returns TFA_B200_TOO_LARGE and launches nothing.  (With 0, that many is up to 32, as many as make
+ * batchSize * numHeadsKV splits fill the GPU twice; how the call is then cut is the library's choice.)
  *
  * The first call on each device resolves the array's device address (cudaGetSymbolAddress, with that device
  * current); make that first call before starting any stream capture.  All calls on a device share the one array:

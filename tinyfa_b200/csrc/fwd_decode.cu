@@ -636,6 +636,17 @@ bool splitkv_applicable(const FwdProblem& p) {
   return (long long)p.seqLenQ * group <= decode::kRows && p.seqLenKV >= 256;
 }
 
+// Key-range splits of every (batch, KV head) pair: none from one wave of pairs on, otherwise as many as fit two waves of
+// two CTAs per SM, at most 32, at least 256 keys each.
+static int splits_of_pairs(const FwdProblem& p, int numSMs) {
+  const long long pairs = (long long)p.batch * p.headsKV;
+  if (pairs >= 2ll * numSMs) return 1;
+  long long splits = 4ll * numSMs / pairs;
+  if (splits > 32) splits = 32;
+  if (splits > (p.seqLenKV + 255) / 256) splits = (p.seqLenKV + 255) / 256;
+  return splits < 1 ? 1 : (int)splits;
+}
+
 // How a call is cut.  forced > 0: that many key-range splits of every pair, on a three-dimensional grid; the same with
 // a number of its own for packed input, whose lengths the host does not know.  Fixed-length input is cut evenly: the key
 // blocks of all batch entries in a row, as many equal runs as the GPU holds at once, so that no SM waits for another at the
@@ -659,17 +670,10 @@ SplitPlan splitkv_plan(const FwdProblem& p, int numSMs, int forced) {
     plan.runs = (int)runs;
     plan.blocksPerEntry = (int)blocks;
     const long long run = total / runs;  // the shortest run; partial results per pair:
-    plan.splits = (int)(runs % p.batch == 0 ? runs / p.batch : (blocks - 2) / run + 2);
+    plan.splits = (int)(p.batch % runs == 0 ? 1 : runs % p.batch == 0 ? runs / p.batch : (blocks - 2) / run + 2);
     return plan;
   }
-  // packed input (and more pairs than the even partition is for): no split from one wave of pairs on, otherwise as many
-  // as fit two waves of two CTAs per SM, at most 32, at least 256 keys each
-  if (pairs < 2ll * numSMs) {
-    long long splits = 4ll * numSMs / pairs;
-    if (splits > 32) splits = 32;
-    if (splits > (p.seqLenKV + 255) / 256) splits = (p.seqLenKV + 255) / 256;
-    plan.splits = splits < 1 ? 1 : (int)splits;
-  }
+  plan.splits = splits_of_pairs(p, numSMs);  // packed input, and more pairs than the even partition is for
   return plan;
 }
 
@@ -836,17 +840,18 @@ extern "C" int tfa_b200_fwd_decode_noalloc(const void* Q, const void* K, const v
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   SplitPlan plan = splitkv_plan(p, sms, numSplits);
-  if (plan.runs > 0 && splitkv_scratch_floats(p, plan) > (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS) {
-    // the even partition's partials do not fit: whole pairs, as many at a time as the GPU holds
-    plan = SplitPlan{1, 0, 0};
-  }
-  const size_t need = splitkv_scratch_floats(p, plan);
-  if (need > (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS) {
+  // What the entry point accepts is stated in splits of pairs; an even partition whose partials do not fit the array gives
+  // way to whole pairs, as many at a time as the GPU holds.
+  const SplitPlan stated = {plan.runs > 0 ? splits_of_pairs(p, sms) : plan.splits, 0, 0};
+  const size_t limit = (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS, statedNeed = splitkv_scratch_floats(p, stated);
+  if (statedNeed > limit) {
     set_error_string("split-KV partials need %zu floats (%d splits x %lld rows x (%d + 1)) but the built-in scratch holds "
                      "%zu; use fewer splits or tfa_b200_fwd",
-                     need, plan.splits, (long long)p.totalQ * numHeadsQ, headDim, (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS);
+                     statedNeed, stated.splits, (long long)p.totalQ * numHeadsQ, headDim, limit);
     return kTooLarge;
   }
+  if (splitkv_scratch_floats(p, plan) > limit) plan = SplitPlan{1, 0, 0};
+  const size_t need = splitkv_scratch_floats(p, plan);
   float* scratch = nullptr;
   if ((rc = decode::static_scratch_ptr(&scratch)) != kOk) return rc;
   // Every (split, row) partial that the combine kernel reads is written by the split kernel of the same call, so
