@@ -14,7 +14,7 @@
 //   * warps are merged through shared memory, partial results through a small fp32 scratch buffer and a combine kernel
 //     that is launched while the split kernel runs (programmatic dependent launch) and reads a row's partials side by side.
 // Measured against a fixed number of splits per pair and a combine kernel that walked them (8 KV heads, D = 128, floor in
-// brackets at 6.54 TB/s): batch 1 x 32768 keys 37.8 -> 31 us (20.5), 8 x 20011 113 -> 103 (100), 40 x 5000 174 -> 135 (125), 13 x
+// brackets at 6.54 TB/s): batch 1 x 32768 keys 37.0 -> 27.8 us (20.5), 8 x 20011 111 -> 100 (100), 40 x 5000 174 -> 135 (125), 13 x
 // 8000 74 -> 74 (65), 6 x 12000 58 -> 55 (45).  What is left at small batch is launch, the first loads and the combine.
 // Numerical contract as in the main kernel (reference csrc/flash_attn/mma/softmax.cuh:67-138): scale 1/sqrt(D)
 // folded into exp2, top-left causal mask, "col >= seqLenKV" mask, P rounded to the 16-bit type before P.V, row sum

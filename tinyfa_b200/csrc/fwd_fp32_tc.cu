@@ -8,8 +8,8 @@
 // maximum, ex2.approx, fp32 row sums, P as all 24 bits (three bf16 parts), and O summed in fp32 registers with round to
 // nearest - the tensor core only ever sums the 128 keys of one block.
 //
-// Measured against the CUDA-core kernels (2-norm error against 64 bits in brackets): non-causal B2 S2048 H16 D128 1593 ->
-// 400 us (9.1e-7 -> 3.1e-7), causal B2 S1999 16 over 4 heads D64 565 -> 133 us (3.9e-7 -> 1.8e-7); on every shape tried,
+// Measured against the CUDA-core kernels (2-norm error against 64 bits in brackets): non-causal B2 S2048 H16 D128 1596 ->
+// 394 us (9.1e-7 -> 3.1e-7), causal B2 S1999 16 over 4 heads D64 563 -> 127 us (3.9e-7 -> 1.8e-7); on every shape tried,
 // short ones included, the error is below that of the CUDA-core kernels, whose sums run over all keys one at a time.
 // One pass over a block takes 7.7 k clocks at D = 128, of which the tensor pipe needs 96 x 64 = 6.1 k; with both products
 // issued by one thread it was 9.4 k.  Left: the dependency S -> softmax -> P.V -> S two blocks on (the two S buffers), the
