@@ -69,3 +69,22 @@ def test_nan_key_poisons_its_rows_and_no_others():
     assert torch.isnan(out[2, :, 4:]).all()
     out[2, :, 4:] = 0
     assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 9000, 8, 2), (2, 24, 4000, 8, 2)])  # decode runs; key ranges of the tensor-core path
+def test_back_to_back_calls_do_not_see_each_others_partials(shape):
+    """Calls in a row on one stream get the same scratch, and a combine kernel is launched while the kernel that writes its
+    partials still runs.  Inputs take turns; every result is bit for bit that of the same call made alone."""
+    B, Sq, Skv, Hq, Hkv = shape
+    sets = [[torch.randn(*s, device="cuda").bfloat16() for s in ((B, Sq, Hq, 128), (B, Skv, Hkv, 128), (B, Skv, Hkv, 128))]
+            for _ in range(2)]
+    alone = []
+    for s in sets:
+        torch.cuda.synchronize()
+        alone.append(tf.flash_attn_forward(*s))
+    torch.cuda.synchronize()
+    assert not torch.equal(*alone)
+    outs = [tf.flash_attn_forward(*sets[i % 2]) for i in range(40)]
+    tf.device_status()
+    for i, out in enumerate(outs):
+        assert torch.equal(out, alone[i % 2]), i

@@ -448,11 +448,12 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
 // O[row] = sum_s 2^(lse_s - M) O_s / sum_s 2^(lse_s - M), one CTA per output row.  Bound by the latency of two dependent
 // reads (the partials' log-sum-exps, the partials), so both are spread over the CTA: every warp reads all lse of the row,
 // D / 4 threads read one split's partial row and 128 / (D / 4) such groups take turns over the splits, four in flight each.
-// The kernel is launched while the split kernel still runs (launch_kernel in tfa_common.cuh).
+// The kernel is launched while the split kernel still runs (launch_kernel in tfa_common.cuh): the partials change during
+// its lifetime, so they are read with coherent loads and their pointers promise the compiler nothing.
 constexpr int kCombineThreads = 128;
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kCombineThreads)
-combine_kernel(const float* __restrict__ partO, const float* __restrict__ partLse, void* O,
+combine_kernel(const float* partO, const float* partLse, void* O,
                long long rows /* totalQ * Hq */, int splits, const int* cuQ, int batch, int headsQ, int runs,
                int blocksPerEntry, long long totalBlocks, int seqLenQ) {
   constexpr int kVec = D / 4, kGroups = kCombineThreads / kVec;
@@ -469,7 +470,7 @@ combine_kernel(const float* __restrict__ partO, const float* __restrict__ partLs
     if (splits == 1) return;  // the split kernel has written the output
   }
   float M = -INFINITY;
-  for (int s = threadIdx.x & 31; s < splits; s += 32) M = fmax_nan(M, partLse[(long long)s * rows + row]);
+  for (int s = threadIdx.x & 31; s < splits; s += 32) M = fmax_nan(M, __ldcg(partLse + (long long)s * rows + row));
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) M = fmax_nan(M, __shfl_xor_sync(0xffffffffu, M, off));
   if (M == -INFINITY) return;  // no keys at all for this row: leave O untouched
@@ -479,8 +480,8 @@ combine_kernel(const float* __restrict__ partO, const float* __restrict__ partLs
     float wsum = 0.f;
 #pragma unroll 4
     for (int s = g; s < splits; s += kGroups) {
-      const float lse = partLse[(long long)s * rows + row];
-      const float4 v = *reinterpret_cast<const float4*>(partO + ((long long)s * rows + row) * D + c4 * 4);
+      const float lse = __ldcg(partLse + (long long)s * rows + row);
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(partO + ((long long)s * rows + row) * D + c4 * 4));
       const float w = exp2f(lse - M);  // 0 for a split without keys, whose partial is zero
       acc.x += w * v.x;
       acc.y += w * v.y;
@@ -516,7 +517,7 @@ combine_kernel(const float* __restrict__ partO, const float* __restrict__ partLs
 // row, several rows per CTA.
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kCombineThreads)
-combine_parts_kernel(const float* __restrict__ partO, const float* __restrict__ partLse, void* O, long long rows, int partBlocks,
+combine_parts_kernel(const float* partO, const float* partLse, void* O, long long rows, int partBlocks,
                      int seqLenQ, int seqLenKV, int headsQ, int causal, int rowsPerTile) {
   constexpr int kVec = D / 4, kGroups = kCombineThreads / kVec;
   ptx::grid_wait_previous();
@@ -533,13 +534,13 @@ combine_parts_kernel(const float* __restrict__ partO, const float* __restrict__ 
   if (parts == 1) return;  // the attention kernel has written the output
   float M = -INFINITY;
 #pragma unroll 8
-  for (int s = 0; s < parts; s++) M = fmax_nan(M, partLse[s * rows + row]);
+  for (int s = 0; s < parts; s++) M = fmax_nan(M, __ldcg(partLse + s * rows + row));
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float wsum = 0.f;
 #pragma unroll 4
   for (int s = 0; s < parts; s++) {
-    const float4 v = *reinterpret_cast<const float4*>(partO + (s * rows + row) * D + c4 * 4);
-    const float w = exp2f(partLse[s * rows + row] - M);  // part 0 holds key 0, which every row sees: M is not -inf
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(partO + (s * rows + row) * D + c4 * 4));
+    const float w = exp2f(__ldcg(partLse + s * rows + row) - M);  // part 0 holds key 0, which every row sees: M is not -inf
     acc.x += w * v.x;
     acc.y += w * v.y;
     acc.z += w * v.z;

@@ -829,15 +829,15 @@ __global__ void __launch_bounds__(kMergeThreads) merge_kernel(const Params p) {
   if (parts == 1) return;  // the attention kernel has written the output
   float M = -INFINITY;  // finite after range 0: key 0 is seen by every row
 #pragma unroll 4
-  for (int s = 0; s < parts; s++) M = fmaxf(M, p.partM[s * p.rows + row]);
+  for (int s = 0; s < parts; s++) M = fmaxf(M, __ldcg(p.partM + s * p.rows + row));
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float l = 0.f;
 #pragma unroll 4
   for (int s = 0; s < parts; s++) {
     const long long i = s * p.rows + row;
-    const float4 v = *reinterpret_cast<const float4*>(p.partO + i * kHD + c4 * 4);
-    const float f = tc::ex2((p.partM[i] - M) * p.w.scaleLog2);
-    l = fmaf(p.partL[i], f, l);
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(p.partO + i * kHD + c4 * 4));
+    const float f = tc::ex2((__ldcg(p.partM + i) - M) * p.w.scaleLog2);
+    l = fmaf(__ldcg(p.partL + i), f, l);
     acc.x = fmaf(v.x, f, acc.x);
     acc.y = fmaf(v.y, f, acc.y);
     acc.z = fmaf(v.z, f, acc.z);
