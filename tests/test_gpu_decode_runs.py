@@ -88,3 +88,33 @@ def test_back_to_back_calls_do_not_see_each_others_partials(shape):
     tf.device_status()
     for i, out in enumerate(outs):
         assert torch.equal(out, alone[i % 2]), i
+
+
+@pytest.mark.parametrize("shape,D", [  # batch, seqQ, seqKV, headsQ, headsKV
+    ((1, 1, 9000, 8, 2), 128),  # one entry in many runs
+    ((40, 1, 5000, 32, 8), 64),  # more than two waves of (batch, KV head) pairs, entries across run boundaries
+    ((300, 1, 300, 8, 8), 128),  # whole entries per run
+    ((2, 8, 12289, 32, 8), 128),  # key ranges, combined side by side
+    ((1, 512, 2048, 16, 16), 64),  # key ranges, combined one after the other
+    ((2, 300, 3000, 2, 2), 256),
+])
+def test_rows_without_a_score_above_minus_infinity_are_zero(shape, D):
+    """A mask carried in the head dim (a K column of -inf against a Q column of 1): a masked entry gives exact zeros, a masked
+    half of the keys no weight, however the keys are cut."""
+    B, Sq, Skv, Hq, Hkv = shape
+    Q, K, V = (torch.randn(*s, device="cuda").half() for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
+    Q[..., 0] = 1
+    K[..., 0] = 0
+    K[0, Skv // 2:, :, 0] = float("-inf")
+    want = tf.flash_attn_forward(Q[:1], K[:1, :Skv // 2].contiguous(), V[:1, :Skv // 2].contiguous())
+    masked = K.clone()
+    masked[-1, :, :, 0] = float("-inf")
+    junk = torch.full_like(Q, 7.0)
+    del junk  # the allocator hands this block out again
+    out = tf.flash_attn_forward(Q, masked, V)
+    tf.device_status()
+    assert (out[-1] == 0).all()
+    if B > 1:
+        assert (out[0].float() - want[0].float()).abs().max() <= 2e-3
+    else:
+        assert (tf.flash_attn_forward(Q, K, V).float() - want.float()).abs().max() <= 2e-3

@@ -473,7 +473,10 @@ combine_kernel(const float* partO, const float* partLse, void* O,
   for (int s = threadIdx.x & 31; s < splits; s += 32) M = fmax_nan(M, __ldcg(partLse + (long long)s * rows + row));
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) M = fmax_nan(M, __shfl_xor_sync(0xffffffffu, M, off));
-  if (M == -INFINITY) return;  // no keys at all for this row: leave O untouched
+  if (M == -INFINITY) {  // no key with a score above -inf: all weights and the row are 0, as in the unsplit kernels
+    if (cuQ != nullptr) return;  // packed input: no keys at all for this row, leave O untouched
+    M = 0.f;
+  }
   const int g = threadIdx.x / kVec, c4 = threadIdx.x % kVec;
   if (g < kGroups) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -482,7 +485,7 @@ combine_kernel(const float* partO, const float* partLse, void* O,
     for (int s = g; s < splits; s += kGroups) {
       const float lse = __ldcg(partLse + (long long)s * rows + row);
       const float4 v = __ldcg(reinterpret_cast<const float4*>(partO + ((long long)s * rows + row) * D + c4 * 4));
-      const float w = exp2f(lse - M);  // 0 for a split without keys, whose partial is zero
+      const float w = exp2f(lse - M);  // 0 for a split without a score above -inf, whose partial is zero
       acc.x += w * v.x;
       acc.y += w * v.y;
       acc.z += w * v.z;
@@ -505,7 +508,7 @@ combine_kernel(const float* partO, const float* partLse, void* O,
       acc.w += v.w;
       wsum += sSum[i];
     }
-    const float inv = 1.f / wsum;
+    const float inv = (wsum == 0.f) ? 0.f : (1.f / wsum);  // NaN stays NaN
     uint2 out;
     out.x = pack2<kBf16>(acc.x * inv, acc.y * inv);
     out.y = pack2<kBf16>(acc.z * inv, acc.w * inv);
@@ -535,19 +538,20 @@ combine_parts_kernel(const float* partO, const float* partLse, void* O, long lon
   float M = -INFINITY;
 #pragma unroll 8
   for (int s = 0; s < parts; s++) M = fmax_nan(M, __ldcg(partLse + s * rows + row));
+  if (M == -INFINITY) M = 0.f;  // no score above -inf: all weights and the row are 0, as in the unsplit kernel
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float wsum = 0.f;
 #pragma unroll 4
   for (int s = 0; s < parts; s++) {
     const float4 v = __ldcg(reinterpret_cast<const float4*>(partO + (s * rows + row) * D + c4 * 4));
-    const float w = exp2f(__ldcg(partLse + s * rows + row) - M);  // part 0 holds key 0, which every row sees: M is not -inf
+    const float w = exp2f(__ldcg(partLse + s * rows + row) - M);
     acc.x += w * v.x;
     acc.y += w * v.y;
     acc.z += w * v.z;
     acc.w += w * v.w;
     wsum += w;
   }
-  const float inv = 1.f / wsum;
+  const float inv = (wsum == 0.f) ? 0.f : (1.f / wsum);  // NaN stays NaN
   uint2 out;
   out.x = pack2<kBf16>(acc.x * inv, acc.y * inv);
   out.y = pack2<kBf16>(acc.z * inv, acc.w * inv);

@@ -827,9 +827,10 @@ __global__ void __launch_bounds__(kMergeThreads) merge_kernel(const Params p) {
   }
   const int parts = (blocks + p.partBlocks - 1) / p.partBlocks;
   if (parts == 1) return;  // the attention kernel has written the output
-  float M = -INFINITY;  // finite after range 0: key 0 is seen by every row
+  float M = -INFINITY;
 #pragma unroll 4
   for (int s = 0; s < parts; s++) M = fmaxf(M, __ldcg(p.partM + s * p.rows + row));
+  if (M == -INFINITY) M = 0.f;  // no score above -inf: all weights and the row are 0
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float l = 0.f;
 #pragma unroll 4
