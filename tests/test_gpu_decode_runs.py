@@ -118,3 +118,28 @@ def test_rows_without_a_score_above_minus_infinity_are_zero(shape, D):
         assert (out[0].float() - want[0].float()).abs().max() <= 2e-3
     else:
         assert (tf.flash_attn_forward(Q, K, V).float() - want.float()).abs().max() <= 2e-3
+
+
+@pytest.mark.parametrize("Hq,Hkv,most", [(16, 2, 1), (4, 4, 2), (4, 1, 3)])
+def test_packed_rows_without_partials_stay_zero(Hq, Hkv, most):
+    """Packed decode with key splits: rows before the first sequence, past the last one, of a sequence without keys and past a
+    tile's sixteen are zero whatever the scratch held, and so are rows without a score above -inf; all others are those of a
+    call on their sequence alone."""
+    D, group = 64, Hq // Hkv
+    cu_q = torch.tensor([3, 3 + most, 23 + most, 24 + most, 25 + most, 26 + most], dtype=torch.int32, device="cuda")
+    cu_kv = torch.tensor([0, 3000, 5500, 5500, 7500, 9500], dtype=torch.int32, device="cuda")
+    Q, K, V = (torch.randn(*s, device="cuda").half() for s in ((30, Hq, D), (9500, Hkv, D), (9500, Hkv, D)))
+    Q[..., 0] = 1
+    K[..., 0] = 0
+    K[5500:7500, :, 0] = float("-inf")
+    want = torch.zeros(Q.shape, device="cuda")
+    rows = max(most, 16 // group)  # positions of the second, longer sequence that its tile holds
+    for a, n, c, d in ((3, most, 0, 3000), (3 + most, rows, 3000, 5500), (25 + most, 1, 7500, 9500)):
+        want[a:a + n] = tf.flash_attn_forward(Q[None, a:a + n], K[None, c:d], V[None, c:d])[0].float()
+    for _ in range(3):
+        tf.flash_attn_forward(*(torch.full(s, 50.0, device="cuda").half() for s in ((4, 1, 16, D), (4, 9000, 2, D), (4, 9000, 2, D))))
+        junk = torch.full_like(Q, 7.0)
+        del junk  # the allocator hands this block out again
+        out = tf.flash_attn_varlen_forward(Q, K, V, cu_q, cu_kv, most, 3000).float()
+        assert (out - want).abs().max() <= 2e-3
+        assert (out[want.abs().amax(dim=(1, 2)) == 0] == 0).all()

@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
       kvRow0 = (long long)b * skv;
     }
     if (sq <= 0) return;
-    if (skv <= 0 && p.splits == 1) return;  // nothing to write; with splits > 1 the partials must still be defined
+    if (skv <= 0) return;  // nothing to write
     keyEnd = p.causal ? min(skv, sq) : skv;
     // keysPerSplit comes from the caller's maximum key length, which only sizes the launch: the last split runs to
     // the real end of the sequence, so an understated maximum loses no keys (the reference derives its key loop from
@@ -450,69 +450,76 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
 // D / 4 threads read one split's partial row and 128 / (D / 4) such groups take turns over the splits, four in flight each.
 // The kernel is launched while the split kernel still runs (launch_kernel in tfa_common.cuh): the partials change during
 // its lifetime, so they are read with coherent loads and their pointers promise the compiler nothing.
+// Packed input: the grid is that of the split kernel with the rows of a tile in place of the splits, so that exactly the rows
+// that have partials are stored - none before cu_seqlens_q[0], past the last sequence or past a tile's sixteen.
 constexpr int kCombineThreads = 128;
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kCombineThreads)
-combine_kernel(const float* partO, const float* partLse, void* O,
-               long long rows /* totalQ * Hq */, int splits, const int* cuQ, int batch, int headsQ, int runs,
-               int blocksPerEntry, long long totalBlocks, int seqLenQ) {
+combine_kernel(const float* partO, const float* partLse, void* O, long long rows /* totalQ * Hq */, int splits, const int* cuQ,
+               const int* cuKV, int headsQ, int group, int runs, int blocksPerEntry, long long totalBlocks, int seqLenQ) {
   constexpr int kVec = D / 4, kGroups = kCombineThreads / kVec;
   __shared__ float4 sAcc[kGroups][kVec];
   __shared__ float sSum[kGroups];
   ptx::grid_wait_previous();
   ptx::grid_allow_next();
-  const long long row = blockIdx.x;
-  // packed input: rows past the last sequence (a Q tensor longer than cu_seqlens_q[batch]) have no partials
-  if (cuQ != nullptr && row / headsQ >= cuQ[batch]) return;
-  if (runs > 0) {  // even partition: how many runs touch this row's batch entry
+  int r = 0, nRows = 1;  // rows of this CTA: r, r + gridDim.x, ... (packed input), one (fixed length)
+  long long row = blockIdx.x, qRow0 = 0;
+  if (cuQ != nullptr) {
+    const int b = blockIdx.z;
+    if (cuKV[b + 1] <= cuKV[b]) return;  // no keys: leave O untouched
+    qRow0 = cuQ[b];
+    r = blockIdx.x;
+    nRows = min((cuQ[b + 1] - cuQ[b]) * group, kRows);  // as in the split kernel
+  } else if (runs > 0) {  // even partition: how many runs touch this row's batch entry
     const long long first = row / headsQ / seqLenQ * blocksPerEntry;
     splits = run_of_block(first + blocksPerEntry - 1, totalBlocks, runs) - run_of_block(first, totalBlocks, runs) + 1;
     if (splits == 1) return;  // the split kernel has written the output
   }
-  float M = -INFINITY;
-  for (int s = threadIdx.x & 31; s < splits; s += 32) M = fmax_nan(M, __ldcg(partLse + (long long)s * rows + row));
+  for (; r < nRows; r += gridDim.x) {
+    if (cuQ != nullptr) row = (qRow0 + r / group) * headsQ + blockIdx.y * group + r % group;
+    float M = -INFINITY;
+    for (int s = threadIdx.x & 31; s < splits; s += 32) M = fmax_nan(M, __ldcg(partLse + (long long)s * rows + row));
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) M = fmax_nan(M, __shfl_xor_sync(0xffffffffu, M, off));
-  if (M == -INFINITY) {  // no key with a score above -inf: all weights and the row are 0, as in the unsplit kernels
-    if (cuQ != nullptr) return;  // packed input: no keys at all for this row, leave O untouched
-    M = 0.f;
-  }
-  const int g = threadIdx.x / kVec, c4 = threadIdx.x % kVec;
-  if (g < kGroups) {
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float wsum = 0.f;
+    for (int off = 16; off > 0; off >>= 1) M = fmax_nan(M, __shfl_xor_sync(0xffffffffu, M, off));
+    if (M == -INFINITY) M = 0.f;  // no key with a score above -inf: all weights and the row are 0, as in the unsplit kernels
+    const int g = threadIdx.x / kVec, c4 = threadIdx.x % kVec;
+    if (g < kGroups) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      float wsum = 0.f;
 #pragma unroll 4
-    for (int s = g; s < splits; s += kGroups) {
-      const float lse = __ldcg(partLse + (long long)s * rows + row);
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(partO + ((long long)s * rows + row) * D + c4 * 4));
-      const float w = exp2f(lse - M);  // 0 for a split without a score above -inf, whose partial is zero
-      acc.x += w * v.x;
-      acc.y += w * v.y;
-      acc.z += w * v.z;
-      acc.w += w * v.w;
-      wsum += w;
+      for (int s = g; s < splits; s += kGroups) {
+        const float lse = __ldcg(partLse + (long long)s * rows + row);
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(partO + ((long long)s * rows + row) * D + c4 * 4));
+        const float w = exp2f(lse - M);  // 0 for a split without a score above -inf, whose partial is zero
+        acc.x += w * v.x;
+        acc.y += w * v.y;
+        acc.z += w * v.z;
+        acc.w += w * v.w;
+        wsum += w;
+      }
+      sAcc[g][c4] = acc;
+      if (c4 == 0) sSum[g] = wsum;
     }
-    sAcc[g][c4] = acc;
-    if (c4 == 0) sSum[g] = wsum;
-  }
-  __syncthreads();
-  if (threadIdx.x < kVec) {
-    float4 acc = sAcc[0][threadIdx.x];
-    float wsum = sSum[0];
+    __syncthreads();
+    if (threadIdx.x < kVec) {
+      float4 acc = sAcc[0][threadIdx.x];
+      float wsum = sSum[0];
 #pragma unroll
-    for (int i = 1; i < kGroups; i++) {
-      const float4 v = sAcc[i][threadIdx.x];
-      acc.x += v.x;
-      acc.y += v.y;
-      acc.z += v.z;
-      acc.w += v.w;
-      wsum += sSum[i];
+      for (int i = 1; i < kGroups; i++) {
+        const float4 v = sAcc[i][threadIdx.x];
+        acc.x += v.x;
+        acc.y += v.y;
+        acc.z += v.z;
+        acc.w += v.w;
+        wsum += sSum[i];
+      }
+      const float inv = (wsum == 0.f) ? 0.f : (1.f / wsum);  // NaN stays NaN
+      uint2 out;
+      out.x = pack2<kBf16>(acc.x * inv, acc.y * inv);
+      out.y = pack2<kBf16>(acc.z * inv, acc.w * inv);
+      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(O) + row * D + threadIdx.x * 4) = out;
     }
-    const float inv = (wsum == 0.f) ? 0.f : (1.f / wsum);  // NaN stays NaN
-    uint2 out;
-    out.x = pack2<kBf16>(acc.x * inv, acc.y * inv);
-    out.y = pack2<kBf16>(acc.z * inv, acc.w * inv);
-    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(O) + row * D + threadIdx.x * 4) = out;
+    if (r + (int)gridDim.x < nRows) __syncthreads();  // sAcc is written again
   }
 }
 
@@ -568,7 +575,7 @@ int launch_combine(const FwdProblem& p, int packShift, const TcSplit& split) {
     // all ranges).  us a call, the kernel below -> this one: 60 rows of four heads x 20000 keys D64 19.2 -> 14.1, 34 x 7508 16 heads
     // 25.5 -> 23.3, 1400 x 8000 2 heads 30.2 -> 28.0, 2 x 8 x 12289 32 heads 31.5 -> 31.1.
     e = launch_kernel(combine_kernel<D, kBf16>, dim3((unsigned)rows), kCombineThreads, 0, p.stream, p.overlap, split.partO,
-                      split.partLse, p.O, rows, split.parts, nullptr, p.batch, p.headsQ, 0, 0, 0ll, p.seqLenQ);
+                      split.partLse, p.O, rows, split.parts, nullptr, nullptr, p.headsQ, 1, 0, 0, 0ll, p.seqLenQ);
   } else {
     e = launch_kernel(combine_parts_kernel<D, kBf16>, dim3((unsigned)((rows + kGroups - 1) / kGroups)), kCombineThreads, 0, p.stream,
                       p.overlap, split.partO, split.partLse, p.O, rows, split.partBlocks, p.seqLenQ, p.seqLenKV, p.headsQ, p.causal,
@@ -631,8 +638,10 @@ int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* par
   cudaError_t e = launch_kernel(kernel, grid, kThreads, kSmem, pr.stream, pr.overlap, p);
   if (e == cudaSuccess && plan.splits > 1) {
     const long long rows = pr.totalQ * pr.headsQ;
-    e = launch_kernel(combine_kernel<D, kBf16>, dim3((unsigned)rows), kCombineThreads, 0, pr.stream, pr.overlap, partO, partLse,
-                      pr.O, rows, plan.splits, pr.cuQ, pr.batch, pr.headsQ, p.runs, p.blocksPerEntry, p.totalBlocks, pr.seqLenQ);
+    const int tileRows = pr.seqLenQ * p.group;  // a longer sequence than the caller's maximum: the CTAs take turns
+    const dim3 combineGrid = pr.cuQ != nullptr ? dim3((unsigned)tileRows, (unsigned)pr.headsKV, (unsigned)pr.batch) : dim3((unsigned)rows);
+    e = launch_kernel(combine_kernel<D, kBf16>, combineGrid, kCombineThreads, 0, pr.stream, pr.overlap, partO, partLse, pr.O, rows,
+                      plan.splits, pr.cuQ, pr.cuKV, pr.headsQ, p.group, p.runs, p.blocksPerEntry, p.totalBlocks, pr.seqLenQ);
   }
   if (e != cudaSuccess) {
     set_error_string("split-KV kernel launch failed: %s", cudaGetErrorString(e));
