@@ -105,3 +105,33 @@ def test_captured_calls_replay():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("shape,D,lens", [  # batch, seqQ, seqKV, headsQ, headsKV
+    ((9, 900, 900, 32, 32), 256, None),  # pieces of batch entries, the last one smaller
+    ((1, 40, 90000, 16, 8), 128, None),  # one entry: pieces of KV heads
+    ((3, 0, 0, 48, 12), 192, [9000, 7000, 6000]),  # packed: pieces of KV heads
+])
+def test_calls_in_pieces(shape, D, lens):
+    """Calls whose parts take more than the 1 GiB of workspace that is kept.  Bound: the CUDA-core kernel adds its keys one by
+    one, a walk of as many roundings of 2^-24 as there are keys; the other one's error is a few such roundings."""
+    B, Sq, Skv, Hq, Hkv = shape
+    g = torch.Generator(device="cuda").manual_seed(D)
+
+    def normal(*s):
+        return torch.randn(*s, device="cuda", generator=g)
+
+    if lens is None:
+        Q, K, V = normal(B, Sq, Hq, D), normal(B, Skv, Hkv, D), normal(B, Skv, Hkv, D)
+        call = lambda: tf.flash_attn_forward(Q, K, V)
+    else:
+        Q, K, V = normal(sum(lens), Hq, D), normal(sum(lens), Hkv, D), normal(sum(lens), Hkv, D)
+        cu = torch.tensor([0] + lens).cumsum(0).int().cuda()
+        call = lambda: tf.flash_attn_varlen_forward(Q, K, V, cu, cu, max(lens), max(lens), is_causal=True)
+    assert 6 * (Q.numel() + 2 * K.numel()) > 1 << 30
+    got, old = _with(1, call), _with(0, call)
+    assert (got - old).abs().max() <= 1e-5
+    assert (got - old).norm() <= 2.0**-24 * (max(lens or [Skv]) ** 0.5 + 8) * old.norm()
+    V[(-1,) + (0,) * (V.dim() - 1)] = float("nan")  # seen by the last piece only: the whole call is the CUDA cores'
+    got, old = _with(1, call), _with(0, call)
+    assert torch.equal(got.view(torch.int32), old.view(torch.int32))

@@ -60,8 +60,8 @@ int launch_combine_parts(const FwdProblem& p, int packShift, const TcSplit& spli
 
 // ---- fp32 on the tensor cores (fwd_fp32_tc.cu)
 bool fp32tc_applicable(const FwdProblem& p, int option);
-size_t fp32tc_workspace_bytes(const FwdProblem& p, int packShift, int numSMs);
-int launch_fwd_fp32tc(const FwdProblem& p, int packShift, void* ws, int epoch);
+size_t fp32tc_workspace_bytes(const FwdProblem& p, const Fp32Piece& piece, int packShift, int numSMs);
+int launch_fwd_fp32tc(const FwdProblem& p, const Fp32Piece& piece, int packShift, void* ws, int epoch);
 
 static thread_local char g_err[512] = "";
 
@@ -397,13 +397,33 @@ static int dispatch_fp32(const FwdProblem& p) {
   cudaMemPool_t pool = scratch_pool(device);
   void* ws = nullptr;
   const int ps = pick_pack_shift(p);
-  if (pool == nullptr || cudaMallocFromPoolAsync(&ws, fp32tc_workspace_bytes(p, ps, device_num_sms(device)), pool, p.stream) != cudaSuccess) {
+  // A workspace beyond what the pool keeps would be taken from the driver and given back around every synchronisation, at
+  // about 11 ms per GB: 512 x 512 tokens, 16 heads of 64 10.3 ms a call, 49.9 when the caller waits for each (CUDA cores 13.0; in pieces 5.6 either way).  So
+  // a larger call runs in pieces, one after the other in the same workspace: fewer batch entries, then fewer heads.
+  Fp32Piece piece = {0, p.batch, 0, p.headsKV};
+  auto bytes = [&] { return fp32tc_workspace_bytes(p, piece, ps, device_num_sms(device)); };
+  while (bytes() > kPoolKeepBytes && p.cuQ == nullptr && piece.batches > 1) piece.batches = (piece.batches + 1) / 2;
+  while (bytes() > kPoolKeepBytes && piece.heads > 1) piece.heads = (piece.heads + 1) / 2;
+  const Fp32Piece first = piece;
+  size_t need = bytes();
+  if (p.batch % first.batches != 0) {  // the last piece has fewer tiles and maybe key ranges with partial results
+    piece.batches = p.batch % first.batches;
+    if (bytes() > need) need = bytes();
+  }
+  if (pool == nullptr || cudaMallocFromPoolAsync(&ws, need, pool, p.stream) != cudaSuccess) {
     (void)cudaGetLastError();
     return launch_fwd_fp32(p);
   }
   const int epoch = next_epoch();
-  int rc = launch_fwd_fp32tc(p, ps, ws, epoch);
-  if (rc == kOk) {
+  int rc = kOk;
+  for (piece.batch0 = 0; rc == kOk && piece.batch0 < p.batch; piece.batch0 += first.batches) {
+    piece.batches = p.batch - piece.batch0 < first.batches ? p.batch - piece.batch0 : first.batches;
+    for (piece.head0 = 0; rc == kOk && piece.head0 < p.headsKV; piece.head0 += first.heads) {
+      piece.heads = p.headsKV - piece.head0 < first.heads ? p.headsKV - piece.head0 : first.heads;
+      rc = launch_fwd_fp32tc(p, piece, ps, ws, epoch);
+    }
+  }
+  if (rc == kOk) {  // one flag for all pieces: the CUDA-core kernel computes the whole call or none of it
     FwdProblem rest = p;
     rest.gate = static_cast<const int*>(ws);
     rest.gateEpoch = epoch;

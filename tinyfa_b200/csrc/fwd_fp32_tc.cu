@@ -66,6 +66,8 @@ struct SplitParams {
   const float* src[3];  // Q, K, V
   uint16_t* dst[3];     // three parts each, count[i] elements apart
   long long count[3];   // elements, multiples of 8
+  int width[3];         // elements of a row that are taken ...
+  int pitch[3];         // ... and of a row in memory
   int* flag;            // set to epoch when a value is outside the exact range
   int epoch;
 };
@@ -91,12 +93,14 @@ __global__ void __launch_bounds__(kSplitThreads) split_kernel(const SplitParams 
 #pragma unroll
   for (int t = 0; t < 3; t++) {
     const long long n8 = p.count[t] >> 3;
+    const int w8 = p.width[t] >> 3, gap8 = (p.pitch[t] - p.width[t]) >> 3;
     const float4* src = reinterpret_cast<const float4*>(p.src[t]);
     uint4* d0 = reinterpret_cast<uint4*>(p.dst[t]);
     uint4* d1 = reinterpret_cast<uint4*>(p.dst[t] + p.count[t]);
     uint4* d2 = reinterpret_cast<uint4*>(p.dst[t] + 2 * p.count[t]);
     for (long long i = (long long)blockIdx.x * kSplitThreads + threadIdx.x; i < n8; i += (long long)gridDim.x * kSplitThreads) {
-      const float4 u = src[2 * i], v = src[2 * i + 1];
+      const long long at = gap8 == 0 ? i : i + i / w8 * gap8;
+      const float4 u = src[2 * at], v = src[2 * at + 1];
       uint4 a, b, c;
       split3(u.x, u.y, a.x, b.x, c.x);
       split3(u.z, u.w, a.y, b.y, c.y);
@@ -875,11 +879,11 @@ static int make_map(CUtensorMap* m, const void* base, long long batches, long lo
 struct Ranges {
   int parts = 1, blocks = 0x7FFFFFFF;  // ranges, key blocks of each
 };
-static Ranges plan_ranges(const FwdProblem& pr, int packShift, int numSMs) {
+static Ranges plan_ranges(const FwdProblem& pr, const Fp32Piece& piece, int packShift, int numSMs) {
   Ranges r;
-  if (pr.cuQ != nullptr) return r;
+  if (pr.cuQ != nullptr || piece.heads != pr.headsKV) return r;
   const int rows = kBlockM >> packShift;
-  const long long tiles = (long long)((pr.seqLenQ + rows - 1) / rows) * (pr.headsQ >> packShift) * pr.batch;
+  const long long tiles = (long long)((pr.seqLenQ + rows - 1) / rows) * (pr.headsQ >> packShift) * piece.batches;
   const int seen = pr.causal && pr.seqLenQ < pr.seqLenKV ? pr.seqLenQ : pr.seqLenKV;
   const int n = (seen + kBlockN - 1) / kBlockN;
   long long parts = numSMs / tiles;
@@ -895,15 +899,20 @@ static Ranges plan_ranges(const FwdProblem& pr, int packShift, int numSMs) {
 struct Layout {
   size_t q, k, v, part, partRows, bytes;  // byte offsets of the parts behind the flag, and of the partial results
 };
-static Layout layout(const FwdProblem& pr, const Ranges& ranges) {
+// Rows of Q and of K / V that a piece covers (packed input: all of them).
+static long long rows_q(const FwdProblem& pr, const Fp32Piece& piece) { return pr.cuQ != nullptr ? pr.totalQ : (long long)piece.batches * pr.seqLenQ; }
+static long long rows_kv(const FwdProblem& pr, const Fp32Piece& piece) { return pr.cuQ != nullptr ? pr.totalKV : (long long)piece.batches * pr.seqLenKV; }
+
+static Layout layout(const FwdProblem& pr, const Fp32Piece& piece, const Ranges& ranges) {
   auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
-  const size_t q = (size_t)pr.totalQ * pr.headsQ * pr.headDim * 6, kv = (size_t)pr.totalKV * pr.headsKV * pr.headDim * 6;
+  const size_t rowsQ = (size_t)rows_q(pr, piece), headsQ = (size_t)piece.heads * (pr.headsQ / pr.headsKV);
+  const size_t q = rowsQ * headsQ * pr.headDim * 6, kv = (size_t)rows_kv(pr, piece) * piece.heads * pr.headDim * 6;
   Layout l;
   l.q = 1024;
   l.k = l.q + up(q);
   l.v = l.k + up(kv);
   l.part = l.v + up(kv);
-  l.partRows = ranges.parts > 1 ? (size_t)ranges.parts * pr.totalQ * pr.headsQ : 0;
+  l.partRows = ranges.parts > 1 ? ranges.parts * rowsQ * headsQ : 0;
   l.bytes = l.part + l.partRows * (pr.headDim + 2) * sizeof(float);
   return l;
 }
@@ -919,7 +928,7 @@ constexpr auto kernel_of() {
 }
 
 template <int kHD>
-int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
+int launch(const FwdProblem& pr, const Fp32Piece& piece, int packShift, uint8_t* ws, int epoch) {
   constexpr int kSmem = kHD > 128 ? CfgWide<(kHD > 128 ? kHD : 256)>::kSmemBytes : Cfg<(kHD <= 64 ? 64 : 128)>::kSmemBytes;
   constexpr int threads = kHD > 128 ? kThreadsWide : kThreads;
   const bool varlen = (pr.cuQ != nullptr);
@@ -938,19 +947,22 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
     set_error_string("cudaFuncSetAttribute(%d bytes): %s", kSmem, cudaGetErrorString(attrErr[device]));
     return kCudaError;
   }
-  const Ranges ranges = plan_ranges(pr, packShift, device_num_sms(device));
-  const Layout lay = layout(pr, ranges);
-  const int gp = 1 << packShift, rowsPerTile = kBlockM >> packShift;
-  const long long nb = varlen ? 1 : pr.batch;
+  const Ranges ranges = plan_ranges(pr, piece, packShift, device_num_sms(device));
+  const Layout lay = layout(pr, piece, ranges);
+  const int gp = 1 << packShift, rowsPerTile = kBlockM >> packShift, group = pr.headsQ / pr.headsKV, headsQ = piece.heads * group;
+  const long long nb = varlen ? 1 : piece.batches;
   const long long rowsQ = varlen ? pr.totalQ : pr.seqLenQ, rowsKV = varlen ? pr.totalKV : pr.seqLenKV;
+  // elements of Q (and O) and of K / V ahead of the piece
+  const long long skipQ = ((long long)piece.batch0 * pr.seqLenQ * pr.headsQ + piece.head0 * group) * pr.headDim;
+  const long long skipKV = ((long long)piece.batch0 * pr.seqLenKV * pr.headsKV + piece.head0) * pr.headDim;
   CUtensorMap tmQ, tmK, tmV;
   int rc;
-  if ((rc = make_map(&tmQ, ws + lay.q, nb, rowsQ, pr.headsQ, pr.headDim, gp, rowsPerTile)) != kOk) return rc;
-  if ((rc = make_map(&tmK, ws + lay.k, nb, rowsKV, pr.headsKV, pr.headDim, 1, kBlockN)) != kOk) return rc;
-  if ((rc = make_map(&tmV, ws + lay.v, nb, rowsKV, pr.headsKV, pr.headDim, 1, kBlockN)) != kOk) return rc;
+  if ((rc = make_map(&tmQ, ws + lay.q, nb, rowsQ, headsQ, pr.headDim, gp, rowsPerTile)) != kOk) return rc;
+  if ((rc = make_map(&tmK, ws + lay.k, nb, rowsKV, piece.heads, pr.headDim, 1, kBlockN)) != kOk) return rc;
+  if ((rc = make_map(&tmV, ws + lay.v, nb, rowsKV, piece.heads, pr.headDim, 1, kBlockN)) != kOk) return rc;
 
   Params p = {};
-  p.w.O = pr.O;
+  p.w.O = static_cast<float*>(pr.O) + skipQ;
   p.w.cuQ = pr.cuQ;
   p.w.cuKV = pr.cuKV;
   p.w.seqLenQ = pr.seqLenQ;
@@ -958,16 +970,16 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
   p.w.headsQ = pr.headsQ;
   p.w.headsKV = pr.headsKV;
   p.w.headDim = pr.headDim;
-  p.w.group = pr.headsQ / pr.headsKV;
+  p.w.group = group;
   p.w.packShift = packShift;
   p.w.numPairs = (pr.seqLenQ + rowsPerTile - 1) / rowsPerTile;
-  p.w.numUnits = pr.headsQ / gp;
+  p.w.numUnits = headsQ / gp;
   p.w.causal = pr.causal;
   p.w.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)pr.headDim));
   p.w.epoch = epoch;
   p.w.status = device_status_word(device);
   if (p.w.status == nullptr) return kCudaError;
-  const long long per = (long long)p.w.numUnits * pr.batch, numWork = per * p.w.numPairs;
+  const long long per = (long long)p.w.numUnits * piece.batches, numWork = per * p.w.numPairs;
   if (numWork > 0x7FFFFFFFll) {
     set_error_string("too many work items (%lld)", numWork);
     return kTooLarge;
@@ -982,7 +994,7 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
     p.w.chunk = (int)(width < per ? width : per);
   }
   p.partBlocks = ranges.blocks;
-  p.rows = pr.totalQ * pr.headsQ;
+  p.rows = rows_q(pr, piece) * headsQ;
   p.partO = reinterpret_cast<float*>(ws + lay.part);
   p.partM = p.partO + lay.partRows * kHD;
   p.partL = p.partM + lay.partRows;
@@ -990,14 +1002,18 @@ int launch(const FwdProblem& pr, int packShift, uint8_t* ws, int epoch) {
   p.flag = reinterpret_cast<const int*>(ws);
 
   SplitParams sp;
-  sp.src[0] = static_cast<const float*>(pr.Q);
-  sp.src[1] = static_cast<const float*>(pr.K);
-  sp.src[2] = static_cast<const float*>(pr.V);
+  sp.src[0] = static_cast<const float*>(pr.Q) + skipQ;
+  sp.src[1] = static_cast<const float*>(pr.K) + skipKV;
+  sp.src[2] = static_cast<const float*>(pr.V) + skipKV;
   sp.dst[0] = reinterpret_cast<uint16_t*>(ws + lay.q);
   sp.dst[1] = reinterpret_cast<uint16_t*>(ws + lay.k);
   sp.dst[2] = reinterpret_cast<uint16_t*>(ws + lay.v);
-  sp.count[0] = pr.totalQ * pr.headsQ * pr.headDim;
-  sp.count[1] = sp.count[2] = pr.totalKV * pr.headsKV * pr.headDim;
+  sp.width[0] = headsQ * pr.headDim;
+  sp.pitch[0] = pr.headsQ * pr.headDim;
+  sp.width[1] = sp.width[2] = piece.heads * pr.headDim;
+  sp.pitch[1] = sp.pitch[2] = pr.headsKV * pr.headDim;
+  sp.count[0] = rows_q(pr, piece) * sp.width[0];
+  sp.count[1] = sp.count[2] = rows_kv(pr, piece) * sp.width[1];
   sp.flag = reinterpret_cast<int*>(ws);
   sp.epoch = epoch;
   cudaError_t e = launch_kernel(split_kernel, dim3(8u * (unsigned)device_num_sms(device)), kSplitThreads, 0, pr.stream, pr.overlap, sp);
@@ -1029,44 +1045,45 @@ bool fp32tc_applicable(const FwdProblem& p, int option) {
   return (ctas + 147) / 148 * blocks * p.headDim >= 256;
 }
 
-size_t fp32tc_workspace_bytes(const FwdProblem& p, int packShift, int numSMs) {
-  return fp32tc::layout(p, fp32tc::plan_ranges(p, packShift, numSMs)).bytes;
+size_t fp32tc_workspace_bytes(const FwdProblem& p, const Fp32Piece& piece, int packShift, int numSMs) {
+  return fp32tc::layout(p, piece, fp32tc::plan_ranges(p, piece, packShift, numSMs)).bytes;
 }
 
-// Enqueues the split and the attention kernel.  *ws begins with the word that reads `epoch` when the call is left to the
+// Enqueues the split and the attention kernel of a piece.  *ws begins with the word that reads `epoch` when the call is left to the
 // CUDA-core kernel.
-int launch_fwd_fp32tc(const FwdProblem& p, int packShift, void* ws, int epoch) {
+int launch_fwd_fp32tc(const FwdProblem& p, const Fp32Piece& piece, int packShift, void* ws, int epoch) {
 #if TFA_HAVE_FP32
   uint8_t* w = static_cast<uint8_t*>(ws);
   switch (p.headDim) {
 #if TFA_HAVE_HD32
     case 32:
-      return fp32tc::launch<32>(p, packShift, w, epoch);
+      return fp32tc::launch<32>(p, piece, packShift, w, epoch);
 #endif
 #if TFA_HAVE_HD64
     case 64:
-      return fp32tc::launch<64>(p, packShift, w, epoch);
+      return fp32tc::launch<64>(p, piece, packShift, w, epoch);
 #endif
 #if TFA_HAVE_HD96
     case 96:
-      return fp32tc::launch<96>(p, packShift, w, epoch);
+      return fp32tc::launch<96>(p, piece, packShift, w, epoch);
 #endif
 #if TFA_HAVE_HD128
     case 128:
-      return fp32tc::launch<128>(p, packShift, w, epoch);
+      return fp32tc::launch<128>(p, piece, packShift, w, epoch);
 #endif
 #if TFA_HAVE_HD192
     case 192:
-      return fp32tc::launch<192>(p, packShift, w, epoch);
+      return fp32tc::launch<192>(p, piece, packShift, w, epoch);
 #endif
 #if TFA_HAVE_HD256
     case 256:
-      return fp32tc::launch<256>(p, packShift, w, epoch);
+      return fp32tc::launch<256>(p, piece, packShift, w, epoch);
 #endif
     default:
       break;
   }
 #endif
+  (void)piece;
   (void)packShift;
   (void)ws;
   (void)epoch;

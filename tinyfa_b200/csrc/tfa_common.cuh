@@ -68,6 +68,13 @@ struct TcSplit {
   float* partLse = nullptr;
 };
 
+// A piece of an fp32 call on the tensor cores, which works with one workspace at a time (dispatch_fp32 in c_abi.cu): batch
+// entries [batch0, batch0 + batches) and KV heads [head0, head0 + heads) with their Q heads.  Packed input: all entries.
+struct Fp32Piece {
+  int batch0, batches;
+  int head0, heads;
+};
+
 // The device status word holds 0, or (launch epoch << 8) | site code once a bounded wait inside a kernel gave up.
 
 // Kernels of this library let the next kernel of the stream start early (griddepcontrol.launch_dependents) and, launched
