@@ -135,3 +135,22 @@ def test_calls_in_pieces(shape, D, lens):
     V[(-1,) + (0,) * (V.dim() - 1)] = float("nan")  # seen by the last piece only: the whole call is the CUDA cores'
     got, old = _with(1, call), _with(0, call)
     assert torch.equal(got.view(torch.int32), old.view(torch.int32))
+
+
+@pytest.mark.parametrize("shape,D,causal,cores", [  # the faster path by a factor of 1.3 at least
+    ((512, 64, 64, 8, 8), 64, False, True),
+    ((200, 49, 49, 12, 12), 32, False, True),
+    ((2, 100, 3000, 8, 8), 128, True, True),
+    ((4, 4096, 16, 8, 8), 64, False, True),
+    ((64, 1, 300, 32, 32), 64, False, True),
+    ((64, 256, 256, 8, 8), 64, False, False),
+    ((1, 1000, 1000, 1, 1), 64, False, False),
+    ((8, 1, 4096, 32, 8), 128, False, False),
+    ((128, 77, 77, 12, 12), 128, False, False),
+])
+def test_path_by_size(shape, D, causal, cores):
+    """Short sequences, few keys and few queries ahead of many masked keys stay on the CUDA cores in batches of any size."""
+    B, Sq, Skv, Hq, Hkv = shape
+    Q, K, V = (torch.randn(*s, device="cuda") for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
+    call = lambda: tf.flash_attn_forward(Q, K, V, is_causal=causal)
+    assert torch.equal(_with(-1, call), _with(0 if cores else 1, call))

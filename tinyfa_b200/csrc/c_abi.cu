@@ -59,7 +59,7 @@ int launch_fwd_splitkv(const FwdProblem& p, const SplitPlan& plan, float* scratc
 int launch_combine_parts(const FwdProblem& p, int packShift, const TcSplit& split);
 
 // ---- fp32 on the tensor cores (fwd_fp32_tc.cu)
-bool fp32tc_applicable(const FwdProblem& p, int option);
+bool fp32tc_applicable(const FwdProblem& p, int packShift, int numSMs, int option);
 size_t fp32tc_workspace_bytes(const FwdProblem& p, const Fp32Piece& piece, int packShift, int numSMs);
 int launch_fwd_fp32tc(const FwdProblem& p, const Fp32Piece& piece, int packShift, void* ws, int epoch);
 
@@ -391,15 +391,16 @@ static int dispatch_splitkv(const FwdProblem& p, const SplitPlan& plan) {
 static int dispatch_fp32(const FwdProblem& p) {
   const int opt = g_optFp32Tc.load();
   // an explicit choice of the CUDA-core form (option "fp32_t8") is kept
-  if (opt == 0 || (opt < 0 && g_optFp32T8.load() != 1) || !fp32tc_applicable(p, opt)) return launch_fwd_fp32(p);
+  if (opt == 0 || (opt < 0 && g_optFp32T8.load() != 1)) return launch_fwd_fp32(p);
   int device = 0;
   if (!p.overlap || cudaGetDevice(&device) != cudaSuccess) return launch_fwd_fp32(p);  // under capture
+  const int ps = pick_pack_shift(p);
+  if (!fp32tc_applicable(p, ps, device_num_sms(device), opt)) return launch_fwd_fp32(p);
   cudaMemPool_t pool = scratch_pool(device);
   void* ws = nullptr;
-  const int ps = pick_pack_shift(p);
   // A workspace beyond what the pool keeps would be taken from the driver and given back around every synchronisation, at
-  // about 11 ms per GB: 512 x 512 tokens, 16 heads of 64 10.3 ms a call, 49.9 when the caller waits for each (CUDA cores 13.0; in pieces 5.6 either way).  So
-  // a larger call runs in pieces, one after the other in the same workspace: fewer batch entries, then fewer heads.
+  // about 11 ms per GB.  So a larger call runs in pieces, one after the other in the same workspace: fewer batch entries, then
+  // fewer heads.  512 x 512 tokens, 16 heads of 64, caller waiting for each call: 49.9 ms whole, 5.6 in pieces (CUDA cores 13.0).
   Fp32Piece piece = {0, p.batch, 0, p.headsKV};
   auto bytes = [&] { return fp32tc_workspace_bytes(p, piece, ps, device_num_sms(device)); };
   while (bytes() > kPoolKeepBytes && p.cuQ == nullptr && piece.batches > 1) piece.batches = (piece.batches + 1) / 2;

@@ -1031,18 +1031,46 @@ int launch(const FwdProblem& pr, const Fp32Piece& piece, int packShift, uint8_t*
 
 }  // namespace fp32tc
 
-// A known number of rows.  By size: the CUDA-core kernel takes about D / 20 us per 64-key block
-// and wave of 64-row CTAs, this path about 14 us at least (three or four launches and an allocation).  Measured on both
-// sides of the line, us per call (CUDA cores, tensor cores): D = 128 S64 B8 8 heads 10.9, 16.7; S128 4 heads 18.6, 15.4; D = 96
-// S128 15.2, 16.2; S256 27.7, 19.0; D = 64 S128 11.7, 13.6; S256 21.2, 15.7; D = 32 S256 13.7, 14.9; S512 25.4, 20.8; D = 192
-// S128 28.8, 23.6; D = 256 S60 8 heads 22.5, 21.2.
-bool fp32tc_applicable(const FwdProblem& p, int option) {
+// Mean number of `block`-key blocks that a query row reads.
+static double mean_blocks(double sq, double skv, bool causal, int block) {
+  const double n = ceil((causal ? fmin(sq, skv) : skv) / block);
+  if (!causal) return n;
+  return sq <= skv ? (n + 1.0) * 0.5 : n - (n - 1.0) * 0.5 * skv / sq;
+}
+
+// A known number of rows, and by size: where a model of both paths' times says so.  In us, at 148 SMs: the CUDA cores take 0.13 +
+// 0.062 D per 64 x 64 block and SM (head dim 128 from three CTAs per SM on: 128 x 128 tiles); here a float costs 2e-6 for the
+// split pass, a tile 4.2 + 0.0137 D and a 128 x 128 block 1.34 + 0.027 D, on one CTA per SM.  So short sequences, few
+// keys and masked keys behind few queries stay on the CUDA cores whatever the batch is.  Fitted to 420 drawn calls of all head dims, 1 to 400
+// sequences of 1 to 1500 rows, a quarter of them packed: the pick is within 0.3 % of the faster path on average, 25 % at worst.  us per
+// call (CUDA cores, tensor cores): B512 S64 8 heads of 64 125, 348; B512 S49 12 heads of 32 111, 405; 2 x 100 x 3000 causal 8 heads of
+// 128 18.6, 32.8; B4 4096 x 16 8 heads of 64 61, 88; on the other side B64 S256 8 heads of 64 213, 137; B4 4096 x 77 113, 89.
+// Below the first line the launches decide: S128 4 heads of 64 11.7, 13.6; S128 4 heads of 128 18.6, 15.4; S256 4 heads of 64 21.2, 15.7.
+bool fp32tc_applicable(const FwdProblem& p, int packShift, int numSMs, int option) {
   if (!TFA_HAVE_FP32 || p.dtype != kFp32 || p.totalQ < 0 || p.totalKV < 0) return false;
+  const bool packed = p.cuQ != nullptr;
+  const int rows = fp32tc::kBlockM >> packShift;
+  if ((long long)((p.seqLenQ + rows - 1) / rows) * (p.headsQ >> packShift) * p.batch > 0x7FFFFFFFll) return false;  // grid
   if (option > 0) return true;
-  const int seen = p.causal ? (p.seqLenQ < p.seqLenKV ? p.seqLenQ : p.seqLenKV) : p.seqLenKV;
-  const long long blocks = (seen + 63) / 64;
-  const long long ctas = (long long)((p.seqLenQ + 63) / 64) * p.headsQ * p.batch;
-  return (ctas + 147) / 148 * blocks * p.headDim >= 256;
+  const int seenMax = p.causal ? (p.seqLenQ < p.seqLenKV ? p.seqLenQ : p.seqLenKV) : p.seqLenKV;
+  const long long ctasMax = (long long)((p.seqLenQ + 63) / 64) * p.headsQ * p.batch;
+  if ((ctasMax + numSMs - 1) / numSMs * ((seenMax + 63) / 64) * p.headDim < 256) return false;
+  // packed input: as if all sequences had the mean length
+  const double sq = packed ? ceil((double)p.totalQ / p.batch) : p.seqLenQ, skv = packed ? ceil((double)p.totalKV / p.batch) : p.seqLenKV;
+  const double seen = p.causal ? fmin(sq, skv) : skv, D = p.headDim, heads = (double)p.headsQ * p.batch;
+  const bool wide = p.headDim == 128 && (double)((p.seqLenQ + 127) / 128) * heads >= 3.0 * numSMs;
+  const double coreWaves = wide ? ceil(2.0 * ceil(sq / 128) * heads / numSMs) : ceil(ceil(sq / 64) * heads / numSMs);
+  const double coreMean = wide ? 2.0 * mean_blocks(sq, skv, p.causal, 128) : mean_blocks(sq, skv, p.causal, 64);
+  const double coreLongest = wide ? 2.0 * ceil(seen / 128) : ceil(seen / 64);
+  const double cores = (0.13 + 0.062 * D) * fmax(coreWaves * coreMean, coreLongest);
+  const fp32tc::Ranges ranges = fp32tc::plan_ranges(p, Fp32Piece{0, p.batch, 0, p.headsKV}, packShift, numSMs);
+  const double tiles = ceil(sq / rows) * (p.headsQ >> packShift) * p.batch, waves = ceil(tiles * ranges.parts / numSMs);
+  const double longest = ranges.parts > 1 ? ranges.blocks : ceil(seen / fp32tc::kBlockN);
+  const double mean = ranges.parts > 1 ? longest : mean_blocks(sq, skv, p.causal, fp32tc::kBlockN);
+  const double floats = (sq * heads + 2.0 * skv * p.headsKV * p.batch) * D;
+  const double here = (ranges.parts > 1 ? 3.0 : 0.0) + 2e-6 * floats + (4.2 + 0.0137 * D) * waves +
+                      (1.34 + 0.027 * D) * fmax(waves * mean, longest);
+  return here < cores;
 }
 
 size_t fp32tc_workspace_bytes(const FwdProblem& p, const Fp32Piece& piece, int packShift, int numSMs) {
