@@ -154,3 +154,20 @@ def test_path_by_size(shape, D, causal, cores):
     Q, K, V = (torch.randn(*s, device="cuda") for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
     call = lambda: tf.flash_attn_forward(Q, K, V, is_causal=causal)
     assert torch.equal(_with(-1, call), _with(0 if cores else 1, call))
+
+
+@pytest.mark.parametrize("D", [64, 256])
+def test_rows_of_no_sequence_do_not_matter(D):
+    """Packed input with rows ahead of the first and behind the last sequence: whatever they hold, the call stays on the tensor
+    cores and gives the same bits, also where a key block reaches into them."""
+    cu_q = torch.tensor([7, 300, 500], dtype=torch.int32, device="cuda")
+    cu_kv = torch.tensor([5, 400, 1000], dtype=torch.int32, device="cuda")
+    Q, K, V = (torch.randn(*s, device="cuda") for s in ((530, 4, D), (1090, 2, D), (1090, 2, D)))
+    call = lambda: tf.flash_attn_varlen_forward(Q, K, V, cu_q, cu_kv, 300, 600)
+    for t, cu in ((Q, cu_q), (K, cu_kv), (V, cu_kv)):
+        t[:cu[0]] = t[cu[-1]:] = 0
+    want, old = _with(1, call), _with(0, call)
+    assert not torch.equal(want, old)
+    for t, cu in ((Q, cu_q), (K, cu_kv), (V, cu_kv)):
+        t[:cu[0]] = t[cu[-1]:] = float("nan")
+    assert torch.equal(_with(1, call), want)

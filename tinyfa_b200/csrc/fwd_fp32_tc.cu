@@ -68,6 +68,8 @@ struct SplitParams {
   long long count[3];   // elements, multiples of 8
   int width[3];         // elements of a row that are taken ...
   int pitch[3];         // ... and of a row in memory
+  const int* cu[3];     // packed input: row ranges of the sequences, else null
+  int batches;
   int* flag;            // set to epoch when a value is outside the exact range
   int epoch;
 };
@@ -98,9 +100,18 @@ __global__ void __launch_bounds__(kSplitThreads) split_kernel(const SplitParams 
     uint4* d0 = reinterpret_cast<uint4*>(p.dst[t]);
     uint4* d1 = reinterpret_cast<uint4*>(p.dst[t] + p.count[t]);
     uint4* d2 = reinterpret_cast<uint4*>(p.dst[t] + 2 * p.count[t]);
+    long long first = 0, end = n8;
+    if (p.cu[t] != nullptr) {  // rows of no sequence: zeros in their place, whatever they hold
+      first = (long long)p.cu[t][0] * w8;
+      end = (long long)p.cu[t][p.batches] * w8;
+    }
     for (long long i = (long long)blockIdx.x * kSplitThreads + threadIdx.x; i < n8; i += (long long)gridDim.x * kSplitThreads) {
       const long long at = gap8 == 0 ? i : i + i / w8 * gap8;
-      const float4 u = src[2 * at], v = src[2 * at + 1];
+      float4 u = make_float4(0.f, 0.f, 0.f, 0.f), v = u;
+      if (i >= first && i < end) {
+        u = src[2 * at];
+        v = src[2 * at + 1];
+      }
       uint4 a, b, c;
       split3(u.x, u.y, a.x, b.x, c.x);
       split3(u.z, u.w, a.y, b.y, c.y);
@@ -1012,6 +1023,9 @@ int launch(const FwdProblem& pr, const Fp32Piece& piece, int packShift, uint8_t*
   sp.pitch[0] = pr.headsQ * pr.headDim;
   sp.width[1] = sp.width[2] = piece.heads * pr.headDim;
   sp.pitch[1] = sp.pitch[2] = pr.headsKV * pr.headDim;
+  sp.cu[0] = pr.cuQ;
+  sp.cu[1] = sp.cu[2] = pr.cuKV;
+  sp.batches = pr.batch;
   sp.count[0] = rows_q(pr, piece) * sp.width[0];
   sp.count[1] = sp.count[2] = rows_kv(pr, piece) * sp.width[1];
   sp.flag = reinterpret_cast<int*>(ws);
