@@ -785,3 +785,17 @@ def test_packed_rows_nobody_computes_are_zero(dtype):
         out = tf.flash_attn_varlen_forward(Q, K, V, cu_q, cu_kv, 400, 300).float()
         assert torch.isfinite(out).all()
         assert (out - want).abs().max() <= (2e-3 if dtype == torch.float16 else 5e-6)
+
+
+@pytest.mark.parametrize("n,tail", [(300, 0), (300, 5000), (2, 40000)])
+def test_packed_rows_of_no_sequence_are_zero_for_any_mix_of_lengths(n, tail):
+    """Many one-row sequences, and rows behind the last one that outnumber them: all of those are zeroed, nothing else is."""
+    cu_q = torch.arange(n + 1, dtype=torch.int32, device="cuda")
+    cu_kv = (torch.arange(n + 1, device="cuda") * 20).int()
+    Q, K, V = (torch.randn(r, h, 64, device="cuda").half() for r, h in ((n + tail, 4), (20 * n, 2), (20 * n, 2)))
+    want = tf.flash_attn_forward(Q[:n, None].contiguous(), K.view(n, 20, 2, 64), V.view(n, 20, 2, 64))[:, 0].float()
+    junk = torch.full_like(Q, float("nan"))
+    del junk  # the allocator hands this block out again
+    out = tf.flash_attn_varlen_forward(Q, K, V, cu_q, cu_kv, 1, 20).float()
+    assert (out[:n] - want).abs().max() <= 2e-3
+    assert (out[n:] == 0).all()

@@ -693,7 +693,11 @@ extern "C" int tfa_b200_varlen_zero(void* O, const int* cuSeqLensQ, const int* c
   if ((rc = check_device()) != kOk) return rc;
   const int rowChunks = (int)((long long)numHeadsQ * headDim * (dtype == kFp32 ? 4 : 2) / 16);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const cudaError_t e = launch_kernel(varlen_zero_kernel, dim3((unsigned)batchSize + 1, 16), 256, 0, s, may_overlap(s),
+  // CTAs per sequence: four 16-byte pieces per thread at the mean length, at most 16.  Sixteen for every sequence were 16400 CTAs
+  // with nothing to do on a decode step of 1024 sequences.
+  long long perSequence = totalQ * rowChunks / (1024ll * (batchSize + 1)) + 1;
+  if (perSequence > 16) perSequence = 16;
+  const cudaError_t e = launch_kernel(varlen_zero_kernel, dim3((unsigned)batchSize + 1, (unsigned)perSequence), 256, 0, s, may_overlap(s),
                                       static_cast<uint4*>(O), cuSeqLensQ, cuSeqLensKV, batchSize, maxSeqLenQ, totalQ, rowChunks);
   if (e != cudaSuccess) {
     set_error_string("zero kernel launch failed: %s", cudaGetErrorString(e));
