@@ -708,8 +708,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   if constexpr (kPair) ptx::cluster_sync();  // the other CTA's barriers are initialised before anyone arrives on them
   ptx::tc_fence_after();
   const uint32_t tmem = ctl->tmemBase;
-  if (warp != kLoadWarp) ptx::grid_wait_previous();  // the loading thread: below
-  ptx::grid_allow_next();
+  if (warp != kLoadWarp) {  // the loading thread: below
+    ptx::grid_wait_previous();
+    ptx::grid_allow_next();
+  }
   const WaitCtx wc{&ctl->failed, p.status, p.epoch};
 
   // Every consumer of work items (8 softmax warps, 4 epilogue warps, 2 MMA threads) reads item k from slot k & 1
