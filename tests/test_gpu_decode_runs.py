@@ -2,10 +2,13 @@
 
 Sizes where it can go wrong: an entry that is one run, runs that end inside an entry and go on into the next one, last
 blocks that are nearly empty, more entries than runs, one KV head and many, and the same call through the entry point that
-allocates nothing.  Tolerance: weights and output are rounded to 16 bits, 2^-9 (bf16) or 2^-12 (fp16) of values below 4."""
+allocates nothing.
+
+Bound: weights and output are rounded to 16 bits, in all 2.4e-3 (bf16) or 2.9e-4 (fp16) of the result's 2-norm; over the 32
+and more values of one (entry, head) up to twice that.  The values of the first and last key of every 64-key block are eight times
+as large as the others, so that one of them lost or taken twice moves its rows by about 3 / sqrt(keys): 2e-2 at 20000."""
 import ctypes
 
-import numpy as np
 import pytest
 import torch
 
@@ -35,17 +38,23 @@ def test_even_partition(shape, D, dtype):
     g = torch.Generator(device="cuda").manual_seed(D + Skv)
     Q, K, V = (torch.randn(*s, device="cuda", generator=g).to(dtype)
                for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
+    V[:, sorted({*range(0, Skv, 64), *range(63, Skv, 64), Skv - 1})] *= 8
     got = tf.flash_attn_forward(Q, K, V)
     flat = torch.empty_like(Q)
     rc = _lib.load().tfa_b200_fwd_decode_noalloc(
         *(ctypes.c_void_p(t.data_ptr()) for t in (Q, K, V, flat)), 1 if dtype == torch.float16 else 2, B, Sq, Skv, Hq, Hkv,
         D, 0, 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
     assert rc == 0
+    tf.set_option("split_kv", 1)  # whole (batch, KV head) pairs
+    whole = tf.flash_attn_forward(Q, K, V)
+    tf.set_option("split_kv", -1)
     tf.device_status()
     assert torch.equal(got, flat)
     pick = sorted({0, B // 2, B - 1})
-    ref = ao.fixed(*(t[pick].float().cpu().numpy() for t in (Q, K, V)), False, "f64")
-    assert np.abs(got[pick].float().cpu().numpy() - ref).max() <= (2e-3 if dtype == torch.float16 else 1.6e-2)
+    ref = torch.from_numpy(ao.fixed(*(t[pick].float().cpu().numpy() for t in (Q, K, V)), False, "f64")).cuda()
+    bound = 6e-4 if dtype == torch.float16 else 5e-3
+    for other, mine, times in ((ref.float(), got[pick].float(), 1), (whole.float(), got.float(), 2**0.5)):  # both are rounded
+        assert ((mine - other).norm(dim=(1, 3)) <= times * bound * other.norm(dim=(1, 3))).all()
 
 
 def test_packed_sequence_longer_than_the_stated_maximum():

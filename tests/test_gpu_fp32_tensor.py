@@ -171,3 +171,38 @@ def test_rows_of_no_sequence_do_not_matter(D):
     for t, cu in ((Q, cu_q), (K, cu_kv), (V, cu_kv)):
         t[:cu[0]] = t[cu[-1]:] = float("nan")
     assert torch.equal(_with(1, call), want)
+
+
+@pytest.mark.parametrize("D", [32, 64, 96, 128, 192, 256])
+@pytest.mark.parametrize("shape", [  # batch, seqQ, seqKV, headsQ, headsKV
+    (1, 20, 3000, 4, 2),  # key ranges
+    (2, 129, 200, 4, 4),
+    (4, 260, 300, 40, 8),  # head dim 128: the 8 x 8 form behind it
+])
+def test_calls_left_to_the_cuda_cores_in_every_form(shape, D):
+    """One NaN: the CUDA cores' result bit for bit, at every head dim, with and without key ranges, fixed length and packed."""
+    B, Sq, Skv, Hq, Hkv = shape
+    dev = [torch.from_numpy(x).cuda() for x in _inputs(B, Sq, Skv, Hq, Hkv, D, 9)]
+    dev[2][B - 1, Skv // 2, 1, 3] = float("nan")
+    call = lambda: tf.flash_attn_forward(*dev)
+    got, old = _with(1, call), _with(0, call)
+    assert torch.isnan(old).any() and torch.equal(got.view(torch.int32), old.view(torch.int32))
+    cu = [torch.arange(B + 1, dtype=torch.int32, device="cuda") * n for n in (Sq, Skv)]
+    packed = [t.flatten(0, 1) for t in dev]
+    call = lambda: tf.flash_attn_varlen_forward(*packed, *cu, Sq, Skv)
+    got, old = _with(1, call), _with(0, call)
+    assert torch.isnan(old).any() and torch.equal(got.view(torch.int32), old.view(torch.int32))
+
+
+@pytest.mark.parametrize("shape,D", [((1, 128, 128, 4, 4), 64), ((2, 200, 384, 4, 2), 128), ((1, 300, 700, 2, 2), 256)])
+def test_sums_of_one_sign(shape, D):
+    """An accumulator that cuts off instead of rounding has a bias, which shows where all summands have one sign: positive values,
+    keys and queries with a common offset.  No further off 64 bits than the CUDA cores by more than the spread of the other tests."""
+    Q, K, V = _inputs(*shape, D, 21)
+    for q, k, v in ((Q, K, np.abs(V)), (Q, K, V + np.float32(10)), (Q + np.float32(1), K + np.float32(3), np.abs(V)),
+                    (np.abs(Q), np.abs(K), np.abs(V)), (Q * np.float32(6), K * np.float32(6), V)):
+        dev = [torch.from_numpy(x).cuda() for x in (q, k, v)]
+        ref = ao.fixed(q, k, v, False, "f64")
+        got = _with(1, lambda: tf.flash_attn_forward(*dev)).cpu().numpy()
+        old = _with(0, lambda: tf.flash_attn_forward(*dev)).cpu().numpy()
+        assert np.linalg.norm(got - ref) <= 1.25 * np.linalg.norm(old - ref)

@@ -1,9 +1,11 @@
 """Tensor-core path with every query tile's keys cut into ranges, against the fp64 oracle and the uncut call (run with -m gpu).
 
 Sizes: ranges of one block, a last range of one key, tiles with fewer blocks than a range (causal), a tile pair of which
-only one half reaches a range, grouped heads, every head dim.  The combined result differs from the uncut one by fp32
-roundings before the last rounding to 16 bits, so the same bound as for the uncut kernel holds."""
-import numpy as np
+only one half reaches a range, grouped heads, every head dim.
+
+Bound: weights and output are rounded to 16 bits, in all 2.4e-3 (bf16) or 2.9e-4 (fp16) of the result's 2-norm, over a single row
+up to four times that; the uncut call is within the same bound.  The values of the first and last key of every 128-key block are
+eight times as large as the others, so that one of them lost or weighted wrongly moves its rows by about 3 / sqrt(keys): 8e-2 at 1153."""
 import pytest
 import torch
 
@@ -41,10 +43,13 @@ def test_ranges(shape, D, causal):
     g = torch.Generator(device="cuda").manual_seed(Sq + D)
     Q, K, V = (torch.randn(*s, device="cuda", generator=g).to(dtype)
                for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
-    ref = ao.fixed(*(t.float().cpu().numpy() for t in (Q, K, V)), causal, "f64")
-    for parts in (0, 2, 3, 8):
-        out = _run(parts, lambda: tf.flash_attn_forward(Q, K, V, is_causal=causal)).float().cpu().numpy()
-        assert np.abs(out - ref).max() <= 2e-2, parts
+    V[:, sorted({*range(0, Skv, 128), *range(127, Skv, 128), Skv - 1})] *= 8
+    ref = torch.from_numpy(ao.fixed(*(t.float().cpu().numpy() for t in (Q, K, V)), causal, "f64")).cuda().float()
+    bound = 1.2e-3 if dtype == torch.float16 else 1e-2
+    outs = {parts: _run(parts, lambda: tf.flash_attn_forward(Q, K, V, is_causal=causal)).float() for parts in (0, 2, 3, 8)}
+    for parts, out in outs.items():
+        for other in (ref, outs[0]):  # 2-norm of every row
+            assert ((out - other).norm(dim=3) <= bound * other.norm(dim=3)).all(), parts
 
 
 def test_a_nan_key_poisons_the_rows_that_see_it():
