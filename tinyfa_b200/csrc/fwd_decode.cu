@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
   constexpr int kLdO = merge_ld<D>();
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sBase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  float* sO = reinterpret_cast<float*>(smem + kStages * 2 * kTileBytes);  // [16][kLdO]
+  // merge buffer: behind the ring where the next entry's blocks are on their way into it meanwhile, else in it
+  float* sO = reinterpret_cast<float*>(smem + (p.runs > 0 ? kStages * 2 * kTileBytes : 0));  // [16][kLdO]
   float* sM = sO + kRows * kLdO;                                          // [4][16]
   float* sL = sM + 4 * kRows;                                             // [4][16]
 
@@ -588,7 +589,8 @@ int launch_combine(const FwdProblem& p, int packShift, const TcSplit& split) {
   return kOk;
 }
 
-constexpr int smem_bytes(int D) { return kStages * 2 * kBlockKeys * D * 2 + (kRows * (D + 8) + 8 * kRows) * (int)sizeof(float); }
+constexpr int ring_bytes(int D) { return kStages * 2 * kBlockKeys * D * 2; }
+constexpr int merge_bytes(int D) { return (kRows * (D + 8) + 8 * kRows) * (int)sizeof(float); }
 // CTAs of the even partition, in quarters of an SM's share.  Not all that shared memory holds where it holds more than
 // one: measured us at 8 KV heads, batch 4 / 8 / 28 of D = 128: 296 CTAs 93.2 / 110.6 / 114.4, 280 89.3 / 106.0 / 112.1, 256
 // 86.8 / 102.6 / 108.3, 224 88.5 / 105.1 / 106.6, 148 107 / 125 / 137; D = 64, batch 4 / 24: 592 49.9 / 72.8, 444 46.8 / 66.8,
@@ -597,8 +599,8 @@ constexpr int quarter_ctas_per_sm(int D) { return D == 32 ? 16 : D == 64 ? 12 : 
 
 template <int D, bool kBf16>
 int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* partLse) {
-  constexpr int kSmem = smem_bytes(D);
-  static_assert(kSmem <= 227 * 1024 && merge_ld<D>() == D + 8, "shared memory");
+  constexpr int kSmem = ring_bytes(D) + merge_bytes(D);
+  static_assert(kSmem <= 227 * 1024 && merge_bytes(D) <= ring_bytes(D) && merge_ld<D>() == D + 8, "shared memory");
   auto kernel = fwd_splitkv_kernel<D, kBf16>;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return kCudaError;
@@ -635,7 +637,9 @@ int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* par
   p.totalQ = pr.totalQ;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   const dim3 grid = plan.runs > 0 ? dim3((unsigned)(plan.runs * pr.headsKV)) : dim3((unsigned)plan.splits, (unsigned)pr.headsKV, (unsigned)pr.batch);
-  cudaError_t e = launch_kernel(kernel, grid, kThreads, kSmem, pr.stream, pr.overlap, p);
+  // head dim 96 fits three CTAs per SM without the merge buffer, two with it: 6 x 715 keys, batch 104, 32 heads 162 -> 145 us
+  const size_t smem = plan.runs > 0 ? kSmem : ring_bytes(D);
+  cudaError_t e = launch_kernel(kernel, grid, kThreads, smem, pr.stream, pr.overlap, p);
   if (e == cudaSuccess && plan.splits > 1) {
     const long long rows = pr.totalQ * pr.headsQ;
     const int tileRows = pr.seqLenQ * p.group;  // a longer sequence than the caller's maximum: the CTAs take turns
