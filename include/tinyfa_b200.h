@@ -97,7 +97,8 @@ int tfa_b200_device_status(int* site);
  * at compile time (csrc/flash_attn/config.cuh:133-272).
  *   "pack_gqa" -1/0/1  interleave the Q heads of a KV group into one 128-row tile: auto (short query blocks and
  *                      causal problems) / never / always
- *   "split_kv" -1/0/n  split-KV path for short query blocks (seqQ * group <= 16): auto / never / exactly n splits
+ *   "split_kv" -1/0/n  split-KV path for short query blocks (seqQ * group <= 16): auto / never / exactly n splits; -2: equal
+ *                      runs of key blocks over the batch wherever fixed-length input allows them, also where auto does not cut
  *   "split_tc" -1/0/n  tensor-core path, fixed-length input: every query tile's keys cut into n ranges whose partial results
  *                      a second kernel combines: auto (few query tiles for long keys) / never / n ranges.  Not under
  *                      stream capture.

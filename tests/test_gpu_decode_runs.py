@@ -39,17 +39,20 @@ def test_even_partition(shape, D, dtype):
     Q, K, V = (torch.randn(*s, device="cuda", generator=g).to(dtype)
                for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
     V[:, sorted({*range(0, Skv, 64), *range(63, Skv, 64), Skv - 1})] *= 8
-    got = tf.flash_attn_forward(Q, K, V)
+    def cut(how):
+        tf.set_option("split_kv", how)
+        out = tf.flash_attn_forward(Q, K, V)
+        tf.set_option("split_kv", -1)
+        return out
+
+    got, whole, auto = cut(-2), cut(1), cut(-1)  # equal runs, whole (batch, KV head) pairs, the library's choice
     flat = torch.empty_like(Q)
     rc = _lib.load().tfa_b200_fwd_decode_noalloc(
         *(ctypes.c_void_p(t.data_ptr()) for t in (Q, K, V, flat)), 1 if dtype == torch.float16 else 2, B, Sq, Skv, Hq, Hkv,
         D, 0, 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
     assert rc == 0
-    tf.set_option("split_kv", 1)  # whole (batch, KV head) pairs
-    whole = tf.flash_attn_forward(Q, K, V)
-    tf.set_option("split_kv", -1)
     tf.device_status()
-    assert torch.equal(got, flat)
+    assert torch.equal(auto, flat) and (torch.equal(auto, got) or torch.equal(auto, whole))
     pick = sorted({0, B // 2, B - 1})
     ref = torch.from_numpy(ao.fixed(*(t[pick].float().cpu().numpy() for t in (Q, K, V)), False, "f64")).cuda()
     bound = 6e-4 if dtype == torch.float16 else 5e-3
@@ -152,3 +155,23 @@ def test_packed_rows_without_partials_stay_zero(Hq, Hkv, most):
         out = tf.flash_attn_varlen_forward(Q, K, V, cu_q, cu_kv, most, 3000).float()
         assert (out - want).abs().max() <= 2e-3
         assert (out[want.abs().amax(dim=(1, 2)) == 0] == 0).all()
+
+
+@pytest.mark.parametrize("shape,D,runs", [  # the faster cut by a factor of 1.2 at least
+    ((59, 2, 442, 128, 16), 32, False),
+    ((172, 1, 839, 64, 4), 32, False),
+    ((102, 13, 304, 8, 8), 96, False),
+    ((398, 16, 519, 4, 4), 128, False),
+    ((40, 1, 5000, 32, 8), 128, True),
+    ((1, 1, 32768, 32, 8), 128, True),
+    ((8, 1, 20011, 32, 8), 128, True),
+])
+def test_cut_by_cost(shape, D, runs):
+    """Many short entries are not cut: the combine pass over their rows would cost more than even ends save."""
+    B, Sq, Skv, Hq, Hkv = shape
+    Q, K, V = (torch.randn(*s, device="cuda").bfloat16() for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
+    auto = tf.flash_attn_forward(Q, K, V)
+    tf.set_option("split_kv", -2 if runs else 1)
+    want = tf.flash_attn_forward(Q, K, V)
+    tf.set_option("split_kv", -1)
+    assert torch.equal(auto, want)

@@ -73,7 +73,7 @@ void set_error_string(const char* fmt, ...) {
 }
 
 static std::atomic<int> g_optPackGqa{-1};
-static std::atomic<int> g_optSplitKv{-1};  // -1 auto, 0 never, n > 0 force n splits when applicable
+static std::atomic<int> g_optSplitKv{-1};  // -1 auto, -2 equal runs, 0 never, n > 0 force n splits when applicable
 static std::atomic<int> g_optWorkOrder{-1};  // -1 auto, 0 pair index fastest, n > 0 heaviest first in chunks of n
 static std::atomic<int> g_epoch{1};
 
@@ -746,7 +746,7 @@ extern "C" int tfa_b200_set_option(const char* name, int value) {
     return kOk;
   }
   if (strcmp(name, "split_kv") == 0) {
-    g_optSplitKv.store(value < 0 ? -1 : value);
+    g_optSplitKv.store(value < -2 ? -1 : value);
     return kOk;
   }
   if (strcmp(name, "narrow_mma") == 0) {

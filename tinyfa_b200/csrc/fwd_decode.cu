@@ -597,6 +597,9 @@ constexpr int merge_bytes(int D) { return (kRows * (D + 8) + 8 * kRows) * (int)s
 // 296 46.8 / 68.0; D = 32: 592 47.3, 444 50.4, 296 58.6; D = 96: 296 44.2, 256 44.5; D = 192 / 256 hold one per SM.
 constexpr int quarter_ctas_per_sm(int D) { return D == 32 ? 16 : D == 64 ? 12 : D <= 128 ? 7 : 4; }
 
+// CTAs of an SM without the even partition: registers up to head dim 96, shared memory above.
+constexpr int whole_ctas_per_sm(int D) { return D == 32 ? 5 : D <= 96 ? 3 : D == 128 ? 2 : 1; }
+
 template <int D, bool kBf16>
 int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* partLse) {
   constexpr int kSmem = ring_bytes(D) + merge_bytes(D);
@@ -674,8 +677,8 @@ static int splits_of_pairs(const FwdProblem& p, int numSMs) {
   return splits < 1 ? 1 : (int)splits;
 }
 
-// How a call is cut.  forced > 0: that many key-range splits of every pair, on a three-dimensional grid; the same with
-// a number of its own for packed input, whose lengths the host does not know.  Fixed-length input is cut evenly: the key
+// How a call is cut.  forced > 0: that many key-range splits of every pair, on a three-dimensional grid (-2: the even partition
+// below wherever it is possible, whatever it costs); the same with a number of its own for packed input, whose lengths the host does not know.  Fixed-length input is cut evenly: the key
 // blocks of all batch entries in a row, as many equal runs as the GPU holds at once, so that no SM waits for another at the
 // end whatever the batch is.  All KV heads of a run are cut at the same keys: cut one by one, their CTAs drift apart and
 // read the pieces of a row of K at different times, which cost up to half of the bandwidth (D = 32, 64-byte pieces).
@@ -698,6 +701,17 @@ SplitPlan splitkv_plan(const FwdProblem& p, int numSMs, int forced) {
     plan.blocksPerEntry = (int)blocks;
     const long long run = total / runs;  // the shortest run; partial results per pair:
     plan.splits = (int)(p.batch % runs == 0 ? 1 : runs % p.batch == 0 ? runs / p.batch : (blocks - 2) / run + 2);
+    // Against whole pairs, one CTA each.  In us: a block takes 4e-5 D of the memory rate and at least 0.345 + 0.00425 D in one CTA,
+    // and the combine kernel 3.7 and 0.95e-3 + 4.9e-6 D a row.  Fitted to 196 drawn calls of 120 pairs and more, all head dims: the pick
+    // is within 0.7 % of the faster cut on average, 14 % at worst.  us per call, runs against whole pairs: 59 x 2 x 442 keys, 128
+    // over 16 heads of 32 32.1, 12.3; 172 x 1 x 839, 64 over 4 of 32 32.9, 14.3; 398 x 16 x 519, 4 heads of 128 114, 85; on the
+    // other side 40 x 5000, 32 over 8 of 128 130, 174.
+    const double D = p.headDim, block = 4e-5 * D, chain = 0.345 + 0.00425 * D;
+    const long long held = (long long)numSMs * decode::whole_ctas_per_sm(p.headDim), rest = pairs % held;
+    const double whole = (double)(pairs / held) * blocks * held * block + (rest > 0 ? blocks * fmax(rest * block, chain) : 0.0);
+    const double cut = fmax((double)pairs * blocks * block, (double)((total + runs - 1) / runs) * chain) +
+                       (plan.splits > 1 ? 3.7 + (double)p.totalQ * p.headsQ * (0.95e-3 + 4.9e-6 * D) : 0.0);
+    if (whole <= cut && forced != -2) return SplitPlan{1, 0, 0};
     return plan;
   }
   plan.splits = splits_of_pairs(p, numSMs);  // packed input, and more pairs than the even partition is for
@@ -866,7 +880,7 @@ extern "C" int tfa_b200_fwd_decode_noalloc(const void* Q, const void* K, const v
   }
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  SplitPlan plan = splitkv_plan(p, sms, numSplits);
+  SplitPlan plan = splitkv_plan(p, sms, numSplits > 0 ? numSplits : 0);
   // What the entry point accepts is stated in splits of pairs; an even partition whose partials do not fit the array gives
   // way to whole pairs, as many at a time as the GPU holds.
   const SplitPlan stated = {plan.runs > 0 ? splits_of_pairs(p, sms) : plan.splits, 0, 0};
