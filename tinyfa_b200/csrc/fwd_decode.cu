@@ -571,10 +571,11 @@ int launch_combine(const FwdProblem& p, int packShift, const TcSplit& split) {
   constexpr int kGroups = kCombineThreads / (D / 4);
   const long long rows = p.totalQ * p.headsQ;
   cudaError_t e;
-  if (!p.causal && split.parts >= 6 && rows <= 16384) {
-    // Many ranges for few rows: one CTA per row, whose threads read the ranges side by side (without the mask every tile has
-    // all ranges).  us a call, the kernel below -> this one: 60 rows of four heads x 20000 keys D64 19.2 -> 14.1, 34 x 7508 16 heads
-    // 25.5 -> 23.3, 1400 x 8000 2 heads 30.2 -> 28.0, 2 x 8 x 12289 32 heads 31.5 -> 31.1.
+  if (!p.causal && (rows <= 1024 || (rows <= 3072 && split.parts >= 12))) {
+    // Few rows: one CTA per row, whose threads read the ranges side by side (without the mask every tile has all ranges).  us a call
+    // at head dim 128, the kernel below -> this one, with 3, 6, 12 ranges: 512 rows 15.4 -> 14.7, 16.8 -> 15.1, 17.7 -> 15.8; 1024 16.7 -> 16.2,
+    // 17.9 -> 16.5, 19.2 -> 17.4; 3072 17.4 -> 18.8, 24.8 -> 23.7, 38.7 -> 37.6; 4096 and 4, 6, 8 ranges 22.7 -> 20.6, 24.3 -> 26.0, 24.1 ->
+    // 26.6; 8192 25.9 -> 29.4, 44.0 -> 45.9, 46.6 -> 50.6.
     e = launch_kernel(combine_kernel<D, kBf16>, dim3((unsigned)rows), kCombineThreads, 0, p.stream, p.overlap, split.partO,
                       split.partLse, p.O, rows, split.parts, nullptr, nullptr, p.headsQ, 1, 0, 0, 0ll, p.seqLenQ);
   } else {
