@@ -205,7 +205,9 @@ def measured_hbm():
 def launches_per_step(w):
     """Kernels of this library that one step of the Python API launches on this workload."""
     if w["kind"] == "decode":
-        return 2 if w["B"] * w["Hkv"] < 148 else 1  # the split kernel, and the combine kernel where a sequence is cut
+        # the split kernel, and the combine kernel where an entry is cut: runs of key blocks at head dim 128 and 148 SMs
+        runs = min(max(w["B"] * ((w["Skv"] + 63) // 64) // 4, w["B"]), 148 * 7 // 4 // w["Hkv"])
+        return 1 if w["B"] % runs == 0 else 2
     if w["kind"] == "varlen":
         return 2  # rows nobody writes, attention
     if w["dtype"] == "fp32" and w["Sq"] >= 256:

@@ -13,7 +13,9 @@
  * counters and tensor-map slots, shared-memory opt-in of the kernels, a scratch pool) with synchronous calls; make it
  * outside a stream capture.  After that a forward call only enqueues kernels on `stream` (the split-KV path of
  * tfa_b200_fwd, and eager calls in fp32 or with key ranges, also a stream-ordered allocation and free;
- * tfa_b200_fwd_decode_noalloc none), so it can be captured into a CUDA graph and replayed.  The persistent kernel hands
+ * tfa_b200_fwd_decode_noalloc none), so it can be captured into a CUDA graph and replayed.  Captured calls in fp32 stay on
+ * the CUDA cores and captured calls of few query rows run without key ranges, so that their graphs hold no allocation: the
+ * results may differ from an eager call's in the order of fp32 sums.  The persistent kernel hands
  * out its work through a pair of device counters that two
  * launches must not use at the same time: eager launches take the pair of their stream (up to 1024 distinct streams
  * per device; the per-thread default stream counts once per calling thread), every captured launch takes a pair of
@@ -108,7 +110,9 @@ int tfa_b200_device_status(int* site);
  *                      CTAs per SM (the default) / 8 x 8 always
  *   "fp32_tc" -1/0/1   fp32: on the tensor cores with every float as three bf16 numbers by size /
  *                      never / wherever it applies (not under stream capture, not for packed input of unknown totals).
- *                      Choosing a CUDA-core form with "fp32_t8" switches "by size" off.
+ *                      Choosing a CUDA-core form with "fp32_t8" switches "by size" off.  A NaN, an infinity or a magnitude
+ *                      outside [2^-100, 2^60) other than zero, anywhere in Q, K or V, leaves the call to the CUDA cores on
+ *                      the device: the same result as with 0, in their time and 3 to 16 % more.
  *   "pair_cta" -1/0/1  head dims 192 / 256, fixed-length input: clusters of two CTAs that work on two neighbouring query
  *                      tiles and share every K/V block through one MMA over both SMs (tcgen05 cta_group::2):
  *                      auto (head dim 256: non-causal, and causal from 1024 query rows; head dim 192: never, its

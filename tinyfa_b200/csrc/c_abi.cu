@@ -387,7 +387,9 @@ static int dispatch_splitkv(const FwdProblem& p, const SplitPlan& plan) {
 // fp32: the tensor cores where that pays, else the CUDA cores.  The tensor-core kernel leaves inputs that its three-part
 // form does not hold exactly (infinities, NaN, extreme magnitudes) to the CUDA-core kernel, which is enqueued behind it and
 // decides on the device.  Nothing is refused for lack of workspace: the CUDA cores need none.  A stream under capture stays
-// on the CUDA cores, because an allocation captured into a graph would limit what the caller may do with that graph.
+// on the CUDA cores, as before there were tensor-core kernels: a graph that allocates cannot be cloned or instantiated twice at
+// a time, and graphs of these calls could.  (The split-KV path has always allocated under capture.)  So a captured call and an
+// eager one may differ in the last bits of their sums.
 static int dispatch_fp32(const FwdProblem& p) {
   const int opt = g_optFp32Tc.load();
   // an explicit choice of the CUDA-core form (option "fp32_t8") is kept

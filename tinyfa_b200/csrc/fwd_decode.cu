@@ -13,9 +13,10 @@
 //     (mma.sync m16n8k16, fp32 accumulate: the tensor work is negligible next to the memory stream);
 //   * warps are merged through shared memory, partial results through a small fp32 scratch buffer and a combine kernel
 //     that is launched while the split kernel runs (programmatic dependent launch) and reads a row's partials side by side.
-// Measured against a fixed number of splits per pair and a combine kernel that walked them (8 KV heads, D = 128, floor in
-// brackets at 6.54 TB/s): batch 1 x 32768 keys 37.0 -> 27.8 us (20.5), 8 x 20011 111 -> 100 (100), 40 x 5000 174 -> 135 (125), 13 x
-// 8000 74 -> 74 (65), 6 x 12000 58 -> 55 (45).  What is left at small batch is launch, the first loads and the combine.
+// Measured against a fixed number of splits per pair and a combine kernel that walked them (8 KV heads, D = 128, three sets of
+// inputs in turn, both builds in one job; floor in brackets at 6.54 TB/s): batch 1 x 32768 keys 37.6 -> 28.4 us (20.5), 8 x 20011
+// 112.3 -> 100.4 (100; with inputs spread over more memory 113.4 -> 105.6), 40 x 5000 169.6 -> 127.7 (125), 13 x 8000 76.0 -> 71.6 (65),
+// 6 x 12000 61.6 -> 51.8 (45).  What is left at small batch is launch, the first loads and the combine.
 // Numerical contract as in the main kernel (reference csrc/flash_attn/mma/softmax.cuh:67-138): scale 1/sqrt(D)
 // folded into exp2, top-left causal mask, "col >= seqLenKV" mask, P rounded to the 16-bit type before P.V, row sum
 // from unrounded P, empty rows give 0.
@@ -641,7 +642,7 @@ int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* par
   p.totalQ = pr.totalQ;
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   const dim3 grid = plan.runs > 0 ? dim3((unsigned)(plan.runs * pr.headsKV)) : dim3((unsigned)plan.splits, (unsigned)pr.headsKV, (unsigned)pr.batch);
-  // head dim 96 fits three CTAs per SM without the merge buffer, two with it: 6 x 715 keys, batch 104, 32 heads 162 -> 145 us
+  // head dim 96 fits three CTAs per SM without the merge buffer, two with it: packed, 223 x up to 5432 keys, 2 heads 138 -> 118 us
   const size_t smem = plan.runs > 0 ? kSmem : ring_bytes(D);
   cudaError_t e = launch_kernel(kernel, grid, kThreads, smem, pr.stream, pr.overlap, p);
   if (e == cudaSuccess && plan.splits > 1) {
@@ -712,7 +713,8 @@ SplitPlan splitkv_plan(const FwdProblem& p, int numSMs, int forced) {
     const double whole = (double)(pairs / held) * blocks * held * block + (rest > 0 ? blocks * fmax(rest * block, chain) : 0.0);
     const double cut = fmax((double)pairs * blocks * block, (double)((total + runs - 1) / runs) * chain) +
                        (plan.splits > 1 ? 3.7 + (double)p.totalQ * p.headsQ * (0.95e-3 + 4.9e-6 * D) : 0.0);
-    if (whole <= cut && forced != -2) return SplitPlan{1, 0, 0};
+    // (the factor: without a combine pass both estimates are the bytes, and runs end more evenly than pairs)
+    if (whole <= (plan.splits > 1 ? cut : 0.99 * cut) && forced != -2) return SplitPlan{1, 0, 0};
     return plan;
   }
   plan.splits = splits_of_pairs(p, numSMs);  // packed input, and more pairs than the even partition is for

@@ -9,8 +9,10 @@
 // nearest - the tensor core only ever sums the 128 keys of one block.
 //
 // Measured against the CUDA-core kernels (2-norm error against 64 bits in brackets): non-causal B2 S2048 H16 D128 1596 ->
-// 394 us (9.1e-7 -> 3.1e-7), causal B2 S1999 16 over 4 heads D64 563 -> 127 us (3.9e-7 -> 1.8e-7); on every shape tried,
-// short ones included, the error is below that of the CUDA-core kernels, whose sums run over all keys one at a time.
+// 394 us (9.1e-7 -> 3.1e-7), causal B2 S1999 16 over 4 heads D64 563 -> 127 us (3.9e-7 -> 1.8e-7).  Over ten distributions
+// (zero-mean, one-sign and offset Q, K and V, large and nearly equal scores) x twelve shapes the error is 0.12 to 1.01 of that of the
+// CUDA-core kernels, whose sums run over all keys one at a time; the largest is the accumulator's bias where all values of V are
+// positive and the keys are one block (1.78e-7 against 1.77e-7).
 // One pass over a block takes 7.7 k clocks at D = 128, of which the tensor pipe needs 96 x 64 = 6.1 k; with both products
 // issued by one thread it was 9.4 k.  Left: the dependency S -> softmax -> P.V -> S two blocks on (the two S buffers), the
 // last wave of tiles, and 40 us for the split at that shape (6.2 TB/s).
