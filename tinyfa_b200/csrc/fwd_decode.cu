@@ -33,6 +33,9 @@
 #include "tfa_common.cuh"
 
 namespace tfa_b200 {
+
+int device_num_sms(int device);  // c_abi.cu
+
 namespace decode {
 
 constexpr int kThreads = 128;
@@ -161,28 +164,33 @@ __host__ __device__ __forceinline__ int run_of_block(long long u, long long tota
   return (int)(((u + 1) * runs - 1) / total);
 }
 
-template <int D, bool kBf16>
-__global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
+// kEven: the even partition; else one CTA per (split, KV head, batch entry).  Instantiations of their own, and a load address worked out
+// anew for every block: the code that carries a run on into the next entry cost calls of whole pairs up to 3 % (16 x 16384 keys, 32 heads over 32
+// of 128 667 -> 641 us).  The number of CTAs per SM is stated because without it the compiler keeps to 168 registers at head dim 128, where two
+// CTAs have 255 each: runs 665 -> 617 us there.  Head dim 32 is better off with 8 CTAs than with 7 of 65 registers.
+template <int D, bool kBf16, bool kEven>
+__global__ void __launch_bounds__(kThreads, (D == 32 && !kEven) ? 8 : 1) fwd_splitkv_kernel(const Params p) {
   constexpr int kTileBytes = kBlockKeys * D * 2;
   constexpr int kNT = D / 8;  // 8-wide output column tiles
   constexpr int kLdO = merge_ld<D>();
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sBase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  // merge buffer: behind the ring where the next entry's blocks are on their way into it meanwhile, else in it
-  float* sO = reinterpret_cast<float*>(smem + (p.runs > 0 ? kStages * 2 * kTileBytes : 0));  // [16][kLdO]
-  float* sM = sO + kRows * kLdO;                                          // [4][16]
+  // merge buffer: behind the ring where the next entry's blocks are on their way into it meanwhile, one warp after the other; else
+  // in the ring, all warps at once (320 CTAs of six blocks at head dim 256: 43.2 -> 39.4 us)
+  constexpr int kParts = kEven ? 1 : 4;
+  float* sO = reinterpret_cast<float*>(smem + (kEven ? kStages * 2 * kTileBytes : 0));  // [kParts][16][kLdO]
+  float* sM = sO + kParts * kRows * kLdO;                                 // [4][16]
   float* sL = sM + 4 * kRows;                                             // [4][16]
 
   ptx::grid_wait_previous();
   ptx::grid_allow_next();
-  const bool even = p.runs > 0;
   int b, part;         // batch entry and partial-result slot of the current segment
   int hkv;
   int sq, skv;
   long long qRow0, kvRow0;
   int key0, keyEnd;    // keys of the entry that this CTA starts at / may see
   int count;           // blocks of this CTA
-  if (even) {
+  if constexpr (kEven) {
     // neighbouring CTAs are the KV heads of one run: they read neighbouring parts of the same rows at the same time
     const int run = (int)blockIdx.x / p.headsKV;
     hkv = (int)blockIdx.x - run * p.headsKV;
@@ -279,17 +287,26 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
       MB = fmaxf(MB, sM[w * kRows + rowB]);
     }
     const float fA = (mA == -INFINITY) ? 0.f : ex2((mA - MA) * c), fB = (mB == -INFINITY) ? 0.f : ex2((mB - MB) * c);
+    if constexpr (kEven) {
 #pragma unroll 1
-    for (int w = 0; w < 4; w++) {  // one warp after the other adds its share
-      if (w == warp) {
+      for (int w = 0; w < 4; w++) {  // one warp after the other adds its share
+        if (w == warp) {
 #pragma unroll
-        for (int nt = 0; nt < kNT; nt++) {
-          float2* a = reinterpret_cast<float2*>(sO + rowA * kLdO + nt * 8 + 2 * tig);
-          float2* bq = reinterpret_cast<float2*>(sO + rowB * kLdO + nt * 8 + 2 * tig);
-          const float2 za = (w == 0) ? make_float2(0.f, 0.f) : *a, zb = (w == 0) ? make_float2(0.f, 0.f) : *bq;
-          *a = make_float2(fmaf(o[nt][0], fA, za.x), fmaf(o[nt][1], fA, za.y));
-          *bq = make_float2(fmaf(o[nt][2], fB, zb.x), fmaf(o[nt][3], fB, zb.y));
+          for (int nt = 0; nt < kNT; nt++) {
+            float2* a = reinterpret_cast<float2*>(sO + rowA * kLdO + nt * 8 + 2 * tig);
+            float2* bq = reinterpret_cast<float2*>(sO + rowB * kLdO + nt * 8 + 2 * tig);
+            const float2 za = (w == 0) ? make_float2(0.f, 0.f) : *a, zb = (w == 0) ? make_float2(0.f, 0.f) : *bq;
+            *a = make_float2(fmaf(o[nt][0], fA, za.x), fmaf(o[nt][1], fA, za.y));
+            *bq = make_float2(fmaf(o[nt][2], fB, zb.x), fmaf(o[nt][3], fB, zb.y));
+          }
         }
+        __syncthreads();
+      }
+    } else {
+#pragma unroll
+      for (int nt = 0; nt < kNT; nt++) {
+        *reinterpret_cast<float2*>(sO + (warp * kRows + rowA) * kLdO + nt * 8 + 2 * tig) = make_float2(o[nt][0] * fA, o[nt][1] * fA);
+        *reinterpret_cast<float2*>(sO + (warp * kRows + rowB) * kLdO + nt * 8 + 2 * tig) = make_float2(o[nt][2] * fB, o[nt][3] * fB);
       }
       __syncthreads();
     }
@@ -306,6 +323,14 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
       }
       const float inv = (l > 0.f) ? (1.f / l) : 0.f;
       float4 acc = *reinterpret_cast<const float4*>(sO + r * kLdO + c4 * 4);
+#pragma unroll
+      for (int w = 1; w < kParts; w++) {
+        const float4 v = *reinterpret_cast<const float4*>(sO + (w * kRows + r) * kLdO + c4 * 4);
+        acc.x += v.x;
+        acc.y += v.y;
+        acc.z += v.z;
+        acc.w += v.w;
+      }
       acc.x *= inv;
       acc.y *= inv;
       acc.z *= inv;
@@ -326,34 +351,40 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
 
   startSegment();
   // load cursor: runs kStages - 1 blocks ahead, across segment ends
-  int ldKey = key0;
+  [[maybe_unused]] int ldKey = key0;
   const uint16_t* gK = reinterpret_cast<const uint16_t*>(p.K) + kvRow0 * kvStride + (long long)hkv * D;
   const uint16_t* gV = reinterpret_cast<const uint16_t*>(p.V) + kvRow0 * kvStride + (long long)hkv * D;
-  auto loadNext = [&](int stage) {
-    load_block<D>(sBase + stage * 2 * kTileBytes, gK, kvStride, ldKey, keyEnd);
-    load_block<D>(sBase + stage * 2 * kTileBytes + kTileBytes, gV, kvStride, ldKey, keyEnd);
-    ldKey += kBlockKeys;
-    if (even && ldKey >= keyEnd) {  // the next batch entry
-      ldKey = 0;
-      const long long step = (long long)skv * kvStride;
-      gK += step;
-      gV += step;
+  auto loadBlock = [&](int blk) {
+    const uint32_t stage = sBase + (blk % kStages) * 2 * kTileBytes;
+    if constexpr (kEven) {
+      load_block<D>(stage, gK, kvStride, ldKey, keyEnd);
+      load_block<D>(stage + kTileBytes, gV, kvStride, ldKey, keyEnd);
+      ldKey += kBlockKeys;
+      if (ldKey >= keyEnd) {  // the next batch entry
+        ldKey = 0;
+        const long long step = (long long)skv * kvStride;
+        gK += step;
+        gV += step;
+      }
+    } else {
+      load_block<D>(stage, gK, kvStride, key0 + blk * kBlockKeys, keyEnd);
+      load_block<D>(stage + kTileBytes, gV, kvStride, key0 + blk * kBlockKeys, keyEnd);
     }
   };
 #pragma unroll
   for (int s = 0; s < kStages - 1; s++) {
-    if (s < count) loadNext(s);
+    if (s < count) loadBlock(s);
     cp_async_commit();
   }
-  int segStart = key0, kbase = key0;  // first key of the segment / of the block
+  [[maybe_unused]] int segStart = key0, kbase = key0;  // first key of the segment / of the block
   for (int blk = 0; blk < count; blk++) {
-    if (blk + kStages - 1 < count) loadNext((blk + kStages - 1) % kStages);
+    if (blk + kStages - 1 < count) loadBlock(blk + kStages - 1);
     cp_async_commit();
     cp_async_wait<kStages - 1>();
     __syncthreads();
     const uint32_t sK = sBase + (blk % kStages) * 2 * kTileBytes;
     const uint32_t sV = sK + kTileBytes;
-    const int kb = kbase + warp * 16;  // first key of this warp's 16-key slice
+    const int kb = (kEven ? kbase : key0 + blk * kBlockKeys) + warp * 16;  // first key of this warp's 16-key slice
     if (kb < keyEnd) {
       // ---- S = Q K^T for 16 rows x 16 keys
       float sc[2][4];
@@ -431,20 +462,22 @@ __global__ void __launch_bounds__(kThreads) fwd_splitkv_kernel(const Params p) {
       }
     }
     __syncthreads();
-    kbase += kBlockKeys;
-    const bool entryDone = even && kbase >= keyEnd;
-    if (entryDone || blk + 1 == count) {
-      storeSegment(even ? (entryDone && segStart == 0) : p.splits == 1);
-      if (blk + 1 < count) {  // on to the next batch entry, whose blocks are already on their way
-        qRow0 += sq;
-        segStart = kbase = 0;
-        part = 0;
-        startSegment();
+    if constexpr (kEven) {
+      kbase += kBlockKeys;
+      const bool entryDone = kbase >= keyEnd;
+      if (entryDone || blk + 1 == count) {
+        storeSegment(entryDone && segStart == 0);
+        if (blk + 1 < count) {  // on to the next batch entry, whose blocks are already on their way
+          qRow0 += sq;
+          segStart = kbase = 0;
+          part = 0;
+          startSegment();
+        }
       }
     }
   }
   cp_async_wait<0>();
-  if (count == 0) storeSegment(p.splits == 1);  // a split without keys (never in an even partition): zeros, lse = -inf
+  if constexpr (!kEven) storeSegment(p.splits == 1);  // a split without keys: zeros, lse = -inf
 }
 
 // O[row] = sum_s 2^(lse_s - M) O_s / sum_s 2^(lse_s - M), one CTA per output row.  Bound by the latency of two dependent
@@ -591,31 +624,35 @@ int launch_combine(const FwdProblem& p, int packShift, const TcSplit& split) {
   return kOk;
 }
 
+constexpr int kMaxSmem = 227 * 1024, kSmemReserved = 1024, kSmemPerSm = 228 * 1024;  // of a CTA, taken by the system per CTA, of an SM
 constexpr int ring_bytes(int D) { return kStages * 2 * kBlockKeys * D * 2; }
-constexpr int merge_bytes(int D) { return (kRows * (D + 8) + 8 * kRows) * (int)sizeof(float); }
+constexpr int merge_bytes(int D, int parts) { return (parts * kRows * (D + 8) + 8 * kRows) * (int)sizeof(float); }
 // CTAs of the even partition, in quarters of an SM's share.  Not all that shared memory holds where it holds more than
 // one: measured us at 8 KV heads, batch 4 / 8 / 28 of D = 128: 296 CTAs 93.2 / 110.6 / 114.4, 280 89.3 / 106.0 / 112.1, 256
 // 86.8 / 102.6 / 108.3, 224 88.5 / 105.1 / 106.6, 148 107 / 125 / 137; D = 64, batch 4 / 24: 592 49.9 / 72.8, 444 46.8 / 66.8,
 // 296 46.8 / 68.0; D = 32: 592 47.3, 444 50.4, 296 58.6; D = 96: 296 44.2, 256 44.5; D = 192 / 256 hold one per SM.
 constexpr int quarter_ctas_per_sm(int D) { return D == 32 ? 16 : D == 64 ? 12 : D <= 128 ? 7 : 4; }
 
-// CTAs of an SM without the even partition: registers up to head dim 96, shared memory above.
-constexpr int whole_ctas_per_sm(int D) { return D == 32 ? 5 : D <= 96 ? 3 : D == 128 ? 2 : 1; }
+// CTAs of an SM without the even partition: the stated 8, registers up to head dim 96, shared memory above.
+constexpr int whole_ctas_per_sm(int D) { return D == 32 ? 8 : D == 64 ? 4 : D == 96 ? 3 : D == 128 ? 2 : 1; }
 
 template <int D, bool kBf16>
 int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* partLse) {
-  constexpr int kSmem = ring_bytes(D) + merge_bytes(D);
-  static_assert(kSmem <= 227 * 1024 && merge_bytes(D) <= ring_bytes(D) && merge_ld<D>() == D + 8, "shared memory");
-  auto kernel = fwd_splitkv_kernel<D, kBf16>;
+  constexpr int kSmem = ring_bytes(D) + merge_bytes(D, 1);
+  static_assert(kSmem <= kMaxSmem && merge_bytes(D, 4) <= ring_bytes(D) && merge_ld<D>() == D + 8, "shared memory");
+  auto kernel = plan.runs > 0 ? fwd_splitkv_kernel<D, kBf16, true> : fwd_splitkv_kernel<D, kBf16, false>;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return kCudaError;
   static std::once_flag once[64];
   static cudaError_t attrErr[64];
   std::call_once(once[device], [&] {
-    attrErr[device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    attrErr[device] = cudaFuncSetAttribute(fwd_splitkv_kernel<D, kBf16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    if (attrErr[device] == cudaSuccess) {
+      attrErr[device] = cudaFuncSetAttribute(fwd_splitkv_kernel<D, kBf16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    }
   });
   if (attrErr[device] != cudaSuccess) {
-    set_error_string("cudaFuncSetAttribute(%d bytes): %s", kSmem, cudaGetErrorString(attrErr[device]));
+    set_error_string("cudaFuncSetAttribute(%d bytes): %s", kMaxSmem, cudaGetErrorString(attrErr[device]));
     return kCudaError;
   }
   Params p;
@@ -643,7 +680,7 @@ int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* par
   p.scaleLog2 = (float)(1.4426950408889634 / sqrt((double)D));
   const dim3 grid = plan.runs > 0 ? dim3((unsigned)(plan.runs * pr.headsKV)) : dim3((unsigned)plan.splits, (unsigned)pr.headsKV, (unsigned)pr.batch);
   // head dim 96 fits three CTAs per SM without the merge buffer, two with it: packed, 223 x up to 5432 keys, 2 heads 138 -> 118 us
-  const size_t smem = plan.runs > 0 ? kSmem : ring_bytes(D);
+  size_t smem = plan.runs > 0 ? kSmem : ring_bytes(D);
   cudaError_t e = launch_kernel(kernel, grid, kThreads, smem, pr.stream, pr.overlap, p);
   if (e == cudaSuccess && plan.splits > 1) {
     const long long rows = pr.totalQ * pr.headsQ;
