@@ -650,11 +650,19 @@ int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* par
     if (attrErr[device] == cudaSuccess) {
       attrErr[device] = cudaFuncSetAttribute(fwd_splitkv_kernel<D, kBf16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     }
+    // all of it as shared memory: the spread below counts on it
+    if (attrErr[device] == cudaSuccess) {
+      attrErr[device] = cudaFuncSetAttribute(fwd_splitkv_kernel<D, kBf16, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    }
+    if (attrErr[device] == cudaSuccess) {
+      attrErr[device] = cudaFuncSetAttribute(fwd_splitkv_kernel<D, kBf16, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    }
   });
   if (attrErr[device] != cudaSuccess) {
     set_error_string("cudaFuncSetAttribute(%d bytes): %s", kMaxSmem, cudaGetErrorString(attrErr[device]));
     return kCudaError;
   }
+  const int numSMs = device_num_sms(device);
   Params p;
   p.Q = pr.Q;
   p.K = pr.K;
@@ -681,7 +689,15 @@ int launch(const FwdProblem& pr, const SplitPlan& plan, float* partO, float* par
   const dim3 grid = plan.runs > 0 ? dim3((unsigned)(plan.runs * pr.headsKV)) : dim3((unsigned)plan.splits, (unsigned)pr.headsKV, (unsigned)pr.batch);
   // head dim 96 fits three CTAs per SM without the merge buffer, two with it: packed, 223 x up to 5432 keys, 2 heads 138 -> 118 us
   size_t smem = plan.runs > 0 ? kSmem : ring_bytes(D);
-  cudaError_t e = launch_kernel(kernel, grid, kThreads, smem, pr.stream, pr.overlap, p);
+  // A grid that fits the GPU at once must not crowd on part of the SMs: its CTAs come in while those of the kernel before leave, and would
+  // fill up the SMs that are done first.  So shared memory holds no more CTAs of an SM than an even spread needs.  17 x 2 x 2513 keys, 64
+  // heads over 32 of 32, whole pairs: 42.6 -> 31.3 us.  A grid of several waves does not start early at all (200 x 5360 keys, 16 heads of 32,
+  // whole pairs: 417 -> 368 us).
+  const long long perSm = ((long long)grid.x * grid.y * grid.z + numSMs - 1) / numSMs;
+  const size_t share = (kSmemPerSm / (size_t)(perSm + 1) - kSmemReserved + 255) / 128 * 128;  // perSm + 1 CTAs of it do not fit
+  if (smem < share) smem = share;
+  const bool early = pr.overlap && perSm <= whole_ctas_per_sm(D);
+  cudaError_t e = launch_kernel(kernel, grid, kThreads, smem, pr.stream, early, p);
   if (e == cudaSuccess && plan.splits > 1) {
     const long long rows = pr.totalQ * pr.headsQ;
     const int tileRows = pr.seqLenQ * p.group;  // a longer sequence than the caller's maximum: the CTAs take turns
