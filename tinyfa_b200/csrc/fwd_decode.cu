@@ -756,21 +756,25 @@ SplitPlan splitkv_plan(const FwdProblem& p, int numSMs, int forced) {
     plan.blocksPerEntry = (int)blocks;
     const long long run = total / runs;  // the shortest run; partial results per pair:
     plan.splits = (int)(p.batch % runs == 0 ? 1 : runs % p.batch == 0 ? runs / p.batch : (blocks - 2) / run + 2);
-    // Against whole pairs, one CTA each.  In us: a block takes 4e-5 D of the memory rate and at least 0.345 + 0.00425 D in one CTA,
-    // and the combine kernel 3.7 and 0.95e-3 + 4.9e-6 D a row.  Fitted to 196 drawn calls of 120 pairs and more, all head dims: the pick
-    // is within 0.7 % of the faster cut on average, 14 % at worst.  us per call, runs against whole pairs: 59 x 2 x 442 keys, 128
-    // over 16 heads of 32 32.1, 12.3; 172 x 1 x 839, 64 over 4 of 32 32.9, 14.3; 398 x 16 x 519, 4 heads of 128 114, 85; on the
-    // other side 40 x 5000, 32 over 8 of 128 130, 174.
-    const double D = p.headDim, block = 4e-5 * D, chain = 0.345 + 0.00425 * D;
+    // Against whole pairs, one CTA each.  In us, a block of one CTA: 3.81e-5 D at the memory rate, 0.2 + 0.00415 D at least, and 0.0042 D
+    // for each of the CTAs that share its SM; the combine kernel: 5, and 1e-4 + 1.13e-5 D a row.  Fitted to 791 drawn calls of 40 pairs and
+    // more, all head dims: the pick is
+    // within 0.8 % of the faster cut on average.  us per call, runs against whole pairs: 59 x 2 x 442 keys, 128 heads over 16 of 32 30.7, 11.4;
+    // 172 x 1 x 839, 64 over 4 of 32 31.1, 14.5; 398 x 16 x 519, 4 heads of 128 109, 83; on the other side 40 x 5000, 32 over 8 of 128
+    // 128, 172; 5 x 13900, 32 heads of 128 169, 216.
+    const double D = p.headDim, block = 3.81e-5 * D;
+    auto step = [&](long long ctas) { return fmax(0.2 + 0.00415 * D, (double)((ctas + numSMs - 1) / numSMs) * 0.0042 * D); };
     const long long held = (long long)numSMs * decode::whole_ctas_per_sm(p.headDim), rest = pairs % held;
-    const double whole = (double)(pairs / held) * blocks * held * block + (rest > 0 ? blocks * fmax(rest * block, chain) : 0.0);
-    const double cut = fmax((double)pairs * blocks * block, (double)((total + runs - 1) / runs) * chain) +
-                       (plan.splits > 1 ? 3.7 + (double)p.totalQ * p.headsQ * (0.95e-3 + 4.9e-6 * D) : 0.0);
+    const double whole = (double)(pairs / held) * blocks * held * block + (rest > 0 ? blocks * fmax(rest * block, step(rest)) : 0.0);
+    const double cut = fmax((double)pairs * blocks * block, (double)((total + runs - 1) / runs) * step(runs * p.headsKV)) +
+                       (plan.splits > 1 ? 5.0 + (double)p.totalQ * p.headsQ * (1e-4 + 1.13e-5 * D) : 0.0);
     // (the factor: without a combine pass both estimates are the bytes, and runs end more evenly than pairs)
     if (whole <= (plan.splits > 1 ? cut : 0.99 * cut) && forced != -2) return SplitPlan{1, 0, 0};
     return plan;
   }
   plan.splits = splits_of_pairs(p, numSMs);  // packed input, and more pairs than the even partition is for
+  // causal calls see few keys: 5 x 3 x 556, 64 heads over 32 of 256 24.7 us in three splits, 12.4 whole
+  if (p.cuQ == nullptr && plan.splits > (seen + 255) / 256) plan.splits = (seen + 255) / 256;
   return plan;
 }
 
@@ -939,7 +943,7 @@ extern "C" int tfa_b200_fwd_decode_noalloc(const void* Q, const void* K, const v
   SplitPlan plan = splitkv_plan(p, sms, numSplits > 0 ? numSplits : 0);
   // What the entry point accepts is stated in splits of pairs; an even partition whose partials do not fit the array gives
   // way to whole pairs, as many at a time as the GPU holds.
-  const SplitPlan stated = {plan.runs > 0 ? splits_of_pairs(p, sms) : plan.splits, 0, 0};
+  const SplitPlan stated = {numSplits > 0 ? plan.splits : splits_of_pairs(p, sms), 0, 0};
   const size_t limit = (size_t)TFA_B200_NOALLOC_SCRATCH_FLOATS, statedNeed = splitkv_scratch_floats(p, stated);
   if (statedNeed > limit) {
     set_error_string("split-KV partials need %zu floats (%d splits x %lld rows x (%d + 1)) but the built-in scratch holds "
