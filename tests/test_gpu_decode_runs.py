@@ -175,3 +175,16 @@ def test_cut_by_cost(shape, D, runs):
     want = tf.flash_attn_forward(Q, K, V)
     tf.set_option("split_kv", -1)
     assert torch.equal(auto, want)
+
+
+@pytest.mark.parametrize("shape,D", [((5, 3, 556, 64, 32), 256), ((3, 16, 9000, 2, 2), 64), ((1, 1, 700, 8, 1), 128)])
+def test_causal_calls_are_not_split_over_keys_they_do_not_see(shape, D):
+    B, Sq, Skv, Hq, Hkv = shape
+    Q, K, V = (torch.randn(*s, device="cuda").half() for s in ((B, Sq, Hq, D), (B, Skv, Hkv, D), (B, Skv, Hkv, D)))
+    auto = tf.flash_attn_forward(Q, K, V, is_causal=True)
+    tf.set_option("split_kv", 1)
+    want = tf.flash_attn_forward(Q, K, V, is_causal=True)
+    tf.set_option("split_kv", -1)
+    assert torch.equal(auto, want)
+    ref = ao.fixed(*(t.float().cpu().numpy() for t in (Q, K, V)), True, "f64")
+    assert (auto.cpu().double() - torch.from_numpy(ref).double()).abs().max() <= 4e-3

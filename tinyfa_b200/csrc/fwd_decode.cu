@@ -14,9 +14,9 @@
 //   * warps are merged through shared memory, partial results through a small fp32 scratch buffer and a combine kernel
 //     that is launched while the split kernel runs (programmatic dependent launch) and reads a row's partials side by side.
 // Measured against a fixed number of splits per pair and a combine kernel that walked them (8 KV heads, D = 128, three sets of
-// inputs in turn, both builds in one job; floor in brackets at 6.54 TB/s): batch 1 x 32768 keys 37.6 -> 28.4 us (20.5), 8 x 20011
-// 112.3 -> 100.4 (100; with inputs spread over more memory 113.4 -> 105.6), 40 x 5000 169.6 -> 127.7 (125), 13 x 8000 76.0 -> 71.6 (65),
-// 6 x 12000 61.6 -> 51.8 (45).  What is left at small batch is launch, the first loads and the combine.
+// inputs in turn, both builds in one job; floor in brackets at 6.54 TB/s): batch 1 x 32768 keys 37.3 -> 28.3 us (20.5), 8 x 20011
+// 112.5 -> 101.3 (100), 40 x 5000 168.9 -> 128.3 (125), 13 x 8000 75.9 -> 70.8 (65), 6 x 12000 61.6 -> 52.0 (45).  What is left at
+// small batch is launch, the first loads and the combine.
 // Numerical contract as in the main kernel (reference csrc/flash_attn/mma/softmax.cuh:67-138): scale 1/sqrt(D)
 // folded into exp2, top-left causal mask, "col >= seqLenKV" mask, P rounded to the 16-bit type before P.V, row sum
 // from unrounded P, empty rows give 0.
@@ -759,7 +759,7 @@ SplitPlan splitkv_plan(const FwdProblem& p, int numSMs, int forced) {
     // Against whole pairs, one CTA each.  In us, a block of one CTA: 3.81e-5 D at the memory rate, 0.2 + 0.00415 D at least, and 0.0042 D
     // for each of the CTAs that share its SM; the combine kernel: 5, and 1e-4 + 1.13e-5 D a row.  Fitted to 791 drawn calls of 40 pairs and
     // more, all head dims: the pick is
-    // within 0.8 % of the faster cut on average.  us per call, runs against whole pairs: 59 x 2 x 442 keys, 128 heads over 16 of 32 30.7, 11.4;
+    // within 0.8 % of the faster cut on average, on 250 others within 1.4 %.  us per call, runs against whole pairs: 59 x 2 x 442 keys, 128 heads over 16 of 32 30.7, 11.4;
     // 172 x 1 x 839, 64 over 4 of 32 31.1, 14.5; 398 x 16 x 519, 4 heads of 128 109, 83; on the other side 40 x 5000, 32 over 8 of 128
     // 128, 172; 5 x 13900, 32 heads of 128 169, 216.
     const double D = p.headDim, block = 3.81e-5 * D;
